@@ -7,6 +7,7 @@
  */
 #include <algorithm>
 #include <chrono>
+#include <condition_variable>
 #include <deque>
 #include <thread>
 #include <cmath>
@@ -27,8 +28,7 @@ struct mfcfd_handle {
     Topology T;
     DevCloud d;
     cudaStream_t stream = nullptr;
-    cudaStream_t side = nullptr;          // flux residual beside the chain forward sweep
-    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaEvent_t fork = nullptr;
     double *U_buf[2] = {nullptr, nullptr};
     double *q_buf[2] = {nullptr, nullptr};
     int cur = 0;          // U/q buffer the next iteration reads
@@ -52,21 +52,26 @@ struct mfcfd_handle {
     // host copies held between mfcfd_prepare and mfcfd_attach
     struct Staged {
         std::vector<double> x, y, z, frame;
-        std::vector<int32_t> nbhs, conn, pre;
+        std::vector<int32_t> nbhs, conn;
         ChainSchedule S;
-        int ch_w = 0, ch_wpb = 0;
+        int chains = 0;
     };
     std::unique_ptr<Staged> staged;
     bool dry = false;                      // count device bytes, allocate and copy nothing
     // captured chunks of iterations: (chunk length, U/q buffer at its start)
     struct GraphSlot {
         int chunk = -1, parity = -1;
+        ChainShape shape{};
         cudaGraphExec_t exec = nullptr;
     };
-    GraphSlot graphs[2];
+    GraphSlot graphs[4];
     int graph_next = 0;
     cudaEvent_t batch_ev = nullptr;        // end of the handle's chunk in mfcfd_run_batch / mfcfd_launch
     int pending_chunk = 0;                 // mfcfd_launch: iterations not yet completed
+    int held = 0, held_budget = 0;         // slots of the running chunk, and its budget of them
+    // chain schedule: the warps it may hold beside other handles' (in blocks
+    // of ch_wpb); DevCloud::ch_shape is the shape of the running chunk
+    int ch_budget = 0, ch_wpb = 0;
     int32_t pending_t0 = 0;
     bool graphs_off = false;               // a capture failed: launch one by one
     // device-resident set-up (mfcfd_params.gpu_setup = 1): the topology was
@@ -184,10 +189,15 @@ void drop_graphs(mfcfd_handle *h) {
     }
 }
 
+void give_slots(mfcfd_handle *h);
+
 void release(mfcfd_handle *h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
+    if (h->pending_chunk) {                // launched and never completed
+        give_slots(h);
+        h->pending_chunk = 0;
+    }
     drop_graphs(h);
-    if (h->side) cudaStreamSynchronize(h->side);
     for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
     h->ev.clear();
     for (void *p : h->allocs) {
@@ -199,10 +209,7 @@ void release(mfcfd_handle *h) {
     if (h->batch_ev) cudaEventDestroy(h->batch_ev);
     h->batch_ev = nullptr;
     if (h->fork) cudaEventDestroy(h->fork);
-    if (h->join) cudaEventDestroy(h->join);
-    h->fork = h->join = nullptr;
-    if (h->side) cudaStreamDestroy(h->side);
-    h->side = nullptr;
+    h->fork = nullptr;
     if (h->stream) cudaStreamDestroy(h->stream);
     h->stream = nullptr;
 }
@@ -225,12 +232,78 @@ int launch_one(mfcfd_handle *h, int j) {
     dc.U = h->U_buf[h->cur];
     dc.q = h->q_buf[h->cur];
     cudaEvent_t *ev = h->profiling ? &h->ev[(size_t)j * (MFCFD_NPHASE + 1)] : nullptr;
-    const IterStreams st{h->stream, h->side, h->fork, h->join};
+    const IterStreams st{h->stream, h->fork};
     cudaError_t e = launch_iteration(dc, j, st, h->U_buf[1 - h->cur], h->q_buf[1 - h->cur], ev);
     if (e != cudaSuccess) return cuda_fail(h, e, "kernel launch");
     h->last = h->cur;
     h->cur = 1 - h->cur;
     return MFCFD_OK;
+}
+
+// Slots of a device's chain sweeps in use (chain_slot_capacity), over every
+// handle and thread of the process.  A run holds at least its handles'
+// budgets (mfcfd_info.chain_slots), whose sum over concurrent runs is the
+// callers' to bound; a run of mfcfd_run, mfcfd_run_batch, mfcfd_run_group or
+// the request server may hold more while nobody needs it, for one chunk of
+// iterations at a time, and whoever does not find room for its budget beside
+// such a run waits for that chunk.
+struct SlotPool {
+    std::mutex mu;
+    std::condition_variable freed;
+    int used = 0, excess = 0;
+};
+SlotPool g_slots[256];
+constexpr int EXCESS_CHUNK = 64;           // iterations a run beyond its budget lasts at most
+
+// Take slots for handles of these chain counts: the shape of their sweeps in
+// *shape (the largest teams within max(budget, min(want, what is free))).
+// Returns the slots held; -1, with `wait` false, instead of waiting (for a
+// caller that itself holds more than its budgets).
+int take_slots(int dev, const int *chains, int count, int precision, int spread, int budget, int want, bool wait,
+               ChainShape *shape) {
+    SlotPool &p = g_slots[dev & 255];
+    const int capacity = chain_slot_capacity(dev);
+    std::unique_lock<std::mutex> lock(p.mu);
+    auto room = [&] { return p.used + budget <= capacity || p.excess == 0; };
+    if (!wait && !room()) return -1;
+    p.freed.wait(lock, room);
+    *shape = chain_fit(chains, count, precision, spread, std::max(budget, std::min(want, capacity - p.used)));
+    int hold = 0;
+    for (int i = 0; i < count; ++i) hold += chain_slots(chains[i], *shape, precision);
+    hold = std::max(hold, budget);
+    p.used += hold;
+    p.excess += hold - budget;
+    return hold;
+}
+void give_slots(int dev, int budget, int hold) {
+    SlotPool &p = g_slots[dev & 255];
+    {
+        std::lock_guard<std::mutex> lock(p.mu);
+        p.used -= hold;
+        p.excess -= hold - budget;
+    }
+    p.freed.notify_all();
+}
+int budget_slots(const mfcfd_handle *h) {
+    return h->d.sweep_mode == MFCFD_SWEEP_CHAINS
+               ? chain_budget_slots(h->ch_budget, h->ch_wpb, h->d.precision, h->P.chain_spread)
+               : 0;
+}
+// Slots of one handle's chunk (h->held; 0 for the other schedules), its shape
+// set; false if it would have to wait.
+bool take_slots(mfcfd_handle *h, int want, bool wait) {
+    h->held = h->held_budget = 0;
+    if (h->d.sweep_mode != MFCFD_SWEEP_CHAINS) return true;
+    h->held_budget = budget_slots(h);
+    h->held = take_slots(h->P.device, &h->d.ch_chains, 1, h->d.precision, h->P.chain_spread, h->held_budget, want, wait,
+                         &h->d.ch_shape);
+    if (h->held >= 0) return true;
+    h->held = 0;
+    return false;
+}
+void give_slots(mfcfd_handle *h) {
+    if (h->held > 0) give_slots(h->P.device, h->held_budget, h->held);
+    h->held = 0;
 }
 
 // Launch the iterations of one chunk (slots 0 .. chunk-1).  With graphs, the
@@ -248,11 +321,11 @@ int launch_chunk(mfcfd_handle *h, int chunk, bool batch) {
     const int c0 = h->cur;
     mfcfd_handle::GraphSlot *g = nullptr;
     for (auto &s : h->graphs)
-        if (s.exec && s.chunk == chunk && s.parity == c0) g = &s;
+        if (s.exec && s.chunk == chunk && s.parity == c0 && s.shape == h->d.ch_shape) g = &s;
     if (!g) {
         prepare_launches(h->P.device);
         mfcfd_handle::GraphSlot &slot = h->graphs[h->graph_next];
-        h->graph_next ^= 1;
+        h->graph_next = (h->graph_next + 1) % 4;
         if (slot.exec) cudaGraphExecDestroy(slot.exec);
         slot = mfcfd_handle::GraphSlot();
         const int last0 = h->last;
@@ -281,6 +354,7 @@ int launch_chunk(mfcfd_handle *h, int chunk, bool batch) {
         }
         slot.chunk = chunk;
         slot.parity = c0;
+        slot.shape = h->d.ch_shape;
         g = &slot;
     }
     CK(cudaGraphLaunch(g->exec, h->stream));
@@ -306,16 +380,9 @@ int finish_chunk(mfcfd_handle *h, int32_t t0, int chunk, double *res_hist, int *
     if (h->profiling) {
         for (int j = 0; j < chunk; ++j) {
             const cudaEvent_t *ev = &h->ev[(size_t)j * (MFCFD_NPHASE + 1)];
-            // event pairs per phase; under the chain schedule the flux
-            // residual (ended by event 2, side stream) starts at event 3
-            // and runs beside the forward sweep, after k_pending (1-3)
-            static const int kSeq[MFCFD_NPHASE][2] = {{0, 1}, {1, 2}, {2, 3}, {3, 4}, {4, 5}, {5, 6}, {6, 7}};
-            static const int kFused[MFCFD_NPHASE][2] = {{0, 1}, {3, 2}, {1, 3}, {3, 4}, {4, 5}, {5, 6}, {6, 7}};
-            const bool fused = h->d.sweep_mode == MFCFD_SWEEP_CHAINS;
             for (int ph = 0; ph < MFCFD_NPHASE; ++ph) {
                 float ms = 0.f;
-                const int *pr = fused ? kFused[ph] : kSeq[ph];
-                CK(cudaEventElapsedTime(&ms, ev[pr[0]], ev[pr[1]]));
+                CK(cudaEventElapsedTime(&ms, ev[ph], ev[ph + 1]));
                 h->phase_ms[ph] += ms;
             }
         }
@@ -332,13 +399,14 @@ int finish_chunk(mfcfd_handle *h, int32_t t0, int chunk, double *res_hist, int *
     return MFCFD_OK;
 }
 
-// Rebuild the chain schedule for about `want` warps on the handle's
-// topology and replace its device copy (the term records are re-marked, so
-// they are copied again); *warps receives the new schedule's warps.
+// Rebuild the chain schedule for a budget of about `want` warps on the
+// handle's topology and replace its device copy (the term records are
+// re-marked, so they are copied again); *warps receives the budget.
 int apply_chain_schedule(mfcfd_handle *h, int want, int *warps) {
-    int wpb = 0, blocks = 0;
-    const int w = chain_shape(h->P.device, want, h->P.chain_spread, &wpb, &blocks);
-    if (w < 1) return fail(h, MFCFD_ERR_CUDA, "chain sweep kernel cannot be resident");
+    int wpb = 0;
+    const int budget = chain_budget(h->P.device, want, h->P.chain_spread, &wpb);
+    if (budget < 1) return fail(h, MFCFD_ERR_CUDA, "chain sweep kernel cannot be resident");
+    const int w = chain_count(h->P.device, budget, h->T.max_level_width, h->P.chain_spread);
     if (h->dev_setup) {
         DevCloud &d = h->d;
         for (int dir = 0; dir < 2; ++dir) {
@@ -357,11 +425,11 @@ int apply_chain_schedule(mfcfd_handle *h, int want, int *warps) {
         int64_t terms[3];
         if (int rc = device_chain_schedule(h->P.device, h->dt, d, w, h->stream, alloc, terms, err))
             return fail(h, rc, err.empty() ? h->err : err);
-        d.ch_wpb = wpb;
-        d.ch_spread = h->P.chain_spread;
+        h->ch_budget = budget;
+        h->ch_wpb = wpb;
         drop_graphs(h);
         for (int k = 0; k < 3; ++k) h->chain_terms[k] = terms[k];
-        *warps = w;
+        *warps = budget;
         return MFCFD_OK;
     }
     ChainSchedule S;
@@ -387,16 +455,16 @@ int apply_chain_schedule(mfcfd_handle *h, int want, int *warps) {
         }
     // the host's terms carry the unfolded weights
     if (d.precision != MFCFD_PRECISION_FP64) CK(launch_fold_terms(d, h->w_saved, true, h->stream));
-    d.ch_warps = w;
-    d.ch_wpb = wpb;
-    d.ch_spread = h->P.chain_spread;
+    d.ch_chains = w;
+    h->ch_budget = budget;
+    h->ch_wpb = wpb;
     drop_graphs(h);                        // their launches name the old schedule
     h->chain_terms[0] = S.terms_ring;
     h->chain_terms[1] = S.terms_local;
     h->chain_terms[2] = S.terms_cross;
     cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return cuda_fail(h, e, "cudaStreamSynchronize");
-    *warps = w;
+    *warps = budget;
     return MFCFD_OK;
 }
 
@@ -404,10 +472,13 @@ int run_iterations(mfcfd_handle *h, int32_t t0, int32_t iters, double *res_hist)
     if (!h->have_state) return fail(h, MFCFD_ERR_ARG, "no state: call mfcfd_set_prim first");
     int status = MFCFD_OK;
     for (int32_t done = 0; done < iters;) {
+        take_slots(h, 1 << 20, true);
         int chunk = std::min<int32_t>(iters - done, h->res_cap);
+        if (h->held > h->held_budget) chunk = std::min(chunk, EXCESS_CHUNK);
         int rc = launch_chunk(h, chunk, false);
-        if (rc) return rc;
-        rc = finish_chunk(h, t0 + done, chunk, res_hist ? res_hist + 2 * (size_t)done : nullptr, &status);
+        if (rc) cudaStreamSynchronize(h->stream);
+        if (!rc) rc = finish_chunk(h, t0 + done, chunk, res_hist ? res_hist + 2 * (size_t)done : nullptr, &status);
+        give_slots(h);
         if (rc) return rc;
         done += chunk;
     }
@@ -590,10 +661,11 @@ int stage_host(mfcfd_handle *h, const double *x, const double *y, const double *
         // warp count set before then costs one build
         if (P.chain_warps < 0) return fail(h, MFCFD_ERR_ARG, "chain_warps must not be negative");
         const int want = P.chain_warps > 0 ? P.chain_warps : std::max(1, 2 * h->T.max_level_width);
-        int blocks = 0;
         if (P.chain_spread < 0 || P.chain_spread > 1) return fail(h, MFCFD_ERR_ARG, "chain_spread must be 0 or 1");
-        st->ch_w = chain_shape(P.device, want, P.chain_spread, &st->ch_wpb, &blocks);
-        if (st->ch_w < 1) return fail(h, MFCFD_ERR_CUDA, "chain sweep kernel cannot be resident");
+        h->ch_budget = chain_budget(P.device, want, P.chain_spread, &h->ch_wpb);
+        st->chains = chain_count(P.device, h->ch_budget, h->T.max_level_width, P.chain_spread);
+        if (h->ch_budget < 1 || !chain_fits(P.device, false))
+            return fail(h, MFCFD_ERR_CUDA, "chain sweep kernel cannot be resident");
     }
     h->staged = std::move(st);
     return MFCFD_OK;
@@ -617,17 +689,14 @@ void keep_pool_memory(int device) {
     done.push_back(device);
 }
 
-// The handle's streams: the main stream outranks the side stream, so the
-// chain sweep's blocks are placed before the concurrent flux kernel's.
+// The handle's stream, of the highest priority, and its event.
 int create_streams(mfcfd_handle *h) {
     if (cudaSetDevice(h->P.device) != cudaSuccess) return fail(h, MFCFD_ERR_CUDA, "cudaSetDevice failed");
     keep_pool_memory(h->P.device);
     int least = 0, greatest = 0;
     CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
     CK(cudaStreamCreateWithPriority(&h->stream, cudaStreamNonBlocking, greatest));
-    CK(cudaStreamCreateWithPriority(&h->side, cudaStreamNonBlocking, least));
     CK(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming));
     return MFCFD_OK;
 }
 
@@ -664,17 +733,13 @@ int attach_device(mfcfd_handle *h) {
     if (P.sweep_mode == MFCFD_SWEEP_CHAINS) {
         // the schedule marks the entry lists, so it precedes their upload
         mfcfd_handle::Staged &ms = *h->staged;
-        if (ms.S.warps != ms.ch_w) {
+        if (ms.S.warps != ms.chains) {
             ms.S = ChainSchedule();
-            build_chain_schedule(h->T, ms.ch_w, ms.S);
+            build_chain_schedule(h->T, ms.chains, ms.S);
         }
-        if (ms.pre.empty()) build_pre_order(h->T, ms.pre);
         const ChainSchedule &S = st.S;
-        d.ch_warps = st.ch_w;
-        d.ch_wpb = st.ch_wpb;
-        d.ch_spread = P.chain_spread;
+        d.ch_chains = st.chains;
         d.flux_grid = P.flux_blocks_per_sm > 0 ? P.flux_blocks_per_sm * device_sms(P.device) : 0;
-        if ((rc = upload(h, &d.pre_order, st.pre))) return rc;
         for (int dir = 0; dir < 2; ++dir) {
             if ((rc = upload(h, &d.ch_ptr[dir], S.ptr[dir]))) return rc;
             if ((rc = upload(h, &d.ch_pts[dir], S.pts[dir]))) return rc;
@@ -822,14 +887,13 @@ int create_on_device(mfcfd_handle *h, const double *x, const double *y, const do
     }
     if (P.sweep_mode == MFCFD_SWEEP_CHAINS) {
         const int want = P.chain_warps > 0 ? P.chain_warps : std::max(1, 2 * T.max_level_width);
-        int wpb = 0, blocks = 0;
-        const int w = chain_shape(P.device, want, P.chain_spread, &wpb, &blocks);
-        if (w < 1) return fail(h, MFCFD_ERR_CUDA, "chain sweep kernel cannot be resident");
+        h->ch_budget = chain_budget(P.device, want, P.chain_spread, &h->ch_wpb);
+        const int w = chain_count(P.device, h->ch_budget, T.max_level_width, P.chain_spread);
+        if (h->ch_budget < 1 || !chain_fits(P.device, false))
+            return fail(h, MFCFD_ERR_CUDA, "chain sweep kernel cannot be resident");
         int64_t terms[3];
         if ((rc = device_chain_schedule(P.device, h->dt, d, w, h->stream, alloc, terms, err)))
             return fail(h, rc, err.empty() ? h->err : err);
-        d.ch_wpb = wpb;
-        d.ch_spread = P.chain_spread;
         d.flux_grid = P.flux_blocks_per_sm > 0 ? P.flux_blocks_per_sm * device_sms(P.device) : 0;
         for (int k = 0; k < 3; ++k) h->chain_terms[k] = terms[k];
         if (d.n_g0 > 0 && (rc = dalloc(h, &d.g0, (size_t)d.n_g0 * G0_DOUBLES))) return rc;
@@ -975,7 +1039,7 @@ int mfcfd_fpi_step(mfcfd_handle *h, int32_t t, double *res_new, double *residue)
     });
 }
 
-int mfcfd_launch(mfcfd_handle *h, int32_t t0, int32_t iters) {
+extern "C++" int mfcfd::launch_within(mfcfd_handle *h, int32_t t0, int32_t iters, int slots, bool wait, int *held) {
     return host_guard(h ? &h->err : nullptr, [&]() -> int {
         if (!h || iters < 1) return MFCFD_ERR_ARG;
         if (!h->stream) return fail(h, MFCFD_ERR_ARG, "handle was not created successfully");
@@ -984,14 +1048,23 @@ int mfcfd_launch(mfcfd_handle *h, int32_t t0, int32_t iters) {
         if (iters > h->res_cap) return fail(h, MFCFD_ERR_ARG, "at most 1024 iterations per launch");
         CK(cudaSetDevice(h->P.device));
         if (!h->batch_ev) CK(cudaEventCreateWithFlags(&h->batch_ev, cudaEventDisableTiming));
+        if (!take_slots(h, slots, wait)) return MFCFD_ERR_BUSY;
         int rc = launch_chunk(h, iters, true);
-        if (rc) return rc;
-        CK(cudaEventRecord(h->batch_ev, h->stream));
+        const cudaError_t e = rc ? cudaSuccess : cudaEventRecord(h->batch_ev, h->stream);
+        if (e != cudaSuccess) rc = cuda_fail(h, e, "cudaEventRecord");
+        if (rc) {
+            cudaStreamSynchronize(h->stream);
+            give_slots(h);
+            return rc;
+        }
         h->pending_chunk = iters;
         h->pending_t0 = t0;
+        if (held) *held = h->held;
         return MFCFD_OK;
     });
 }
+
+int mfcfd_launch(mfcfd_handle *h, int32_t t0, int32_t iters) { return mfcfd::launch_within(h, t0, iters, 0, true, nullptr); }
 
 int mfcfd_complete(mfcfd_handle *h, int32_t wait, double *res_hist, int32_t *done) {
     return host_guard(h ? &h->err : nullptr, [&]() -> int {
@@ -1007,6 +1080,7 @@ int mfcfd_complete(mfcfd_handle *h, int32_t wait, double *res_hist, int32_t *don
         const int chunk = h->pending_chunk;
         h->pending_chunk = 0;
         int rc = finish_chunk(h, h->pending_t0, chunk, res_hist, &st);
+        give_slots(h);
         *done = 1;
         return rc ? rc : st;
     });
@@ -1148,7 +1222,7 @@ int mfcfd_debug_digest(mfcfd_handle *h, const char *name, uint64_t *digest, int6
         int32_t ends[2] = {0, 0};
         if (d.fwd_off) CK(cudaMemcpy(&ends[0], d.fwd_off + n, 4, cudaMemcpyDeviceToHost));
         if (d.bwd_off) CK(cudaMemcpy(&ends[1], d.bwd_off + n, 4, cudaMemcpyDeviceToHost));
-        const size_t nsw = (size_t)d.n_swept, w1 = (size_t)d.ch_warps + 1;
+        const size_t nsw = (size_t)d.n_swept, w1 = (size_t)d.ch_chains + 1;
         const bool ch = d.sweep_mode == MFCFD_SWEEP_CHAINS;
         const struct {
             const char *name;
@@ -1170,7 +1244,7 @@ int mfcfd_debug_digest(mfcfd_handle *h, const char *name, uint64_t *digest, int6
             {"fwd_need", d.fwd_need, 4 * n}, {"bwd_need", d.bwd_need, 4 * n},
             {"fwd_old", d.fwd_old, 4 * n}, {"bwd_old", d.bwd_old, 4 * n},
             {"sweep_slot_mask", d.sweep_slot_mask, n * MAX_SLOTS}, {"res_order", d.res_order, 4 * (size_t)d.n_res},
-            {"pre_order", d.pre_order, ch ? 4 * n : 0}, {"g0_pts", d.g0_pts, 4 * (size_t)d.n_g0},
+            {"pre_order", nullptr, 0}, {"g0_pts", d.g0_pts, 4 * (size_t)d.n_g0},
             {"ch_ptr0", d.ch_ptr[0], ch ? 4 * w1 : 0}, {"ch_pts0", d.ch_pts[0], ch ? 4 * nsw : 0},
             {"ch_own0", d.ch_own[0], ch ? 4 * n : 0}, {"ch_items0", d.ch_items[0], ch ? sizeof(ChainItem) * nsw : 0},
             {"ch_ptr1", d.ch_ptr[1], ch ? 4 * w1 : 0}, {"ch_pts1", d.ch_pts[1], ch ? 4 * nsw : 0},
@@ -1207,20 +1281,14 @@ int mfcfd_get_info(mfcfd_handle *h, mfcfd_info *info) {
         info->shared_frame = T.shared_frame;
         info->device_bytes = h->bytes;
         info->sweep_mode = h->P.sweep_mode;
-        info->chain_warps = h->d.ch_warps;
+        info->chain_warps = h->ch_budget;
         info->chain_terms_ring = h->chain_terms[0];
         info->chain_terms_local = h->chain_terms[1];
         info->chain_terms_cross = h->chain_terms[2];
         if (h->P.sweep_mode == MFCFD_SWEEP_CHAINS && h->P.device >= 0) {
-            const int wpb = h->stream ? h->d.ch_wpb : (h->staged ? h->staged->ch_wpb : 0);
-            const int w = h->stream ? h->d.ch_warps : (h->staged ? h->staged->ch_w : 0);
-            info->chain_slots =
-                wpb > 0 ? (w + wpb - 1) / wpb * chain_block_slots(h->P.device, wpb, h->P.precision,
-                                                      h->P.chain_spread)
-                        : 0;
+            info->chain_slots = chain_budget_slots(h->ch_budget, h->ch_wpb, h->P.precision, h->P.chain_spread);
             info->chain_slot_capacity = chain_slot_capacity(h->P.device);
-            info->chain_warps_per_block = wpb;
-            if (!info->chain_warps) info->chain_warps = w;
+            info->chain_warps_per_block = h->ch_wpb;
             info->g0_points = (int32_t)h->T.g0_pts.size();
         }
         return MFCFD_OK;
@@ -1345,30 +1413,35 @@ int mfcfd_run_batch(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
             if (!hs[i]->batch_ev && cudaEventCreateWithFlags(&hs[i]->batch_ev, cudaEventDisableTiming) != cudaSuccess)
                 return cuda_fail(hs[i], cudaGetLastError(), "cudaEventCreateWithFlags");
         }
-        auto slots_of = [&](int32_t i) {
-            const DevCloud &d = hs[i]->d;
-            return d.sweep_mode == MFCFD_SWEEP_CHAINS
-                       ? (d.ch_warps + d.ch_wpb - 1) / d.ch_wpb *
-                             chain_block_slots(hs[i]->P.device, d.ch_wpb, d.precision,
-                                               d.ch_spread)
-                       : 0;
+        // each handle's share of the device, by its budget
+        long budgets = 0;
+        for (int32_t i = 0; i < count; ++i) budgets += budget_slots(hs[i]);
+        // every launched chunk ends (and its slots return) before an error
+        // leaves the call
+        auto drain = [&](int rc) {
+            for (const int32_t i : running) {
+                cudaStreamSynchronize(hs[i]->stream);
+                give_slots(hs[i]);
+            }
+            return rc;
         };
         int used = 0;
         while (!ready.empty() || !running.empty()) {
             while (!ready.empty()) {
                 const int32_t i = ready.front();
-                const int sl = slots_of(i);
-                if (!running.empty() && used + sl > capacity) break;
-                ready.pop_front();
                 mfcfd_handle *h = hs[i];
+                if (!running.empty() && used + budget_slots(h) > capacity) break;
+                const int share = (int)std::min<long>(capacity, (long)capacity * budget_slots(h) / std::max(budgets, 1l));
+                if (!take_slots(h, share, running.empty())) break;
+                ready.pop_front();
                 const int chunk = std::min<int32_t>(iters - done[i], std::max(h->res_cap, 1));
                 int rc = launch_chunk(h, chunk, true);
-                if (rc) return rc;
-                cudaError_t e = cudaEventRecord(h->batch_ev, h->stream);
-                if (e != cudaSuccess) return cuda_fail(h, e, "cudaEventRecord");
-                chunk_of[i] = chunk;
-                used += sl;
+                const cudaError_t e = rc ? cudaSuccess : cudaEventRecord(h->batch_ev, h->stream);
+                if (e != cudaSuccess) rc = cuda_fail(h, e, "cudaEventRecord");
                 running.push_back(i);
+                if (rc) return drain(rc);
+                chunk_of[i] = chunk;
+                used += h->held;
             }
             // wait for the first of the running chunks to complete
             int found = -1;
@@ -1376,16 +1449,17 @@ int mfcfd_run_batch(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
                 for (size_t r = 0; r < running.size() && found < 0; ++r) {
                     const cudaError_t q = cudaEventQuery(hs[running[r]]->batch_ev);
                     if (q == cudaSuccess) found = (int)r;
-                    else if (q != cudaErrorNotReady) return cuda_fail(hs[running[r]], q, "cudaEventQuery");
+                    else if (q != cudaErrorNotReady) return drain(cuda_fail(hs[running[r]], q, "cudaEventQuery"));
                 }
                 if (found < 0) std::this_thread::sleep_for(std::chrono::microseconds(20));
             }
             const int32_t i = running[found];
             running.erase(running.begin() + found);
-            used -= slots_of(i);
+            used -= hs[i]->held;
             int st = MFCFD_OK;
             double *rh = res_hist ? res_hist + 2 * ((size_t)i * iters + done[i]) : nullptr;
             int rc = finish_chunk(hs[i], t0[i] + done[i], chunk_of[i], rh, &st);
+            give_slots(hs[i]);
             if (!rc) rc = st;
             if (status && rc && status[i] == MFCFD_OK) status[i] = rc;
             if (rc && first_err == MFCFD_OK) first_err = rc;
@@ -1400,11 +1474,13 @@ namespace {
 
 // Streams and events of one mfcfd_run_group call, released on every path.
 struct GroupRun {
+    ChainShape shape{};
     cudaStream_t s = nullptr;
     cudaEvent_t start = nullptr, bwd = nullptr;
     struct Graph {
         int chunk;
         std::vector<int> cur;
+        ChainShape shape;
         cudaGraphExec_t exec;
     };
     std::vector<Graph> graphs;
@@ -1431,19 +1507,19 @@ cudaError_t launch_group_chunk(mfcfd_handle *const *hs, int count, int chunk, Gr
             mfcfd_handle *h = hs[i];
             DevCloud &dc = G.cloud[i];
             dc = h->d;
+            dc.ch_shape = gr.shape;
             dc.U = h->U_buf[h->cur];
             dc.q = h->q_buf[h->cur];
-            const IterStreams st{h->stream, h->side, h->fork, h->join};
+            const IterStreams st{h->stream, h->fork};
             e = launch_iteration(dc, j, st, h->U_buf[1 - h->cur], h->q_buf[1 - h->cur], nullptr, ITER_PRE);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(gr.s, h->fork, 0);
         }
-        if (e == cudaSuccess) e = launch_chain_group(G, d0.ch_wpb, d0.precision, d0.ch_spread, 1, gr.s);
-        for (int i = 0; i < count && e == cudaSuccess; ++i) e = cudaStreamWaitEvent(gr.s, hs[i]->join, 0);
-        if (e == cudaSuccess) e = launch_chain_group(G, d0.ch_wpb, d0.precision, d0.ch_spread, 0, gr.s);
+        if (e == cudaSuccess) e = launch_chain_group(G, gr.shape, d0.precision, 1, gr.s);
+        if (e == cudaSuccess) e = launch_chain_group(G, gr.shape, d0.precision, 0, gr.s);
         if (e == cudaSuccess) e = cudaEventRecord(gr.bwd, gr.s);
         for (int i = 0; i < count && e == cudaSuccess; ++i) {
             mfcfd_handle *h = hs[i];
-            const IterStreams st{h->stream, h->side, h->fork, h->join};
+            const IterStreams st{h->stream, h->fork};
             e = cudaStreamWaitEvent(h->stream, gr.bwd, 0);
             if (e == cudaSuccess)
                 e = launch_iteration(G.cloud[i], j, st, h->U_buf[1 - h->cur], h->q_buf[1 - h->cur], nullptr,
@@ -1475,26 +1551,30 @@ int mfcfd_run_group(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
         }
         mfcfd_handle *h0 = hs[0];
         const DevCloud &d0 = h0->d;
-        int slots = 0;
         for (int32_t i = 0; i < count; ++i) {
             const mfcfd_handle *h = hs[i];
             const DevCloud &d = h->d;
             if (d.sweep_mode != MFCFD_SWEEP_CHAINS)
                 return fail(h0, MFCFD_ERR_UNSUPPORTED, "a group runs chain-schedule handles only");
-            if (d.ch_wpb != d0.ch_wpb || d.ch_spread != d0.ch_spread ||
+            if (h->ch_wpb != h0->ch_wpb || h->P.chain_spread != h0->P.chain_spread ||
                 (d.precision == MFCFD_PRECISION_FP64) != (d0.precision == MFCFD_PRECISION_FP64))
                 return fail(h0, MFCFD_ERR_UNSUPPORTED,
                             "a group's handles share one chain block shape, chain_spread and precision class");
             if (h->profiling) return fail(h0, MFCFD_ERR_UNSUPPORTED, "phase timing is per handle, not in a group");
-            slots += (d.ch_warps + d.ch_wpb - 1) / d.ch_wpb * chain_block_slots(dev, d.ch_wpb, d.precision, d.ch_spread);
         }
         mfcfd_handle *const h = h0;        // errors of the group's own calls
         if (cudaSetDevice(dev) != cudaSuccess) return MFCFD_ERR_CUDA;
+        std::vector<int> chains(count);
+        int slots = 0;
+        for (int32_t i = 0; i < count; ++i) {
+            chains[i] = hs[i]->d.ch_chains;
+            slots += budget_slots(hs[i]);
+        }
         if (slots > chain_slot_capacity(dev))
             return fail(h0, MFCFD_ERR_UNSUPPORTED,
                         "the group's chain sweeps (" + std::to_string(slots) + " slots) do not fit the device (" +
                             std::to_string(chain_slot_capacity(dev)) + ")");
-        if (!chain_group_fits(dev, d0.ch_wpb, d0.precision, d0.ch_spread))
+        if (!chain_fits(dev, true))
             return fail(h, MFCFD_ERR_UNSUPPORTED, "the group sweep kernel holds fewer blocks per SM than a handle's");
         for (int32_t i = 0; i < count; ++i)
             if (!hs[i]->batch_ev && cudaEventCreateWithFlags(&hs[i]->batch_ev, cudaEventDisableTiming) != cudaSuccess)
@@ -1502,9 +1582,6 @@ int mfcfd_run_group(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
         prepare_launches(dev);
         auto G = std::make_unique<ChainGroup>();
         G->count = count;
-        G->block_start[0] = 0;
-        for (int32_t i = 0; i < count; ++i)
-            G->block_start[i + 1] = G->block_start[i] + (hs[i]->d.ch_warps + d0.ch_wpb - 1) / d0.ch_wpb;
         GroupRun gr;
         int lo = 0, hi = 0;
         CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
@@ -1518,14 +1595,24 @@ int mfcfd_run_group(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
             graphs = graphs && hs[i]->P.graphs >= 1 && !hs[i]->graphs_off;
         }
         int first_err = MFCFD_OK;
+        // the group's slots for one chunk, returned on every path
+        struct Held {
+            int dev, budget, slots;
+            ~Held() { give_slots(dev, budget, slots); }
+        };
         for (int32_t done = 0; done < iters;) {
-            const int chunk = std::min<int32_t>(iters - done, res_cap);
+            const Held held{dev, slots, take_slots(dev, chains.data(), count, d0.precision, h0->P.chain_spread, slots,
+                                                   1 << 20, true, &gr.shape)};
+            G->block_start[0] = 0;
+            for (int32_t i = 0; i < count; ++i)
+                G->block_start[i + 1] = G->block_start[i] + chain_blocks(chains[i], gr.shape);
+            const int chunk = std::min<int32_t>(iters - done, held.slots > slots ? std::min(res_cap, EXCESS_CHUNK) : res_cap);
             for (int32_t i = 0; i < count; ++i) hs[i]->res_valid = false;
             std::vector<int> cur(count), last(count);
             for (int32_t i = 0; i < count; ++i) cur[i] = hs[i]->cur, last[i] = hs[i]->last;
             GroupRun::Graph *g = nullptr;
             for (auto &x : gr.graphs)
-                if (x.chunk == chunk && x.cur == cur) g = &x;
+                if (x.chunk == chunk && x.cur == cur && x.shape == gr.shape) g = &x;
             if (!g && graphs) {
                 cudaGraph_t graph = nullptr;
                 cudaGraphExec_t exec = nullptr;
@@ -1539,7 +1626,7 @@ int mfcfd_run_group(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
                 if (graph) cudaGraphDestroy(graph);
                 for (int32_t i = 0; i < count; ++i) hs[i]->cur = cur[i], hs[i]->last = last[i];
                 if (e == cudaSuccess && exec) {
-                    gr.graphs.push_back({chunk, cur, exec});
+                    gr.graphs.push_back({chunk, cur, gr.shape, exec});
                     g = &gr.graphs.back();
                 } else {
                     (void)cudaGetLastError();   // launch one by one from here on
@@ -1585,12 +1672,11 @@ int mfcfd_set_chain_warps(mfcfd_handle *h, int32_t warps, int32_t *actual) {
         if (!h->staged) return fail(h, MFCFD_ERR_ARG, "handle has no device state");
         // a prepared handle: rebuild the staged schedule before it is attached
         mfcfd_handle::Staged &st = *h->staged;
-        int blocks = 0;
-        const int w = chain_shape(h->P.device, warps, h->P.chain_spread, &st.ch_wpb, &blocks);
-        if (w < 1) return fail(h, MFCFD_ERR_CUDA, "chain sweep kernel cannot be resident");
-        st.S = ChainSchedule();   // built for w at the next dry run or attach
-        st.ch_w = w;
-        if (actual) *actual = w;
+        h->ch_budget = chain_budget(h->P.device, warps, h->P.chain_spread, &h->ch_wpb);
+        if (h->ch_budget < 1) return fail(h, MFCFD_ERR_CUDA, "chain sweep kernel cannot be resident");
+        st.S = ChainSchedule();   // built for these chains at the next dry run or attach
+        st.chains = chain_count(h->P.device, h->ch_budget, h->T.max_level_width, h->P.chain_spread);
+        if (actual) *actual = h->ch_budget;
         return MFCFD_OK;
     });
 }
@@ -1618,7 +1704,7 @@ int mfcfd_tune_chain(mfcfd_handle *h, const int32_t *candidates, int32_t count, 
         double res_old = 0.0;
         int rc = mfcfd_get_state(h, prim.data(), delu.data(), &res_old);
         if (rc) return rc;
-        const int start = h->d.ch_warps;
+        const int start = h->ch_budget;
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         CK(cudaEventCreate(&e0));
         CK(cudaEventCreate(&e1));
@@ -1652,7 +1738,7 @@ int mfcfd_tune_chain(mfcfd_handle *h, const int32_t *candidates, int32_t count, 
         if (ra && rc == MFCFD_OK) rc = ra;
         const int rs = mfcfd_set_state(h, prim.data(), delu.data(), res_old);
         if (rc == MFCFD_OK) rc = rs;
-        *chosen = h->d.ch_warps;
+        *chosen = h->ch_budget;
         return rc;
     });
 }

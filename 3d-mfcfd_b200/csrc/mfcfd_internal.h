@@ -183,7 +183,6 @@ int prep_alias_gpu(int device, int n, const int32_t *nbhs, const int32_t *conn, 
 // doff[p+1]) (0-based ids); other points get -1.
 int prep_levels_gpu(int device, int n, const std::vector<int> &order, const std::vector<int32_t> &doff,
                     const std::vector<int32_t> &deps, std::vector<int32_t> &level, std::string &err);
-void build_pre_order(const Topology &T, std::vector<int32_t> &order);
 
 // Device-resident set-up (mfcfd_prep.cu; mfcfd_params.gpu_setup = 1 on a
 // handle created with its device).  Every topology array the kernels read
@@ -298,6 +297,16 @@ int build_topology(const mfcfd_params &P, int n, const int32_t *status, const do
                    const double *nor, const int32_t *nbhs, const int32_t *conn,
                    const double *min_dist, Topology &T, std::string &err);
 
+// Launch shape of a chain sweep: the warps that walk a chain together (1, 2 or
+// 4), the FP64 build for three blocks per SM instead of two, one block per SM
+// (mfcfd_params.chain_spread).
+struct ChainShape {
+    int team, dense, spread;
+};
+inline bool operator==(const ChainShape &a, const ChainShape &b) {
+    return a.team == b.team && a.dense == b.dense && a.spread == b.spread;
+}
+
 // Device-side views (plain pointers, passed to kernels by value).
 struct DevCloud {
     int n;
@@ -348,10 +357,9 @@ struct DevCloud {
     int withhold1;                // failure-detection hook: this point (1-based) publishes
                                   // none of its sweep increments; 0: off
     // chain schedule (per direction: 0 forward, 1 backward)
-    int ch_warps, ch_wpb;         // warps and warps per block
-    int ch_spread;                // one chain block per SM (mfcfd_params.chain_spread)
+    int ch_chains;                // chains (warp lists) of the schedule
+    ChainShape ch_shape;
     int flux_grid;                // blocks of the fused flux kernel; 0: one per FLUX_WARPS points
-    const int32_t *pre_order;     // all points, forward sweep order first (fused flux)
     const int32_t *ch_ptr[2], *ch_pts[2], *ch_own[2];
     const ChainItem *ch_items[2];
     const int32_t *g0_pts;        // points of the g0 blocks (Topology::g0_pts)
@@ -380,31 +388,24 @@ struct ChainGroup {
 };
 static_assert(sizeof(ChainGroup) <= 32000, "a group launch's parameters must stay within 32 KB");
 
-// Streams of one handle: the main stream (high priority) and a side stream
-// that runs the flux residual beside the chain schedule's forward sweep,
-// with the events that fork and join them.
+// A handle's stream, and the event that marks where its sweeps may start.
 struct IterStreams {
-    cudaStream_t main, side;
-    cudaEvent_t fork, join;
+    cudaStream_t main;
+    cudaEvent_t fork;
 };
 
 // kernel launchers (mfcfd_kernels.cu)
-// ev: null, or MFCFD_NPHASE+1 events recorded around the phases (ev[2] on
-// the side stream under the chain schedule).
+// ev: null, or MFCFD_NPHASE+1 events recorded around the phases (under the chain
+// schedule the flux residual's phase includes D_inv and the hand-off marks).
 // part: ITER_ALL, or (chain schedule only) ITER_PRE -- every launch before
-// the sweeps, the flux residual on the side stream ending in st.join, with
-// st.fork recorded on the main stream where the forward sweep may start --
-// and ITER_POST, the state update and residual after the backward sweep.
+// the sweeps, ending in st.fork -- and ITER_POST, the state update and
+// residual after the backward sweep.
 enum IterPart { ITER_ALL = 0, ITER_PRE = 1, ITER_POST = 2 };
 cudaError_t launch_iteration(const DevCloud &d, int iter_slot, const IterStreams &st,
                              double *U_next, double *q_next, cudaEvent_t *ev, IterPart part = ITER_ALL);
 // One chain sweep (forward or backward) of every cloud of g in one launch;
-// all the group's clouds have chain blocks of wpb warps and one precision.
-cudaError_t launch_chain_group(const ChainGroup &g, int wpb, int precision, int spread, int forward,
-                               cudaStream_t s);
-// Whether the group kernel of this shape keeps the single-cloud kernel's
-// blocks per SM (so chain_block_slots holds for it too).
-bool chain_group_fits(int device, int wpb, int precision, int spread);
+// all the group's clouds have one shape and one precision.
+cudaError_t launch_chain_group(const ChainGroup &g, const ChainShape &c, int precision, int forward, cudaStream_t s);
 cudaError_t launch_conserved_q(const DevCloud &d, cudaStream_t s);
 // rows [a, a+rows) of width w: scatter from an index-order buffer to storage
 // order (dst[perm[a+i]] = src[i]), or gather the reverse
@@ -415,20 +416,30 @@ cudaError_t launch_forces(const DevCloud &d, cudaStream_t s, double area_each, c
 int reduction_blocks(int n);
 // streaming multiprocessors of a device (cached per device)
 int device_sms(int device);
-// Launch shape of the chain sweep for about `want` warps: warps per block
-// and blocks (at most SMs - 16 blocks); returns the warps, 0 if the kernel
-// cannot run on the device.
-int chain_shape(int device, int want, int spread, int *wpb, int *blocks);
+// Warps a chain schedule may hold beside other handles' (mfcfd_info.chain_warps)
+// for about `want`, in blocks of *wpb (4, or 8 where 4-warp blocks would be
+// more than the SMs of chain_slot_capacity); 0 if the device has too few SMs.
+int chain_budget(int device, int want, int spread, int *wpb);
+// Slots of that budget.
+int chain_budget_slots(int budget, int wpb, int precision, int spread);
+// Chains of a schedule: 1.5 times the widest level (one and a half keeps every
+// level's points moving; 62k points: 6.83 ms per iteration against 6.91 with
+// twice and 6.93 with once), at most what the device holds as teams of four
+// unless that is below 0.85 times the level, and at most the budget.
+int chain_count(int device, int budget, int width, int spread);
+// Blocks and slots of a chain sweep.
+int chain_blocks(int chains, const ChainShape &c);
+int chain_slots(int chains, const ChainShape &c, int precision);
+// The largest teams with which the sweeps of these chain counts fit `slots`
+// together; teams of one (which fit their budgets) if none does.
+ChainShape chain_fit(const int *chains, int count, int precision, int spread, int slots);
+// Whether the chain kernels hold the blocks per SM that the slots count on.
+bool chain_fits(int device, bool group);
 // Per-device launch set-up (kernel attributes), done before a stream capture.
 void prepare_launches(int device);
-// Chain-sweep blocks that may run at once, in slots of a sixth of an SM: a
-// block takes 6 / (its blocks per SM, at most 3), i.e. 2 for a 4-warp block
-// of the mixed-precision sweep (three per SM), 3 for a 4-warp block of the
-// FP64 sweep, 6 for an 8-warp block; see k_sweep_chain.
+// Chain-sweep blocks that may run at once, in slots of a sixth of an SM; see
+// k_sweep_chain.
 int chain_slot_capacity(int device);
-// slots (sixths of an SM) of one chain block of the given shape and
-// precision (MFCFD_PRECISION_*)
-int chain_block_slots(int device, int wpb, int precision, int spread = 0);
 // File formats of the reference program (mfcfd_io.cpp).  Handle-less calls
 // leave their message in g_io_err (mfcfd_last_error(NULL)).
 extern thread_local std::string g_io_err;
@@ -451,6 +462,12 @@ int knn_connectivity(int device, int n, const double *x, const double *y, const 
 // the three weights first into saved[dir], 3 per term, when non-null), or
 // put the saved weights back (fold false).
 cudaError_t launch_fold_terms(const DevCloud &d, double *const saved[2], bool fold, cudaStream_t s);
+
+// mfcfd_launch holding up to `slots` slots (its budget if that is more); *held
+// (may be null) receives the slots it holds until mfcfd_complete.  With `wait`
+// false, MFCFD_ERR_BUSY instead of a wait for slots that other threads' runs
+// hold beyond their budgets.
+int launch_within(mfcfd_handle *h, int32_t t0, int32_t iters, int slots, bool wait, int *held);
 
 // Allocation-free residual (mfcfd_residual_noalloc); the current device must
 // be the handle's.

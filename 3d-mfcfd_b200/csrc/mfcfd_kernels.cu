@@ -3,12 +3,14 @@
  *
  * One iteration (fpi_solver.f90:27-36) is this launch sequence:
  *   k_qderiv      q_derivatives + timestep_delt     thread per point
- *   k_flux        eval_flux_residual                warp per point
+ *   k_flux        eval_flux_residual                warp per point; with the
+ *                 chain schedule also what follows, otherwise:
  *   k_pending     sweep hand-off words set to "not yet published"
  *   k_dinv_gold   D_inv, fluxes of prim in the shared interior frame,
  *                 flux increments of points the sweeps do not update
- *   k_sweep_chain x2  forward / backward LU-SGS sweep: static warp chains
- *                 on all SMs (k_sweep_df: dynamic topological order;
+ *   k_sweep_chain x2  forward / backward LU-SGS sweep: static chains walked
+ *                 by teams of warps on all SMs, mfcfd_chain.cuh
+ *                 (k_sweep_df: dynamic topological order;
  *                 k_sweep_levels: one CTA, level by level)
  *   k_update      state_update_implicit + next iteration's U and q
  *                 (k_update_ss: supersonic points' copies, in order)
@@ -27,6 +29,7 @@
 
 #include "mfcfd_internal.h"
 #include "mfcfd_physics.cuh"
+#include "mfcfd_publish.cuh"
 
 namespace mfcfd {
 
@@ -178,9 +181,7 @@ __global__ void __launch_bounds__(128) k_qinner(DevCloud d, const double *dq_in,
 // producer stores its values with strong (relaxed, gpu-scope) 8-byte stores;
 // a consumer polls the 8-byte words it needs with strong loads until none is
 // DU_PENDING.  Each word is single-copy atomic, so a value read that is not
-// DU_PENDING is the final one: no flags and no fences are needed.  The same
-// hand-off carries the sweep inputs (flux_res, D_inv, Gold) from k_flux<true>
-// to the forward sweep running beside it.
+// DU_PENDING is the final one: no flags and no fences are needed.
 constexpr unsigned long long DU_PENDING = 0xFFF4DEADBEEF0001ull;
 
 __device__ __forceinline__ unsigned long long ld_relaxed_b64(const double *p) {
@@ -304,15 +305,25 @@ __device__ __forceinline__ double dinv_combine(int cls, double delt, const doubl
 
 // The sweep inputs of point i computed by one warp (same arithmetic as
 // k_dinv_gold): lanes 0-5 the D_inv terms, lane (list, component) the flux
-// of prim and, for an unswept point, of prim(U + dU) in the shared frame.
-// Strong stores: the forward sweep polls for these words.  The fluxes are
-// evaluated in R; D_inv stays double.
+// of prim and, for an unswept point, of prim(U + dU) in the shared frame; a
+// swept point's hand-off words are marked DU_PENDING (see k_pending).  The
+// fluxes are evaluated in R; D_inv stays double.
 template <typename R>
 __device__ __forceinline__ void sweep_inputs_warp(const DevCloud &d, int i, int lane) {
     double p[5];
 #pragma unroll
     for (int r = 0; r < 5; ++r) p[r] = d.prim[5 * (size_t)i + r];
     const bool swept = d.swept[i] != 0;
+    if (swept) {
+        const double pend = __longlong_as_double((long long)DU_PENDING);
+        if (d.shared_frame)
+            for (int w = lane; w < DG_STRIDE; w += 32) {
+                d.dgf[DG_STRIDE * (size_t)i + w] = pend;
+                d.dgb[DG_STRIDE * (size_t)i + w] = pend;
+            }
+        if (lane < 5) d.dUp[5 * (size_t)i + lane] = pend;
+        else if (lane < 10) d.dUn[5 * (size_t)i + lane - 5] = pend;
+    }
     if (swept && d.cls[i] <= CLS_WALL) {   // D_inv of wall and interior points
         const double as = sqrt(1.40 * p[4] / p[0]);
         const double u = (lane >> 1) == 0 ? p[1] : ((lane >> 1) == 1 ? p[2] : p[3]);
@@ -320,7 +331,7 @@ __device__ __forceinline__ void sweep_inputs_warp(const DevCloud &d, int i, int 
         double gd[NDIR];
 #pragma unroll
         for (int dd = 0; dd < NDIR; ++dd) gd[dd] = __shfl_sync(FULL, t, dd);
-        if (lane == 0) st_relaxed_f64(d.dinv + i, dinv_combine(d.cls[i], d.delt[i], gd));
+        if (lane == 0) d.dinv[i] = dinv_combine(d.cls[i], d.delt[i], gd);
     } else if (swept && d.cls[i] == CLS_OUTER) {      // backup driver
         const double as = sqrt(1.40 * p[4] / p[0]);
         const double u = lane < 2 ? p[1] : (lane < 4 ? p[2] : p[3]);
@@ -328,7 +339,7 @@ __device__ __forceinline__ void sweep_inputs_warp(const DevCloud &d, int i, int 
         double g5[5];
 #pragma unroll
         for (int dd = 0; dd < 5; ++dd) g5[dd] = __shfl_sync(FULL, t, dd);
-        if (lane == 0) st_relaxed_f64(d.dinv + i, dinv_outer(d, i, g5));
+        if (lane == 0) d.dinv[i] = dinv_outer(d, i, g5);
     }
     if (d.shared_frame && lane < 30) {
         const int dd = lane / 5, c = lane - 5 * dd;
@@ -342,7 +353,7 @@ __device__ __forceinline__ void sweep_inputs_warp(const DevCloud &d, int i, int 
         AxisTermsT<R> At;
         axis_terms(P, dd >> 1, At);
         const R gold = flux_component(dd, c, P, At, At, At);
-        st_relaxed_f64(d.gold + 30 * (size_t)i + lane, (double)gold);
+        d.gold[30 * (size_t)i + lane] = (double)gold;
         if (!swept) {
             R U[5], pn[5];
             FrameT<R> F;
@@ -354,8 +365,8 @@ __device__ __forceinline__ void sweep_inputs_warp(const DevCloud &d, int i, int 
             axis_terms(P, dd >> 1, At);
             const double v = (double)(flux_component(dd, c, P, At, At, At) - gold);
             const size_t o = DG_STRIDE * (size_t)i + DG_LIST * dd + c;
-            st_relaxed_f64(d.dgf + o, v);
-            st_relaxed_f64(d.dgb + o, v);
+            d.dgf[o] = v;
+            d.dgb[o] = v;
         }
         if (d.dg_old) {   // backup driver: the increment from before the sweeps
             R U[5], pn[5];
@@ -366,8 +377,7 @@ __device__ __forceinline__ void sweep_inputs_warp(const DevCloud &d, int i, int 
             conserved_to_primitive(U, F, pn);
             flux_pre(pn, F0, P);
             axis_terms(P, dd >> 1, At);
-            st_relaxed_f64(d.dg_old + DG_STRIDE * (size_t)i + DG_LIST * dd + c,
-                           (double)(flux_component(dd, c, P, At, At, At) - gold));
+            d.dg_old[DG_STRIDE * (size_t)i + DG_LIST * dd + c] = (double)(flux_component(dd, c, P, At, At, At) - gold);
         }
     }
 }
@@ -378,34 +388,26 @@ __device__ __forceinline__ void sweep_inputs_warp(const DevCloud &d, int i, int 
 // then 30 lanes (list, component) sum the list terms in list order and solve
 // the 3x3 least-squares system with the precomputed moments.
 //
-// FUSED (chain schedule): the warps take the points in the forward sweep's
-// order (d.pre_order) and also produce the point's sweep inputs (D_inv,
-// fluxes of prim in the shared frame, the fixed increment of an unswept
-// point) with strong stores, while the forward sweep runs concurrently and
-// polls for them (they start as DU_PENDING).
+// FUSED (chain schedule): the warps also produce the points' sweep inputs
+// (D_inv, fluxes of prim in the shared frame, the fixed increment of an
+// unswept point) and mark the hand-off words.
 //
 // R: the type of the reconstruction, limiter and flux arithmetic (float in
 // mixed precision); the offsets, weights, list sums and 3x3 solves are double.
 // RS: the type of the sweep inputs' fluxes (float whenever the sweeps run in
 // FP32, so that a sweep differences fluxes evaluated the same way).
 // Blocks of the flux kernel per SM the compiler must fit: four for the FP64
-// evaluation (128 registers, 16 warps per SM).  Beside the forward sweep it
-// then keeps ahead of the sweep, which otherwise polled for inputs not yet
-// written (1.1M points: flux 22.1 against 26.5 ms, iteration 53.0 against
-// 55.1 ms with the earlier remedy, a lead launch of the order's first 16%).
-// FP32 keeps the default: it is well ahead anyway.
+// evaluation (128 registers, 16 warps per SM).
 template <typename R>
 constexpr int flux_min_blocks() { return sizeof(R) == 8 ? 4 : 1; }
 
 template <bool FUSED, typename R, typename RS = R>
-__global__ void __launch_bounds__(FLUX_WARPS * 32, flux_min_blocks<R>()) k_flux(DevCloud d, int i0, int i1) {
+__global__ void __launch_bounds__(FLUX_WARPS * 32, flux_min_blocks<R>()) k_flux(DevCloud d) {
     extern __shared__ double smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double *T = smem + warp * FLUX_SMEM_PER_WARP;     // T[(dir*32 + slot)*5 + c]
     double *W = T + NDIR * MAX_SLOTS * 5;             // W[slot*3 + axis]
-    // positions [i0, i1) of the visiting order (pre_order when FUSED)
-    for (int i = i0 + blockIdx.x * FLUX_WARPS + warp; i < i1; i += gridDim.x * FLUX_WARPS) {
-        const int p = FUSED ? d.pre_order[i] : i;
+    for (int p = blockIdx.x * FLUX_WARPS + warp; p < d.n; p += gridDim.x * FLUX_WARPS) {
         const int cls = d.cls[p];
         if (cls <= 2) {
             const int ns = d.nslot[p];
@@ -480,8 +482,7 @@ __global__ void __launch_bounds__(FLUX_WARPS * 32, flux_min_blocks<R>()) k_flux(
                 if (cls == CLS_INTERIOR) r = gd[0] + gd[1] + gd[2] + gd[3] + gd[4] + gd[5];
                 else if (cls == CLS_WALL) r = 2.0 * (gd[0] + gd[1] + gd[2] + gd[3] + gd[5]);
                 else r = gd[0] + gd[1] + gd[2] + gd[3] + gd[4];
-                if (FUSED) st_relaxed_f64(d.flux_res + 5 * (size_t)p + lane, r);
-                else d.flux_res[5 * (size_t)p + lane] = r;
+                d.flux_res[5 * (size_t)p + lane] = r;
             }
         }
         if (FUSED) sweep_inputs_warp<RS>(d, p, lane);
@@ -507,33 +508,23 @@ __device__ __forceinline__ void flux6_frame0(const DevCloud &d, const double pri
         for (int c = 0; c < 5; ++c) out[dd * 5 + c] = flux_component(dd, c, P, A);
 }
 
-// Before the sweeps: every published-increment word, and dU of every swept
-// point, is set to DU_PENDING (coalesced grid-stride fill).  With inputs set,
-// also the swept points' flux_res, D_inv and Gold, which k_flux<true>
-// produces while the forward sweep runs.
-__global__ void k_pending(DevCloud d, int inputs) {
+// Before the sweeps (level and dataflow schedules): every published-increment
+// word, and dU of every swept point, is set to DU_PENDING (coalesced
+// grid-stride fill).
+__global__ void k_pending(DevCloud d) {
     const double pend = __longlong_as_double((long long)DU_PENDING);
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t ng = (size_t)d.n * DG_STRIDE, nu = (size_t)d.n * 5, n30 = (size_t)d.n * 30;
+    const size_t ng = (size_t)d.n * DG_STRIDE, nu = (size_t)d.n * 5;
     for (size_t w = t0; w < ng; w += stride) {
         d.dgf[w] = pend;
         d.dgb[w] = pend;
-        if (inputs && d.dg_old) d.dg_old[w] = pend;   // produced beside the forward sweep
     }
     for (size_t w = t0; w < nu; w += stride) {
         if (d.swept[w / 5]) {
             d.dUp[w] = pend;
             d.dUn[w] = pend;
-            if (inputs && (d.cls[w / 5] <= CLS_WALL || d.cls[w / 5] == CLS_OUTER)) d.flux_res[w] = pend;
         }
-    }
-    if (inputs) {
-        for (size_t w = t0; w < (size_t)d.n; w += stride)
-            if (d.swept[w] && (d.cls[w] <= CLS_WALL || d.cls[w] == CLS_OUTER)) d.dinv[w] = pend;
-        if (d.shared_frame)
-            for (size_t w = t0; w < n30; w += stride)
-                if (d.swept[w / 30]) d.gold[w] = pend;
     }
 }
 
@@ -620,17 +611,15 @@ struct __align__(16) SweepStage {
     int32_t pad[2];
 };
 constexpr int SW_T_DOUBLES = NDIR * MAX_SLOTS * 5;                  // term fluxes, >= SWEEP_MAX_ENTRIES * 5
-constexpr int SW_RING_DOUBLES = CHAIN_RING * 30;                    // chain: last published increments
 constexpr int SWEEP_SMEM_BYTES = SW_T_DOUBLES * 8 + (int)sizeof(SweepStage);   // one stage
-constexpr int CHAIN_SMEM_BYTES = (SW_T_DOUBLES + SW_RING_DOUBLES) * 8 + 2 * (int)sizeof(SweepStage);
 static_assert(SW_T_DOUBLES >= SWEEP_MAX_ENTRIES * 5, "T buffer too small");
 static_assert(SW_T_DOUBLES * 8 >= SWEEP_MAX_ENTRIES * 5 * 8 + SWEEP_MAX_ENTRIES, "no room for the terms' flags");
 static_assert(SW_T_DOUBLES == G0_DOUBLES && G0_DOUBLES % 2 == 0, "a g0 block is one T buffer of 16-byte pairs");
 static_assert(SWEEP_MAX_ENTRIES <= 96, "entries are polled in three passes of 32");
-static_assert(sizeof(SweepStage) % 16 == 0 && SWEEP_SMEM_BYTES % 16 == 0 && CHAIN_SMEM_BYTES % 16 == 0,
+static_assert(sizeof(SweepStage) % 16 == 0 && SWEEP_SMEM_BYTES % 16 == 0,
               "stage alignment");
 
-enum SweepMode { MODE_LEVELS = 0, MODE_DATAFLOW = 1, MODE_CHAINS = 2 };
+enum SweepMode { MODE_LEVELS = 0, MODE_DATAFLOW = 1 };
 
 __device__ __forceinline__ void cp_async16(void *s, const void *g) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(s)),
@@ -755,26 +744,9 @@ __global__ void __launch_bounds__(128) k_g0(DevCloud d) {
 // G(prim_k)).  Phase C: sum each list in list order (30 lanes: list x
 // component), solve the 3x3 systems, update dU and publish this point's own
 // flux increment.
-//
-// The chain schedule reads increments that this warp published within its
-// last CHAIN_RING points from `ring` (slot in the term's ENT_RING bits) and
-// writes its own to ring slot `ring_slot`; a point publishes to global memory
-// only if some consumer reads it there (CI_PUBLISH).
-//
-// R: the type of the flux evaluations (float in mixed precision); the list
-// sums, 3x3 solves, D_inv and the increments themselves are double.
-//
-// A CI_G0 point's phase A is a copy of its k_g0 block into T, which the
-// chain kernel issued as a cp.async group before this call (followed by one
-// more group, the next point's stage, when g0_newer); phase B waits for it.
-// FOLD (mixed precision): each term's weight carries its list's 3x3 solve
-// (folded when the handle is attached), so phase C sums weight x term;
-// otherwise phase C sums
-// the three weighted moments in FP64 and solves, as the reference does.
-template <int MODE, typename R, bool FOLD = false>
+template <int MODE, typename R>
 __device__ void sweep_point(const DevCloud &d, const ChainItem &it, const SweepStage *st, bool forward, int lane,
-                            double *T, double *ring, int ring_slot, bool g0_newer = false) {
-    constexpr bool CHAINS = MODE == MODE_CHAINS;
+                            double *T) {
     const int p = it.p;
     const bool wall = (it.info & CI_WALL) != 0;
     const bool shared = (it.info & CI_SHARED) != 0;
@@ -832,15 +804,14 @@ __device__ void sweep_point(const DevCloud &d, const ChainItem &it, const SweepS
             if (!hold) st_relaxed_f64(dst, dnew);
         }
     } else {
-        double sx = 0.0, sy = 0.0, sz = 0.0, G0acc = 0.0;   // phase C's list sums
+        double sx = 0.0, sy = 0.0, sz = 0.0;   // phase C's list sums
         const uint32_t need = shared ? 0u : st->need;
         const bool mine = !shared && (need >> lane) & 1u;
-        const bool g0 = CHAINS && (it.info & CI_G0) != 0;   // warp-uniform
         int k_slot = 0, mask_slot = 0;
         if (mine) {
             k_slot = st->slot_nbr[lane];
             mask_slot = st->slot_mask[lane];
-            if (!g0) neighbour_fluxes<R>(d, cls, Fp, k_slot, mask_slot, lane, T);
+            neighbour_fluxes<R>(d, cls, Fp, k_slot, mask_slot, lane, T);
         }
 
         // ---- phase B
@@ -861,16 +832,8 @@ __device__ void sweep_point(const DevCloud &d, const ChainItem &it, const SweepS
             for (int q = 0; q < 3; ++q) {
                 const int j = lane + 32 * q;
                 if (j >= total) continue;
-                const int pad = E[j].pad;
-                if (CHAINS && (pad & ENT_RING)) {
-                    const double *rs = ring + 30 * ((pad >> ENT_RING_SHIFT) & 15) + 5 * (pad & 255);
-#pragma unroll
-                    for (int cc = 0; cc < 5; ++cc) T[j * 5 + cc] = rs[cc];
-                    rdy[j] = 1;
-                } else {
-                    pend |= 1u << q;
-                    rdy[j] = 0;
-                }
+                pend |= 1u << q;
+                rdy[j] = 0;
             }
             int spins = 0;
             for (;;) {
@@ -909,13 +872,9 @@ __device__ void sweep_point(const DevCloud &d, const ChainItem &it, const SweepS
                 if (lane < 30) {
                     while (pos < hi && rdy[pos]) {
                         const double t = T[pos * 5 + c];
-                        if constexpr (FOLD) {
-                            G0acc = G0acc + t * E[pos].w[0];
-                        } else {
-                            sx = sx + t * E[pos].w[0];
-                            sy = sy + t * E[pos].w[1];
-                            sz = sz + t * E[pos].w[2];
-                        }
+                        sx = sx + t * E[pos].w[0];
+                        sy = sy + t * E[pos].w[1];
+                        sz = sz + t * E[pos].w[2];
                         ++pos;
                     }
                 }
@@ -948,12 +907,6 @@ __device__ void sweep_point(const DevCloud &d, const ChainItem &it, const SweepS
                 for (int a = 0; a < 3; ++a)
                     if (axes & (1 << a)) axis_terms(Pn, a, An[a]);
             }
-            if (g0) {
-                // the copied phase-A fluxes: every lane's copies have landed
-                if (g0_newer) cp_async_wait_one();
-                else cp_async_wait_all();
-                __syncwarp();
-            }
             if (mine) {
                 for (int e = 0; e < NDIR; ++e) {
                     if (!(mask_slot & (1 << e))) continue;
@@ -970,31 +923,18 @@ __device__ void sweep_point(const DevCloud &d, const ChainItem &it, const SweepS
 
         // ---- phase C (from pos: the terms not yet summed)
         double G = 0.0;
-        if constexpr (FOLD) {
-            // mixed precision: each term's weight already carries the list's
-            // 3x3 solve (cofactors / det, FP64, computed at set-up)
-            G = G0acc;
-            if (lane < 30) {
+        if (lane < 30) {
+            // unrolled so the next terms' shared-memory loads overlap; the
+            // additions keep their order
 #pragma unroll 4
-                for (int jj = pos; jj < hi; ++jj) {
-                    const double t = shared ? T[jj * 5 + c] : T[(dd * MAX_SLOTS + ((E[jj].pad >> 8) & 255)) * 5 + c];
-                    G = G + t * E[jj].w[0];
-                }
+            for (int jj = pos; jj < hi; ++jj) {
+                const double t = shared ? T[jj * 5 + c] : T[(dd * MAX_SLOTS + ((E[jj].pad >> 8) & 255)) * 5 + c];
+                sx = sx + t * E[jj].w[0];
+                sy = sy + t * E[jj].w[1];
+                sz = sz + t * E[jj].w[2];
             }
-        } else {
-            if (lane < 30) {
-                // unrolled so the next terms' shared-memory loads overlap; the
-                // additions keep their order
-#pragma unroll 4
-                for (int jj = pos; jj < hi; ++jj) {
-                    const double t = shared ? T[jj * 5 + c] : T[(dd * MAX_SLOTS + ((E[jj].pad >> 8) & 255)) * 5 + c];
-                    sx = sx + t * E[jj].w[0];
-                    sy = sy + t * E[jj].w[1];
-                    sz = sz + t * E[jj].w[2];
-                }
-            }
-            if (lane < 30) G = cramer_num(dd >> 1, g, sx, sy, sz) / g[6];
         }
+        if (lane < 30) G = cramer_num(dd >> 1, g, sx, sy, sz) / g[6];
         double gd[NDIR];
 #pragma unroll
         for (int e = 0; e < NDIR; ++e) gd[e] = __shfl_sync(FULL, G, e * 5 + (lane % 5));
@@ -1028,7 +968,6 @@ __device__ void sweep_point(const DevCloud &d, const ChainItem &it, const SweepS
             const double v = (double)(flux_component(dd, c, P, At, At, At) - (R)gold);
             if ((it.info & CI_PUBLISH) && !hold)
                 st_relaxed_f64((forward ? d.dgf : d.dgb) + DG_STRIDE * (size_t)p + DG_LIST * dd + c, v);
-            if (CHAINS) ring[30 * ring_slot + lane] = v;
         }
     }
     __syncwarp();
@@ -1044,7 +983,7 @@ __device__ __forceinline__ void sweep_point_sync(const DevCloud &d, int p, bool 
     cp_async_commit();
     cp_async_wait_all();
     __syncwarp();
-    sweep_point<MODE, double>(d, it, st, forward, lane, T, nullptr, 0);
+    sweep_point<MODE, double>(d, it, st, forward, lane, T);
 }
 
 // Level-synchronous sweep in one CTA: the points of a level are independent
@@ -1087,76 +1026,27 @@ __global__ void __launch_bounds__(DF_WARPS * 32) k_sweep_df(DevCloud d, int forw
     }
 }
 
-// Chain sweep: each warp walks its own list of point records (fixed at
-// set-up, topological order).  The stage of the next point is copied in
-// while the current one is processed (two stage buffers).
-//
-// Residency: an SM holds three 4-warp blocks of the mixed-precision sweep
-// (71 KB of shared memory each; at most 168 registers, which the launch
-// bounds below ask for), two 4-warp blocks of the FP64 sweep (226
-// registers) or one 8-warp block; in slots of a sixth of an SM, 2, 3 or 6
-// (chain_block_slots).  The chain blocks running at once (one cloud, or the
-// handles of a batch) take at most 6 * (SMs - CH_FREE_SMS) slots.  So all of
-// them fit together, and at least CH_FREE_SMS SMs' worth of room stays
-// free for blocks of the concurrent flux kernels, whose outputs the forward
-// sweeps poll for (a flux kernel never waits, so the blocks it holds are
-// released): every poll ends.
+}  // namespace mfcfd
+
+#include "mfcfd_chain.cuh"
+
+namespace mfcfd {
+
+// Residency.  Every wait of a sweep is for a point of the same sweep, so all
+// blocks of the chain sweeps running at once have to fit the device together.
+// They are counted in slots of a sixth of an SM: a 4-warp block takes 2 in
+// mixed precision (three per SM: at most 168 registers and 76 KB of shared
+// memory), 3 in FP64 (two per SM: 234 registers, no spills), or 2 in the dense
+// FP64 build (168 registers, 20 bytes spilled), which a cloud takes whose teams
+// need more than two blocks per SM (1.1M points, 376 teams of four: 37.0 ms
+// per iteration against 41.5 as teams of two on more chains).  The sweeps at
+// once take at most 6 * (SMs - CH_FREE_SMS) slots; the other SMs' room is for
+// the kernels of other handles between their sweeps.
 constexpr int CH_FREE_SMS = 16;
 
-template <int WPB, bool FOLD>
-constexpr int chain_min_blocks() {
-    return (WPB == 4 && FOLD) ? 3 : 1;
-}
-
-// One block of a cloud's chain sweep: block `block` of the cloud's
-// (ch_warps + WPB - 1) / WPB.  R: the type of the sweep's flux evaluations;
-// FOLD: folded term weights (MFCFD_PRECISION_MIXED and MIXED_DC).  FP64
-// <double, false>; mixed and defect correction <float, true>.
-template <int WPB, typename R, bool FOLD>
-__device__ __forceinline__ void chain_sweep(const DevCloud &d, int forward, int block) {
-    extern __shared__ double smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    char *smb = reinterpret_cast<char *>(smem) + warp * CHAIN_SMEM_BYTES;
-    double *T = reinterpret_cast<double *>(smb);
-    double *ring = T + SW_T_DOUBLES;
-    SweepStage *stg = reinterpret_cast<SweepStage *>(ring + SW_RING_DOUBLES);
-    const int me = block * WPB + warp;
-    if (me >= d.ch_warps) return;
-    const int dir = forward ? 0 : 1;
-    const int a = d.ch_ptr[dir][me], b = d.ch_ptr[dir][me + 1];
-    if (a >= b) return;
-    const ChainItem *items = d.ch_items[dir];
-    ChainItem cur = items[a];
-    stage_issue(d, cur, forward != 0, lane, &stg[0]);
-    cp_async_commit();
-    ChainItem nxt = a + 1 < b ? items[a + 1] : cur;
-    for (int idx = a; idx < b; ++idx) {
-        const int s = (idx - a) & 1;
-        cp_async_wait_all();
-        __syncwarp();
-        if (cur.info & CI_G0) {
-            // phase A of this point, computed before the sweep (k_g0): into T,
-            // which the previous point no longer uses
-            const char *src = reinterpret_cast<const char *>(d.g0 + (size_t)(cur.info >> CI_G0_SHIFT) * G0_DOUBLES);
-            char *dst = reinterpret_cast<char *>(T);
-            for (int j = lane; j < G0_DOUBLES / 2; j += 32) cp_async16(dst + 16 * j, src + 16 * j);
-            cp_async_commit();
-        }
-        if (idx + 1 < b) {
-            stage_issue(d, nxt, forward != 0, lane, &stg[s ^ 1]);
-            cp_async_commit();
-        }
-        const ChainItem after = idx + 2 < b ? items[idx + 2] : nxt;
-        sweep_point<MODE_CHAINS, R, FOLD>(d, cur, &stg[s], forward != 0, lane, T, ring, (idx - a) % CHAIN_RING,
-                                          idx + 1 < b);
-        cur = nxt;
-        nxt = after;
-    }
-}
-
-template <int WPB, typename R, bool FOLD>
-__global__ void __launch_bounds__(WPB * 32, chain_min_blocks<WPB, FOLD>()) k_sweep_chain(DevCloud d, int forward) {
-    chain_sweep<WPB, R, FOLD>(d, forward, blockIdx.x);
+template <typename R, bool FOLD, bool DENSE>
+__global__ void __launch_bounds__(CH_WPB * 32, DENSE ? 3 : 2) k_sweep_chain(const __grid_constant__ DevCloud d, int forward) {
+    chain_sweep<R, FOLD>(d, forward, blockIdx.x);
 }
 
 // The chain sweeps of a group of clouds in one launch: blocks
@@ -1164,31 +1054,26 @@ __global__ void __launch_bounds__(WPB * 32, chain_min_blocks<WPB, FOLD>()) k_swe
 // nothing; a block finds its cloud and runs that cloud's schedule as the
 // single-cloud kernel would.  The group lives in the launch's parameters, so
 // every block reads its cloud's pointers from the constant bank.
-template <int WPB, typename R, bool FOLD>
-__global__ void __launch_bounds__(WPB * 32, chain_min_blocks<WPB, FOLD>())
+template <typename R, bool FOLD, bool DENSE>
+__global__ void __launch_bounds__(CH_WPB * 32, DENSE ? 3 : 2)
     k_sweep_chain_group(const __grid_constant__ ChainGroup g, int forward) {
     int c = 0;
     while (c + 1 < g.count && (int)blockIdx.x >= g.block_start[c + 1]) ++c;
-    chain_sweep<WPB, R, FOLD>(g.cloud[c], forward, (int)blockIdx.x - g.block_start[c]);
+    chain_sweep<R, FOLD>(g.cloud[c], forward, (int)blockIdx.x - g.block_start[c]);
 }
 
-template <int WPB>
-static int chain_smem() {
-    return WPB * CHAIN_SMEM_BYTES;
-}
-// three 4-warp blocks per SM: 228 KB of shared memory, 1 KB of it reserved per block
-static_assert(3 * (4 * CHAIN_SMEM_BYTES + 1024) <= 228 * 1024, "three 4-warp chain blocks per SM");
+// three blocks per SM: 228 KB of shared memory, 1 KB of it reserved per block
+static_assert(3 * (chain_smem_bytes(1) + 1024) <= 228 * 1024 && 3 * (chain_smem_bytes(2) + 1024) <= 228 * 1024 &&
+                  3 * (chain_smem_bytes(4) + 1024) <= 228 * 1024,
+              "three chain blocks per SM");
 // A spread chain block asks for this much shared memory, so that no second
 // block fits beside it (2 x (116 + 1) KB > 228 KB) and each of its four
 // warps has one of the SM's four sub-partitions to itself.
 constexpr int CHAIN_SPREAD_SMEM = 116 * 1024;
-static_assert(2 * (CHAIN_SPREAD_SMEM + 1024) > 228 * 1024 && CHAIN_SPREAD_SMEM >= 4 * CHAIN_SMEM_BYTES,
+static_assert(2 * (CHAIN_SPREAD_SMEM + 1024) > 228 * 1024 && CHAIN_SPREAD_SMEM >= chain_smem_bytes(2),
               "a spread block holds its SM alone");
 
-static int chain_smem_bytes(int wpb, int spread) {
-    if (wpb == 4) return spread ? CHAIN_SPREAD_SMEM : chain_smem<4>();
-    return chain_smem<8>();
-}
+static int chain_smem(const ChainShape &c) { return c.spread ? CHAIN_SPREAD_SMEM : chain_smem_bytes(c.team); }
 
 // ---------------------------------------------------------------- state update
 
@@ -1478,123 +1363,104 @@ static void set_attributes(int device) {
     cudaFuncSetAttribute(k_sweep_levels, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          SWEEP_WARPS * SWEEP_SMEM_BYTES);
     cudaFuncSetAttribute(k_sweep_df, cudaFuncAttributeMaxDynamicSharedMemorySize, DF_WARPS * SWEEP_SMEM_BYTES);
-    // three 4-warp blocks of the mixed-precision sweep per SM need the largest
-    // shared-memory carveout; the other variants leave the choice to the
-    // driver, which keeps more L1 for their loads and the flux kernel's
-    cudaFuncSetAttribute(k_sweep_chain<4, float, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(k_sweep_chain<4, double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN_SPREAD_SMEM);
-    cudaFuncSetAttribute(k_sweep_chain<8, double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, chain_smem<8>());
-    cudaFuncSetAttribute(k_sweep_chain<4, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN_SPREAD_SMEM);
-    cudaFuncSetAttribute(k_sweep_chain<8, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, chain_smem<8>());
-    cudaFuncSetAttribute(k_sweep_chain_group<4, float, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(k_sweep_chain_group<4, double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         CHAIN_SPREAD_SMEM);
-    cudaFuncSetAttribute(k_sweep_chain_group<8, double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         chain_smem<8>());
-    cudaFuncSetAttribute(k_sweep_chain_group<4, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         CHAIN_SPREAD_SMEM);
-    cudaFuncSetAttribute(k_sweep_chain_group<8, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         chain_smem<8>());
+    // the chain blocks need the largest shared-memory carveout
+    auto chain = [](auto *kern) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN_SPREAD_SMEM);
+    };
+    chain(k_sweep_chain<double, false, false>);
+    chain(k_sweep_chain<double, false, true>);
+    chain(k_sweep_chain<float, true, true>);
+    chain(k_sweep_chain_group<double, false, false>);
+    chain(k_sweep_chain_group<double, false, true>);
+    chain(k_sweep_chain_group<float, true, true>);
     done[device] = true;
 }
 
 void prepare_launches(int device) { set_attributes(device); }
 
-int chain_slot_capacity(int device) {
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    return 6 * (sms - CH_FREE_SMS);
-}
+static int chain_sms(int device) { return device_sms(device) - CH_FREE_SMS; }
 
-int chain_block_slots(int device, int wpb, int precision, int spread) {
+int chain_slot_capacity(int device) { return 6 * chain_sms(device); }
+
+bool chain_fits(int device, bool group) {
     static std::mutex mu;
-    static int cache[256][2][3] = {};
-    if (device < 0 || device >= 256 || spread) return 6;
-    const int w8 = wpb == 8 ? 1 : 0, m = precision < 0 || precision > 2 ? 0 : precision;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (cache[device][w8][m]) return cache[device][w8][m];
-    }
-    set_attributes(device);
-    int per_sm = 0;
-    cudaError_t e;
-    if (w8)
-        e = m != 0 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_chain<8, float, true>, 256, chain_smem<8>())
-                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_chain<8, double, false>, 256, chain_smem<8>());
-    else
-        e = m != 0 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_chain<4, float, true>, 128, chain_smem<4>())
-                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_chain<4, double, false>, 128, chain_smem<4>());
-    if (e != cudaSuccess) {
-        (void)cudaGetLastError();
-        per_sm = 1;
-    }
-    per_sm = per_sm < 1 ? 1 : (per_sm > 3 ? 3 : per_sm);
+    static int known[256][2] = {};                   // 0: not asked yet, 1: no, 2: yes
+    if (device < 0 || device >= 256) return false;
     std::lock_guard<std::mutex> lock(mu);
-    return cache[device][w8][m] = 6 / per_sm;
-}
-
-bool chain_group_fits(int device, int wpb, int precision, int spread) {
+    int &k = known[device][group ? 1 : 0];
+    if (k) return k == 2;
     set_attributes(device);
-    const bool mixed = precision != MFCFD_PRECISION_FP64;
-    const int smem = chain_smem_bytes(wpb, spread);
-    int one = 0, group = 0;
-    cudaError_t e1, e2;
-    if (wpb == 8) {
-        e1 = mixed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, k_sweep_chain<8, float, true>, 256, smem)
-                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, k_sweep_chain<8, double, false>, 256, smem);
-        e2 = mixed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&group, k_sweep_chain_group<8, float, true>, 256, smem)
-                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&group, k_sweep_chain_group<8, double, false>, 256,
-                                                                   smem);
-    } else {
-        e1 = mixed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, k_sweep_chain<4, float, true>, 128, smem)
-                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, k_sweep_chain<4, double, false>, 128, smem);
-        e2 = mixed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&group, k_sweep_chain_group<4, float, true>, 128, smem)
-                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&group, k_sweep_chain_group<4, double, false>, 128,
-                                                                   smem);
-    }
-    if (e1 != cudaSuccess || e2 != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
-    }
-    return group >= 1 && group >= one;
-}
-
-int chain_shape(int device, int want, int spread, int *wpb, int *blocks) {
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    set_attributes(device);
-    const int max_blocks = sms - CH_FREE_SMS;
-    if (max_blocks < 1) return 0;
-    if (spread) {
-        // 4-warp blocks, one per SM
+    auto holds = [](auto *kern, int blocks) {
         int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_chain<4, double, false>, 4 * 32, CHAIN_SPREAD_SMEM);
-        if (per_sm < 1) return 0;
-        *wpb = 4;
-        int b = (want + 3) / 4;
-        b = b > max_blocks ? max_blocks : (b < 1 ? 1 : b);
-        *blocks = b;
-        return 4 * b;
-    }
-    *wpb = want <= 4 * max_blocks ? 4 : 8;
-    // with 8-warp blocks, three quarters of the warps: more SMs stay with the
-    // concurrent flux kernel, which then keeps ahead of the forward sweep
+        for (int team = 1; team <= CH_WPB; team *= 2) {
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, CH_WPB * 32, chain_smem_bytes(team)) !=
+                cudaSuccess) {
+                (void)cudaGetLastError();
+                return false;
+            }
+            if (per_sm < blocks) return false;
+        }
+        return true;
+    };
+    const bool fits = chain_sms(device) >= 1 &&
+                      (group ? holds(k_sweep_chain_group<double, false, false>, 2) &&
+                                   holds(k_sweep_chain_group<double, false, true>, 3) &&
+                                   holds(k_sweep_chain_group<float, true, true>, 3)
+                             : holds(k_sweep_chain<double, false, false>, 2) &&
+                                   holds(k_sweep_chain<double, false, true>, 3) &&
+                                   holds(k_sweep_chain<float, true, true>, 3));
+    k = fits ? 2 : 1;
+    return fits;
+}
+
+int chain_budget(int device, int want, int spread, int *wpb) {
+    const int max_blocks = chain_sms(device);
+    if (max_blocks < 1) return 0;
+    *wpb = spread || want <= 4 * max_blocks ? 4 : 8;
     if (*wpb == 8) want = want * 3 / 4;
-    int per_sm = 0;
-    if (*wpb == 4)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_chain<4, double, false>, 4 * 32, chain_smem<4>());
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_chain<8, double, false>, 8 * 32, chain_smem<8>());
-    if (per_sm < 1) return 0;
     int b = (want + *wpb - 1) / *wpb;
-    if (b > max_blocks) b = max_blocks;
-    if (b < 1) b = 1;
-    *blocks = b;
-    // fewer warps than one block asked for (a single-warp chain measures the
-    // per-point latency floor): the block's other warps exit at once
-    return want < *wpb ? (want < 1 ? 1 : want) : b * *wpb;
+    b = b > max_blocks ? max_blocks : (b < 1 ? 1 : b);
+    return !spread && want < *wpb ? (want < 1 ? 1 : want) : b * *wpb;
+}
+
+int chain_budget_slots(int budget, int wpb, int precision, int spread) {
+    if (wpb < 1) return 0;
+    const int each = spread || wpb == 8 ? 6 : (precision != MFCFD_PRECISION_FP64 ? 2 : 3);
+    return (budget + wpb - 1) / wpb * each;
+}
+
+int chain_count(int device, int budget, int width, int spread) {
+    if (spread) return budget;
+    int c = 3 * width / 2;
+    const int most = 3 * chain_sms(device);          // teams of four the device holds
+    if (c > most && 20 * most >= 17 * width) c = most;
+    c = c < budget ? c : budget;
+    return c < 1 ? 1 : c;
+}
+
+int chain_blocks(int chains, const ChainShape &c) { return (chains * c.team + CH_WPB - 1) / CH_WPB; }
+
+int chain_slots(int chains, const ChainShape &c, int precision) {
+    const int each = c.spread ? 6 : (precision != MFCFD_PRECISION_FP64 || c.dense ? 2 : 3);
+    return chain_blocks(chains, c) * each;
+}
+
+ChainShape chain_fit(const int *chains, int count, int precision, int spread, int slots) {
+    ChainShape c{};
+    c.spread = spread;
+    c.team = spread ? 1 : CH_WPB;
+    for (;; c.team /= 2) {
+        for (c.dense = 0; c.dense < 2; ++c.dense) {
+            int sum = 0;
+            for (int i = 0; i < count; ++i) sum += chain_slots(chains[i], c, precision);
+            if (sum <= slots) return c;
+            if (precision != MFCFD_PRECISION_FP64) break;
+        }
+        if (c.team == 1) break;
+    }
+    c.dense = 0;
+    return c;
 }
 
 // Rows [a, a + rows) of width w between the reference's index order and
@@ -1655,16 +1521,12 @@ static cudaError_t launch_prio(void (*kern)(Args...), int grid, int block, size_
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Act>(args)...);
 }
 
-cudaError_t launch_chain_group(const ChainGroup &g, int wpb, int precision, int spread, int forward,
-                               cudaStream_t s) {
-    const int blocks = g.block_start[g.count];
-    const int csm = chain_smem_bytes(wpb, spread);
-    if (precision != MFCFD_PRECISION_FP64) {
-        if (wpb == 4) return launch_prio(k_sweep_chain_group<4, float, true>, blocks, 4 * 32, csm, s, true, g, forward);
-        return launch_prio(k_sweep_chain_group<8, float, true>, blocks, 8 * 32, csm, s, true, g, forward);
-    }
-    if (wpb == 4) return launch_prio(k_sweep_chain_group<4, double, false>, blocks, 4 * 32, csm, s, true, g, forward);
-    return launch_prio(k_sweep_chain_group<8, double, false>, blocks, 8 * 32, csm, s, true, g, forward);
+cudaError_t launch_chain_group(const ChainGroup &g, const ChainShape &c, int precision, int forward, cudaStream_t s) {
+    const int blocks = g.block_start[g.count], smem = chain_smem(c), threads = CH_WPB * 32;
+    if (precision != MFCFD_PRECISION_FP64)
+        return launch_prio(k_sweep_chain_group<float, true, true>, blocks, threads, smem, s, true, g, forward);
+    if (c.dense) return launch_prio(k_sweep_chain_group<double, false, true>, blocks, threads, smem, s, true, g, forward);
+    return launch_prio(k_sweep_chain_group<double, false, false>, blocks, threads, smem, s, true, g, forward);
 }
 
 cudaError_t launch_iteration(const DevCloud &d, int iter_slot, const IterStreams &st, double *U_next,
@@ -1685,15 +1547,12 @@ cudaError_t launch_iteration(const DevCloud &d, int iter_slot, const IterStreams
     const bool dc = d.precision == MFCFD_PRECISION_MIXED_DC;   // ... with the FP64 flux residual
     auto sweep = [&](int forward) {
         if (chains) {
-            const int blocks = (d.ch_warps + d.ch_wpb - 1) / d.ch_wpb;
-            const int csm = chain_smem_bytes(d.ch_wpb, d.ch_spread);
-            if (mixed) {   // MIXED and MIXED_DC: folded weights
-                if (d.ch_wpb == 4) launch_prio(k_sweep_chain<4, float, true>, blocks, 4 * 32, csm, s, true, d, forward);
-                else launch_prio(k_sweep_chain<8, float, true>, blocks, 8 * 32, csm, s, true, d, forward);
-            } else {
-                if (d.ch_wpb == 4) launch_prio(k_sweep_chain<4, double, false>, blocks, 4 * 32, csm, s, true, d, forward);
-                else launch_prio(k_sweep_chain<8, double, false>, blocks, 8 * 32, csm, s, true, d, forward);
-            }
+            const ChainShape &c = d.ch_shape;
+            const int blocks = chain_blocks(d.ch_chains, c), smem = chain_smem(c), threads = CH_WPB * 32;
+            // MIXED and MIXED_DC: folded weights
+            if (mixed) launch_prio(k_sweep_chain<float, true, true>, blocks, threads, smem, s, true, d, forward);
+            else if (c.dense) launch_prio(k_sweep_chain<double, false, true>, blocks, threads, smem, s, true, d, forward);
+            else launch_prio(k_sweep_chain<double, false, false>, blocks, threads, smem, s, true, d, forward);
         } else if (d.sweep_mode == MFCFD_SWEEP_LEVELS) {
             k_sweep_levels<<<1, SWEEP_THREADS, SWEEP_WARPS * SWEEP_SMEM_BYTES, s>>>(d, forward);
         } else {
@@ -1722,36 +1581,29 @@ cudaError_t launch_iteration(const DevCloud &d, int iter_slot, const IterStreams
         else k_g0<double><<<gb, 128, 0, s>>>(d);
     }
     if (chains) {
-        // the flux residual and the sweep inputs run on the side stream beside
-        // the forward sweep, in its order; the sweep polls for them.  The flux
-        // kernel is issued first: where kernels run one at a time (a profiler,
-        // blocking launches) it completes before the sweep starts, and it
-        // never waits on the sweep, so no order of execution can stall.  The
-        // main stream's higher priority places the sweep's blocks first when
-        // both run.
-        k_pending<<<sms * 8, 256, 0, s>>>(d, 1);
-        mark(3, s);
+        // the flux residual, the sweep inputs and the hand-off marks; before the
+        // sweeps, whose teams leave no room beside them (1.1M points: 37.0 ms
+        // per iteration against 39.5 to 112 with the flux residual beside the
+        // forward sweep; 62k: 7.0 against 6.9)
         const size_t fsm = FLUX_WARPS * FLUX_SMEM_PER_WARP * 8;
-        auto flux = [&](int i0, int i1, int grid, cudaStream_t on, bool high) {
-            if (dc) launch_prio(k_flux<true, double, float>, grid, FLUX_WARPS * 32, fsm, on, high, d, i0, i1);
-            else if (mixed) launch_prio(k_flux<true, float>, grid, FLUX_WARPS * 32, fsm, on, high, d, i0, i1);
-            else launch_prio(k_flux<true, double>, grid, FLUX_WARPS * 32, fsm, on, high, d, i0, i1);
-        };
-        cudaEventRecord(st.fork, s);
-        cudaStreamWaitEvent(st.side, st.fork, 0);
         // a smaller grid walks the same order with its warps striding through it
         const int fgrid = d.flux_grid > 0 && d.flux_grid < fblocks ? d.flux_grid : fblocks;
-        flux(0, n, fgrid, st.side, false);
-        mark(2, st.side);
-        cudaEventRecord(st.join, st.side);
-        if (part == ITER_PRE) return cudaGetLastError();
+        auto flux = [&](auto *kern) { launch_prio(kern, fgrid, FLUX_WARPS * 32, fsm, s, false, d); };
+        if (dc) flux(k_flux<true, double, float>);
+        else if (mixed) flux(k_flux<true, float>);
+        else flux(k_flux<true, double>);
+        mark(2, s);
+        mark(3, s);
+        if (part == ITER_PRE) {
+            cudaEventRecord(st.fork, s);
+            return cudaGetLastError();
+        }
         sweep(1);
         mark(4, s);
-        cudaStreamWaitEvent(s, st.join, 0);
     } else {
-        k_flux<false, double><<<fblocks, FLUX_WARPS * 32, FLUX_WARPS * FLUX_SMEM_PER_WARP * 8, s>>>(d, 0, n);
+        k_flux<false, double><<<fblocks, FLUX_WARPS * 32, FLUX_WARPS * FLUX_SMEM_PER_WARP * 8, s>>>(d);
         mark(2, s);
-        k_pending<<<sms * 8, 256, 0, s>>>(d, 0);
+        k_pending<<<sms * 8, 256, 0, s>>>(d);
         k_dinv_gold<<<(n + 127) / 128, 128, 0, s>>>(d);
         mark(3, s);
         sweep(1);

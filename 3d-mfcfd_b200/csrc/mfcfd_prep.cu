@@ -962,27 +962,6 @@ __global__ void k_g0_emit(int n, const int32_t *perm, const int *flag, const int
     }
 }
 
-// the fused flux kernel's visiting order: keys as build_pre_order's, sorted
-// stably (ties in storage index order)
-__global__ void k_pre_keys(int n, const uint8_t *swept, const int32_t *level, uint32_t *key, int32_t *idx) {
-    GRID_STRIDE(t, (size_t)n) {
-        key[t] = swept[t] ? 2u * (uint32_t)level[t] + 1u : 0xffffffffu;
-        idx[t] = (int32_t)t;
-    }
-}
-
-__global__ void k_pre_min(int nsw, const int32_t *order, const int32_t *off, const SweepEntry *ent,
-                          const uint8_t *swept, const int32_t *level, uint32_t *key) {
-    GRID_STRIDE(t, (size_t)nsw) {
-        const int p = order[t];
-        for (int e = off[p]; e < off[p + 1]; ++e) {
-            if (ent[e].pad & (ENT_COPY | ENT_OLD)) continue;
-            const int k = ent[e].k;
-            if (!swept[k]) atomicMin(&key[k], 2u * (uint32_t)level[p]);
-        }
-    }
-}
-
 }  // namespace
 
 #define DS_TMP(ptr, count)                                                              \
@@ -1463,20 +1442,6 @@ int device_setup(int device, const mfcfd_params &P, Topology &T, const double *x
         d.n_wall = (int)T.wall_idx.size();
     }
 
-    // ---- the fused flux kernel's visiting order (build_pre_order)
-    d.pre_order = nullptr;
-    if (chains) {
-        uint32_t *key, *key_sorted;
-        int32_t *idx, *pre;
-        DS_TMP(key, n); DS_TMP(key_sorted, n); DS_TMP(idx, n);
-        DS_KEEP(pre, n);
-        k_pre_keys<<<g, PREP_THREADS, 0, s>>>(n, swept, dt.level[0], key, idx);
-        if (nsw > 0)
-            k_pre_min<<<gs, PREP_THREADS, 0, s>>>(nsw, order[0], off_dir[0], ent_dir[0], swept, dt.level[0], key);
-        PREP_CK(cudaGetLastError());
-        if (int rc = sort_pairs(key, key_sorted, idx, pre, n, s, tmp, err)) return rc;
-        d.pre_order = pre;
-    }
     PREP_CK(cudaStreamSynchronize(s));
     return MFCFD_OK;
 }
@@ -1572,7 +1537,7 @@ int device_chain_schedule(int device, DevTopology &dt, DevCloud &d, int warps, c
         d.ch_own[dir] = down;
         d.ch_items[dir] = items;
     }
-    d.ch_warps = warps;
+    d.ch_chains = warps;
     return MFCFD_OK;
 }
 

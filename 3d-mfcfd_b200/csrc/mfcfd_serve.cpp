@@ -53,6 +53,7 @@ struct Request {
     std::string err;
     bool done = false;
     int slots = 0;                    // SM slots of its chain sweep (mfcfd_info)
+    int held = 0;                     // ... of its running chunk
     int slot_capacity = 0;            // the device's chain slots (mfcfd_info)
     bool running = false;             // a chunk is launched and not yet completed
     double t_launch = 0.0;            // server clock at its running chunk's launch
@@ -378,11 +379,16 @@ void mfcfd_server::scheduler_loop() {
             }
 
             // launches: the next chunk of every idle request whose chain sweeps
-            // fit beside the running ones (one always may run)
+            // fit beside the running ones (one always may run), with an even
+            // share of the device among the live requests for larger teams
+            int active = 0;
+            for (const RequestPtr &r : live) active += r->retiring ? 0 : 1;
             for (const RequestPtr &r : live) {
                 if (r->running || r->retiring) continue;
                 if (running > 0 && used + r->slots > capacity) continue;
-                const int rc = mfcfd_launch(r->h, r->t, chunk);
+                const int share = std::min(capacity / std::max(active, 1), capacity - used);
+                const int rc = mfcfd::launch_within(r->h, r->t, chunk, share, running == 0, &r->held);
+                if (rc == MFCFD_ERR_BUSY) continue;
                 progress = true;
                 if (rc) {
                     r->fail = rc;
@@ -392,7 +398,7 @@ void mfcfd_server::scheduler_loop() {
                 account();
                 r->running = true;
                 r->t_launch = now();
-                used += r->slots;
+                used += r->held;
                 ++running;
             }
 
@@ -406,7 +412,7 @@ void mfcfd_server::scheduler_loop() {
                 account();
                 r->res.run_s += now() - r->t_launch;
                 r->running = false;
-                used -= r->slots;
+                used -= r->held;
                 --running;
                 {
                     std::lock_guard<std::mutex> lk(mu);

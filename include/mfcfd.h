@@ -103,8 +103,10 @@ typedef struct mfcfd_params {
     int32_t sweep_mode;       /* MFCFD_SWEEP_CHAINS (default), _DATAFLOW or _LEVELS */
     int32_t update_variant;   /* MFCFD_UPDATE_IMPLICIT (default) or MFCFD_UPDATE_EXPLICIT */
     int32_t sweep_variant;    /* MFCFD_SWEEPS_ALIAS (default) or MFCFD_SWEEPS_BACKUP */
-    int32_t chain_warps;      /* CHAINS: warps of the schedule; 0 picks about twice the
-                                 widest level (fewer warps leave SMs to other clouds) */
+    int32_t chain_warps;      /* CHAINS: warps the sweep may hold beside other handles'
+                                 sweeps; 0 picks about twice the widest level (fewer
+                                 leave SMs to other clouds).  A sweep with the device to
+                                 itself takes more */
     int32_t gpu_setup;        /* 1: the set-up runs on params->device with the host's
                                  results.  mfcfd_create computes every topology array on
                                  the device (the host classifies and orders the points
@@ -120,9 +122,9 @@ typedef struct mfcfd_params {
                                  holds one, so every warp has an SM sub-partition to
                                  itself; 0 (default) packs blocks as residency allows */
     int32_t storage_order;    /* MFCFD_ORDER_MORTON (default) or MFCFD_ORDER_INDEX */
-    int32_t flux_blocks_per_sm;   /* CHAINS: the flux residual beside the forward sweep as a
-                                     grid of this many blocks per SM walking the sweep's
-                                     order; 0 (default): one block per four points */
+    int32_t flux_blocks_per_sm;   /* CHAINS: the flux residual as a grid of this many blocks
+                                     per SM walking the points; 0 (default): one block per
+                                     four points */
 } mfcfd_params;
 
 /* Order of the points in device memory.  The set-up (split lists, alias
@@ -159,10 +161,10 @@ typedef struct mfcfd_params {
  * CTA processes level after level with a block barrier between levels. */
 #define MFCFD_SWEEP_DATAFLOW  0
 #define MFCFD_SWEEP_LEVELS    1
-/* CHAINS: points are assigned to warps ahead of time so that a point usually
- * runs on the warp that processed its deepest dependency, which hands its
- * increment over in shared memory; other neighbours are polled for.  One
- * cooperative launch keeps all warps resident. */
+/* CHAINS: points are assigned to chains ahead of time so that a point usually
+ * follows its deepest dependency in its chain; a team of warps of one block
+ * walks a chain, handing increments over in shared memory, and other
+ * neighbours are polled for.  All blocks of a sweep are resident at once. */
 #define MFCFD_SWEEP_CHAINS    2
 
 typedef struct mfcfd_info {
@@ -175,22 +177,23 @@ typedef struct mfcfd_info {
     int32_t shared_frame;         /* 1 if interior points share one frame */
     int64_t device_bytes;         /* device memory held by the handle */
     int32_t sweep_mode;           /* MFCFD_SWEEP_* of the handle */
-    int32_t chain_warps;          /* CHAINS: warps of the schedule, else 0 */
+    int32_t chain_warps;          /* CHAINS: the schedule's budget of warps, else 0 */
     /* CHAINS: sweep terms (both directions) of shared-frame consumers whose
-     * producer is a swept point, by where the increment is read: the warp's
-     * shared-memory ring, global memory written by the same warp, or global
-     * memory written by another warp */
+     * producer is a swept point, by where the increment is read: the chain's
+     * shared-memory ring, global memory written by the same chain, or global
+     * memory written by another chain */
     int64_t chain_terms_ring, chain_terms_local, chain_terms_cross;
-    /* CHAINS: slots (sixths of an SM) the handle's chain sweep holds while it
-     * runs (a 4-warp block 2 in mixed precision, 3 in FP64; an 8-warp block
-     * 6), and the slots all chain sweeps running at once may hold on the
-     * device (mfcfd_launch) */
+    /* CHAINS: slots (sixths of an SM) of the handle's budget, which its chain
+     * sweep keeps to beside others' (a 4-warp block 2 in mixed precision, 3
+     * in FP64; an 8-warp block 6), and the slots all chain sweeps running at
+     * once may hold on the device (mfcfd_launch) */
     int32_t chain_slots, chain_slot_capacity;
     /* CHAINS: swept points outside the shared frame (walls) whose neighbour
      * fluxes at the start of the sweeps one extra kernel per iteration
      * computes for both sweeps; 0 when there are none or too many */
     int32_t g0_points;
-    /* CHAINS: warps per block of the chain sweep (4 or 8); handles of one
+    /* CHAINS: warps per block of the budget (4, or 8 for one of more warps than
+     * 4-warp blocks on the SMs of chain_slot_capacity); handles of one
      * mfcfd_run_group share it */
     int32_t chain_warps_per_block;
 } mfcfd_info;
@@ -453,15 +456,15 @@ int mfcfd_forces(mfcfd_handle *h, double wall_area, double ref_area, double *cl,
  * `iters` iterations (after one untimed) of each candidate warp count from
  * the current state, restores that state after each, and keeps the
  * fastest schedule.  candidates NULL with count 0 tries 1.5, 2, 3 and 4
- * times the widest sweep level (the default schedule uses 2).  *chosen
- * receives the kept schedule's warps and ms (count or 4 entries, may be
+ * times the widest sweep level (the default budget is 2).  *chosen
+ * receives the kept schedule's budget and ms (count or 4 entries, may be
  * NULL) each candidate's milliseconds per iteration.  The schedule orders
  * the work only: results are the same bits with any choice.
  */
 int mfcfd_tune_chain(mfcfd_handle *h, const int32_t *candidates, int32_t count, int32_t iters, int32_t *chosen,
                      double *ms);
-/* Rebuild the chain schedule for about `warps` warps (prepared or attached
- * handle); *actual (may be NULL) receives the schedule's warps.  In a batch,
+/* Rebuild the chain schedule for a budget of about `warps` warps (prepared or
+ * attached handle); *actual (may be NULL) receives the budget.  In a batch,
  * fewer warps per cloud (about the widest level) let more clouds share the
  * device; alone, about twice the widest level is fastest. */
 int mfcfd_set_chain_warps(mfcfd_handle *h, int32_t warps, int32_t *actual);

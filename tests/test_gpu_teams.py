@@ -1,0 +1,71 @@
+"""The chain sweep's teams against the level schedule.
+
+A handle alone sweeps with teams of up to four warps per chain; launched beside
+others it keeps to its budget (chain_warps: teams of one at 3 and 8 here, of
+two at 32).  Every budget, alone, launched and in a batch, gives the level
+schedule's bits: one chain, chains shorter than a team, more chains than points
+per level, walls and varying frames (points outside the shared frame),
+supersonic copies and the backup driver (terms from before the sweep).
+"""
+import dataclasses
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+REPO = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def _cloud(kind):
+    from mfcfd import cloud
+    c = cloud.small_sphere(6, 100, r1=1.5, seed=3)
+    if kind == "supersonic":
+        return cloud.with_supersonic_boundary(cloud.small_sphere(8, 150, seed=4))
+    if kind == "frames":
+        # one interior point with turned axes: no shared frame
+        t1, t2 = c.tan1.copy(), c.tan2.copy()
+        i = int(np.flatnonzero(c.status == 0)[5])
+        t1[i], t2[i] = (0.0, 1.0, 0.0), (-1.0, 0.0, 0.0)
+        return dataclasses.replace(c, tan1=t1, tan2=t2)
+    return c
+
+
+CASES = {"sphere": {}, "supersonic": {}, "frames": {}, "backup": {"sweep_variant": 1}}
+
+
+@pytest.mark.parametrize("case", sorted(CASES))
+@pytest.mark.parametrize("warps", [1, 3, 8, 32, 400])
+def test_team_sweeps_equal_the_level_schedule(mfcfd_lib, case, warps):
+    from mfcfd import batch
+    from mfcfd.solver import Solver
+    c = _cloud(case)
+    # the backup driver reaches NaN at outer points within a few iterations
+    iters = 1 if case == "backup" else 4
+    ss = [Solver(c, 0.5, 1.0, sweep_mode=1, **CASES[case])] + \
+         [Solver(c, 0.5, 1.0, chain_warps=warps, **CASES[case]) for _ in range(4)]
+    for s in ss:
+        s.initial_conditions()
+    ss[0].q_lskum(iters)
+    ss[1].q_lskum(iters)                       # alone: the largest team
+    ss[2].launch(1, iters)                     # within its budget
+    ss[2].complete()
+    batch.run_batch(ss[3:], iters)             # a share of the device each
+    for f in ("DELUP", "DELUN", "PRIM"):
+        want = ss[0].get(getattr(mfcfd_lib, "FIELD_" + f))
+        for s in ss[1:]:
+            assert np.array_equal(s.get(getattr(mfcfd_lib, "FIELD_" + f)).view(np.uint64), want.view(np.uint64)), f
+    for s in ss:
+        s.close()
+
+
+def test_ieee_functions_equal_the_operators(tmp_path):
+    """mfcfd_ieee.cuh against the FP64 operators (tests/ieee_check.cu): no
+    result differs."""
+    exe = str(tmp_path / "ieee_check")
+    subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-fmad=false", "-o", exe,
+                    os.path.join(REPO, "tests", "ieee_check.cu")], check=True)
+    out = subprocess.run([exe, "128"], capture_output=True, text=True)
+    assert out.returncode == 0, out.stdout + out.stderr
