@@ -808,7 +808,7 @@ int attach_state(mfcfd_handle *h) {
 #define AL(ptr, cnt) if ((rc = dalloc(h, &ptr, cnt))) return rc
     AL(d.prim, n5); AL(h->U_buf[0], n5); AL(h->U_buf[1], n5); AL(h->q_buf[0], n5);
     AL(h->q_buf[1], n5); AL(d.qm, (size_t)n * 10); AL(d.dq, (size_t)n * 15);
-    AL(d.delt, n); AL(d.flux_res, n5); AL(d.dUp, n5); AL(d.dUn, n5); AL(d.dinv, n);
+    AL(d.delt, n); AL(d.pos, (size_t)n * 4); AL(d.flux_res, n5); AL(d.dUp, n5); AL(d.dUn, n5); AL(d.dinv, n);
     AL(d.gold, (size_t)n * 30); AL(d.dgf, (size_t)n * DG_STRIDE); AL(d.dgb, (size_t)n * DG_STRIDE);
     AL(d.res_sqr, n); AL(d.partial, 1024); AL(d.res_dev, h->res_cap);
     if (P.inner_iterations > 0) AL(d.dq_tmp, (size_t)n * 15);
@@ -818,6 +818,12 @@ int attach_state(mfcfd_handle *h) {
         d.n_ss = (int)T.ss_pts.size();
         if ((rc = upload(h, &d.ss_pts, T.ss_pts))) return rc;
         if ((rc = upload(h, &d.ss_src, T.ss_src))) return rc;
+    }
+    {
+        double *qgeo = nullptr;
+        AL(qgeo, (size_t)n * QGEO_STRIDE);
+        d.qgeo = qgeo;
+        if (!h->dry) CK(launch_qgeo(d, qgeo, h->stream));
     }
     if (P.precision == MFCFD_PRECISION_MIXED_DC) {
         AL(h->w_saved[0], 3 * (size_t)std::max<int64_t>(h->n_ent[0], 1));

@@ -402,27 +402,24 @@ __device__ __forceinline__ void shared_point(const DevCloud &d, const ChainItem 
     team_leave(team, pos, lane);
 }
 
-// A slot's fluxes along the three axes, straight-line: lists 2a and 2a + 1 of
-// a slot are taken at once by selecting the sign (a wall slot on a list plane
-// is in both; the second goes in another pass).  T gets flux - T.
+// A wall or interior point's slot: its fluxes along the three axes, less what T
+// holds, into T.  The sign of each axis's list is selected, not branched on.
 template <typename R>
 __device__ __forceinline__ void slot_fluxes(bool wall, int mask, const FluxPreT<R> &P, const AxisTermsT<R> A[3], int lane,
                                             double *T) {
-    while (__any_sync(FULL, mask != 0)) {
+    for (; __any_sync(FULL, mask != 0); mask = mask_rest(mask)) {
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             const int both = (mask >> (2 * a)) & 3;
             const bool pos = (both & 1) != 0;
             R f[5];
-            axis_flux(wall && a < 2, a, pos, P, A[a], A[2], f);
+            axis_flux(wall && a < 2, a, pos, P, A[a], A[2].An, -A[2].B, f);
             double *t = T + ((2 * a + (pos ? 0 : 1)) * MAX_SLOTS + lane) * 5;
             if (both) {
 #pragma unroll
                 for (int c = 0; c < 5; ++c) t[c] = (double)(f[c] - (R)t[c]);
             }
         }
-        // each axis's first list is done
-        mask &= ~(mask & 0x15) & ~((mask & 0x2a) & ~((mask & 0x15) << 1));
     }
 }
 

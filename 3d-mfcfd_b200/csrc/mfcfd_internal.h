@@ -21,6 +21,7 @@ constexpr int MAX_CONN = 27;      // conn(27, max_points), data_structure.f90:80
 constexpr int MAX_SLOTS = 32;     // distinct neighbours a point's lists may name
 constexpr int LIST_STRIDE = 28;   // bytes per (point, list) entry table: <= 27 entries
 constexpr int GEO_STRIDE = 48;    // doubles per point: 6 lists x 8
+constexpr int QGEO_STRIDE = 8;    // doubles per point: moments of its conn
 constexpr int NDIR = 6;           // xpos, xneg, ypos, yneg, zpos, zneg
 
 // status 0, 1, 2 and 5/6 (supersonic inlet / outlet: not in any split list;
@@ -323,6 +324,7 @@ struct DevCloud {
     const int32_t *nbhs;
     const int32_t *conn;          // 27 per point, 0-based
     const double *eps2;
+    const double *qgeo;           // QGEO_STRIDE per point: moments of conn (q-derivatives), 1/det
     const double *wq, *wf;        // weights (power != 0), else null: weight 1
     const int32_t *slot_nbr;
     const uint8_t *nslot;
@@ -367,6 +369,7 @@ struct DevCloud {
     int n_g0;
     // state (Fortran layout, point-major)
     double *prim, *U, *q, *qm, *dq, *delt, *flux_res, *dUp, *dUn, *dinv;
+    double *pos;                  // 4 per point: x, y, z, signal speed of the time step
     double *dq_tmp;               // 15 per point: inner-iteration output (or null)
     double *dU_old;               // 5 per point: delUn before the sweeps (supersonic copies)
     int n_ss;                     // supersonic points (state-update copies)
@@ -406,6 +409,8 @@ cudaError_t launch_iteration(const DevCloud &d, int iter_slot, const IterStreams
 // One chain sweep (forward or backward) of every cloud of g in one launch;
 // all the group's clouds have one shape and one precision.
 cudaError_t launch_chain_group(const ChainGroup &g, const ChainShape &c, int precision, int forward, cudaStream_t s);
+// the points' moments (DevCloud::qgeo) from their coordinates, conn and weights
+cudaError_t launch_qgeo(const DevCloud &d, double *qgeo, cudaStream_t s);
 cudaError_t launch_conserved_q(const DevCloud &d, cudaStream_t s);
 // rows [a, a+rows) of width w: scatter from an index-order buffer to storage
 // order (dst[perm[a+i]] = src[i]), or gather the reverse

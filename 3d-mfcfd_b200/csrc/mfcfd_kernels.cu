@@ -42,6 +42,12 @@ constexpr unsigned FULL = 0xffffffffu;
 
 // ---------------------------------------------------------------- U and q
 
+// The speed of timestep_delt.f90:243-247 at a point: |u| + 3 sqrt(p / rho).
+__device__ __forceinline__ double signal_speed(const double p[5]) {
+    const double mod_u = sqrt(p[1] * p[1] + p[2] * p[2] + p[3] * p[3]);
+    return mod_u + 3.0 * sqrt(p[4] / p[0]);
+}
+
 // compute_conserved_vector + eval_q_variables for every point.
 __global__ void k_conserved_q(DevCloud d) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -53,6 +59,7 @@ __global__ void k_conserved_q(DevCloud d) {
     for (int r = 0; r < 5; ++r) p[r] = d.prim[5 * (size_t)i + r];
     primitive_to_rotated_conserved(p, F, U);
     primitive_to_q(p, q);
+    d.pos[4 * (size_t)i + 3] = signal_speed(p);
 #pragma unroll
     for (int r = 0; r < 5; ++r) {
         d.U[5 * (size_t)i + r] = U[r];
@@ -61,68 +68,6 @@ __global__ void k_conserved_q(DevCloud d) {
 }
 
 // ---------------------------------------------------------------- q-derivatives
-
-// eval_q_derivatives (q_derivatives.f90:25-110) and timestep_delt
-// (timestep_delt.f90:227-259), thread per point.  Weights come from d.wq
-// (power != 0); with power = 0 they are exactly 1, and delx*delx*1 and
-// 1*delx*temp round like the unweighted products.
-__global__ void __launch_bounds__(128) k_qderiv(DevCloud d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= d.n) return;
-    const double xi = d.x[i], yi = d.y[i], zi = d.z[i];
-    double qi[5], qmax[5], qmin[5];
-#pragma unroll
-    for (int r = 0; r < 5; ++r) { qi[r] = d.q[5 * (size_t)i + r]; qmax[r] = qi[r]; qmin[r] = qi[r]; }
-    double xx = 0, yy = 0, zz = 0, xy = 0, yz = 0, zx = 0;
-    double sx[5] = {0, 0, 0, 0, 0}, sy[5] = {0, 0, 0, 0, 0}, sz[5] = {0, 0, 0, 0, 0};
-    double min_delt = 1.0;
-    const int nb = d.nbhs[i];
-    const int32_t *cn = d.conn + (size_t)MAX_CONN * i;
-    for (int j = 0; j < nb; ++j) {
-        const int k = cn[j];
-        const double w = d.wq ? d.wq[(size_t)MAX_CONN * i + j] : 1.0;
-        double qk[5];
-#pragma unroll
-        for (int r = 0; r < 5; ++r) {
-            qk[r] = d.q[5 * (size_t)k + r];
-            if (qk[r] > qmax[r]) qmax[r] = qk[r];
-            if (qk[r] < qmin[r]) qmin[r] = qk[r];
-        }
-        const double delx = d.x[k] - xi, dely = d.y[k] - yi, delz = d.z[k] - zi;
-        const double dist = sqrt(delx * delx + dely * dely + delz * delz);
-        xx = xx + delx * delx * w;
-        yy = yy + dely * dely * w;
-        zz = zz + delz * delz * w;
-        xy = xy + delx * dely * w;
-        yz = yz + dely * delz * w;
-        zx = zx + delz * delx * w;
-#pragma unroll
-        for (int r = 0; r < 5; ++r) {
-            const double t = qk[r] - qi[r];
-            sx[r] = sx[r] + w * delx * t;
-            sy[r] = sy[r] + w * dely * t;
-            sz[r] = sz[r] + w * delz * t;
-        }
-        // timestep_delt.f90:235-253
-        const double *pk = d.prim + 5 * (size_t)k;
-        const double rho = pk[0], u1 = pk[1], u2 = pk[2], u3 = pk[3], pr = pk[4];
-        const double mod_u = sqrt(u1 * u1 + u2 * u2 + u3 * u3);
-        const double delt = d.cfl * dist / (mod_u + 3.0 * sqrt(pr / rho));
-        if (delt < min_delt) min_delt = delt;
-    }
-    const double g[6] = {xx, yy, zz, xy, yz, zx};
-    const double det = xx * (yy * zz - yz * yz) - xy * (xy * zz - yz * zx) + zx * (xy * yz - yy * zx);
-    const double one_by_det = 1.0 / det;
-#pragma unroll
-    for (int r = 0; r < 5; ++r) {
-        d.dq[15 * (size_t)i + 3 * r + 0] = cramer_num(0, g, sx[r], sy[r], sz[r]) * one_by_det;
-        d.dq[15 * (size_t)i + 3 * r + 1] = cramer_num(1, g, sx[r], sy[r], sz[r]) * one_by_det;
-        d.dq[15 * (size_t)i + 3 * r + 2] = cramer_num(2, g, sx[r], sy[r], sz[r]) * one_by_det;
-        d.qm[10 * (size_t)i + 2 * r + 0] = qmax[r];
-        d.qm[10 * (size_t)i + 2 * r + 1] = qmin[r];
-    }
-    d.delt[i] = min_delt;
-}
 
 // One inner iteration of the second-order q-derivatives
 // (q_derivatives.f90:116-201): least squares over conn of the differences of
@@ -303,83 +248,185 @@ __device__ __forceinline__ double dinv_combine(int cls, double delt, const doubl
     return 1.0 / temp;
 }
 
-// The sweep inputs of point i computed by one warp (same arithmetic as
-// k_dinv_gold): lanes 0-5 the D_inv terms, lane (list, component) the flux
-// of prim and, for an unswept point, of prim(U + dU) in the shared frame; a
-// swept point's hand-off words are marked DU_PENDING (see k_pending).  The
-// fluxes are evaluated in R; D_inv stays double.
+// The sweep inputs of point i (chain schedule; as k_dinv_gold): D_inv, the
+// fluxes of prim in the shared frame and, of a point the sweeps do not update,
+// the published increment G(prim(U + dU)) - G(prim).  The fluxes are evaluated
+// in R and go into gold[0..29]; D_inv is double.
 template <typename R>
-__device__ __forceinline__ void sweep_inputs_warp(const DevCloud &d, int i, int lane) {
+__device__ __forceinline__ void point_inputs(const DevCloud &d, int i, double *gold) {
     double p[5];
 #pragma unroll
     for (int r = 0; r < 5; ++r) p[r] = d.prim[5 * (size_t)i + r];
     const bool swept = d.swept[i] != 0;
-    if (swept) {
-        const double pend = __longlong_as_double((long long)DU_PENDING);
-        if (d.shared_frame)
-            for (int w = lane; w < DG_STRIDE; w += 32) {
-                d.dgf[DG_STRIDE * (size_t)i + w] = pend;
-                d.dgb[DG_STRIDE * (size_t)i + w] = pend;
-            }
-        if (lane < 5) d.dUp[5 * (size_t)i + lane] = pend;
-        else if (lane < 10) d.dUn[5 * (size_t)i + lane - 5] = pend;
-    }
-    if (swept && d.cls[i] <= CLS_WALL) {   // D_inv of wall and interior points
+    const int cls = d.cls[i];
+    if (swept && cls <= CLS_OUTER) {
         const double as = sqrt(1.40 * p[4] / p[0]);
-        const double u = (lane >> 1) == 0 ? p[1] : ((lane >> 1) == 1 ? p[2] : p[3]);
-        const double t = lane < NDIR ? dinv_term(d, i, lane, u, as) : 0.0;
         double gd[NDIR];
+        if (cls <= CLS_WALL) {
 #pragma unroll
-        for (int dd = 0; dd < NDIR; ++dd) gd[dd] = __shfl_sync(FULL, t, dd);
-        if (lane == 0) d.dinv[i] = dinv_combine(d.cls[i], d.delt[i], gd);
-    } else if (swept && d.cls[i] == CLS_OUTER) {      // backup driver
-        const double as = sqrt(1.40 * p[4] / p[0]);
-        const double u = lane < 2 ? p[1] : (lane < 4 ? p[2] : p[3]);
-        const double t = lane < 5 ? dinv_term(d, i, lane, u, as, lane == 4 ? 5 : lane) : 0.0;
-        double g5[5];
+            for (int dd = 0; dd < NDIR; ++dd) gd[dd] = dinv_term(d, i, dd, p[1 + (dd >> 1)], as);
+            d.dinv[i] = dinv_combine(cls, d.delt[i], gd);
+        } else {                                      // backup driver
 #pragma unroll
-        for (int dd = 0; dd < 5; ++dd) g5[dd] = __shfl_sync(FULL, t, dd);
-        if (lane == 0) d.dinv[i] = dinv_outer(d, i, g5);
-    }
-    if (d.shared_frame && lane < 30) {
-        const int dd = lane / 5, c = lane - 5 * dd;
-        FrameT<R> F0;
-        load_frame(d.frame0, F0);
-        R pr[5];
-#pragma unroll
-        for (int r = 0; r < 5; ++r) pr[r] = (R)p[r];
-        FluxPreT<R> P;
-        flux_pre(pr, F0, P);
-        AxisTermsT<R> At;
-        axis_terms(P, dd >> 1, At);
-        const R gold = flux_component(dd, c, P, At, At, At);
-        d.gold[30 * (size_t)i + lane] = (double)gold;
-        if (!swept) {
-            R U[5], pn[5];
-            FrameT<R> F;
-            load_frame(d.frame + 9 * (size_t)i, F);
-#pragma unroll
-            for (int r = 0; r < 5; ++r) U[r] = (R)(d.dUp[5 * (size_t)i + r] + d.U[5 * (size_t)i + r]);
-            conserved_to_primitive(U, F, pn);
-            flux_pre(pn, F0, P);
-            axis_terms(P, dd >> 1, At);
-            const double v = (double)(flux_component(dd, c, P, At, At, At) - gold);
-            const size_t o = DG_STRIDE * (size_t)i + DG_LIST * dd + c;
-            d.dgf[o] = v;
-            d.dgb[o] = v;
-        }
-        if (d.dg_old) {   // backup driver: the increment from before the sweeps
-            R U[5], pn[5];
-            FrameT<R> F;
-            load_frame(d.frame + 9 * (size_t)i, F);
-#pragma unroll
-            for (int r = 0; r < 5; ++r) U[r] = (R)(d.dU_old[5 * (size_t)i + r] + d.U[5 * (size_t)i + r]);
-            conserved_to_primitive(U, F, pn);
-            flux_pre(pn, F0, P);
-            axis_terms(P, dd >> 1, At);
-            d.dg_old[DG_STRIDE * (size_t)i + DG_LIST * dd + c] = (double)(flux_component(dd, c, P, At, At, At) - gold);
+            for (int dd = 0; dd < 5; ++dd) gd[dd] = dinv_term(d, i, dd, p[1 + (dd >> 1)], as, dd == 4 ? 5 : dd);
+            d.dinv[i] = dinv_outer(d, i, gd);
         }
     }
+    if (!d.shared_frame) return;
+    FrameT<R> F0, F;
+    load_frame(d.frame0, F0);
+    R pr[5];
+#pragma unroll
+    for (int r = 0; r < 5; ++r) pr[r] = (R)p[r];
+    FluxPreT<R> P;
+    AxisTermsT<R> A[3];
+    prim_terms(pr, F0, P, A);
+#pragma unroll
+    for (int dd = 0; dd < NDIR; ++dd) {
+        R f[5];
+        axis_flux(false, dd >> 1, (dd & 1) == 0, P, A[dd >> 1], R(0), R(0), f);
+#pragma unroll
+        for (int c = 0; c < 5; ++c) gold[5 * dd + c] = (double)f[c];
+    }
+    // increments at U + dU: of a point the sweeps leave alone, and (backup
+    // driver) of every point before the sweeps
+    for (int old = 0; old < 2; ++old) {
+        if (old ? d.dg_old == nullptr : swept) continue;
+        const double *du = (old ? d.dU_old : d.dUp) + 5 * (size_t)i;
+        R U[5];
+#pragma unroll
+        for (int r = 0; r < 5; ++r) U[r] = (R)(du[r] + d.U[5 * (size_t)i + r]);
+        load_frame(d.frame + 9 * (size_t)i, F);
+        conserved_to_primitive(U, F, pr);
+        prim_terms(pr, F0, P, A);
+        const size_t o = DG_STRIDE * (size_t)i;
+#pragma unroll
+        for (int dd = 0; dd < NDIR; ++dd) {
+            R f[5];
+            axis_flux(false, dd >> 1, (dd & 1) == 0, P, A[dd >> 1], R(0), R(0), f);
+#pragma unroll
+            for (int c = 0; c < 5; ++c) {
+                const double v = (double)(f[c] - (R)gold[5 * dd + c]);
+                if (old) d.dg_old[o + DG_LIST * dd + c] = v;
+                else d.dgf[o + DG_LIST * dd + c] = d.dgb[o + DG_LIST * dd + c] = v;
+            }
+        }
+    }
+}
+
+// Least-squares moments of every point's conn (q_derivatives.f90:44-90), which
+// do not change over a run: xx, yy, zz, xy, yz, zx, 1/det into d.qgeo when the
+// handle is attached.  Weights come from d.wq (power != 0); with power = 0
+// they are exactly 1, and delx*delx*1 rounds like the unweighted product.
+// Also the points' coordinates into d.pos, where a neighbour's x, y, z and
+// signal speed share one 32-byte sector.
+__global__ void k_qgeo(DevCloud d, double *qgeo) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= d.n) return;
+    const double xi = d.x[i], yi = d.y[i], zi = d.z[i];
+    d.pos[4 * (size_t)i + 0] = xi;
+    d.pos[4 * (size_t)i + 1] = yi;
+    d.pos[4 * (size_t)i + 2] = zi;
+    double xx = 0, yy = 0, zz = 0, xy = 0, yz = 0, zx = 0;
+    const int nb = d.nbhs[i];
+    for (int j = 0; j < nb; ++j) {
+        const int k = d.conn[(size_t)MAX_CONN * i + j];
+        const double w = d.wq ? d.wq[(size_t)MAX_CONN * i + j] : 1.0;
+        const double delx = d.x[k] - xi, dely = d.y[k] - yi, delz = d.z[k] - zi;
+        xx = xx + delx * delx * w;
+        yy = yy + dely * dely * w;
+        zz = zz + delz * delz * w;
+        xy = xy + delx * dely * w;
+        yz = yz + dely * delz * w;
+        zx = zx + delz * delx * w;
+    }
+    const double det = xx * (yy * zz - yz * yz) - xy * (xy * zz - yz * zx) + zx * (xy * yz - yy * zx);
+    double *g = qgeo + QGEO_STRIDE * (size_t)i;
+    g[0] = xx;
+    g[1] = yy;
+    g[2] = zz;
+    g[3] = xy;
+    g[4] = yz;
+    g[5] = zx;
+    g[6] = 1.0 / det;
+    g[7] = 0.0;
+}
+
+// eval_q_derivatives (q_derivatives.f90:25-110) and timestep_delt
+// (timestep_delt.f90:227-259): five lanes per point, one per component of q,
+// six points per warp.  What bounds it is the latency of the neighbours'
+// gathers, so each lane has QD_BATCH neighbours' loads in flight.  The time
+// step's neighbours are dealt out over the five lanes (a minimum does not
+// depend on its order; a neighbour's signal speed was evaluated with its
+// state, k_update).  600 points: 12 us against 32 with a thread per point and
+// every neighbour's square roots; 62,400: 46 against 56; 1.1M: 0.60 against
+// 0.67 ms.
+constexpr int QD_THREADS = 128, QD_POINTS = QD_THREADS / 32 * 6, QD_BATCH = 5;
+__global__ void __launch_bounds__(QD_THREADS) k_qderiv(const __grid_constant__ DevCloud d) {
+    const int lane = threadIdx.x & 31, r = lane % 5;
+    const int i0 = blockIdx.x * QD_POINTS + (threadIdx.x >> 5) * 6;
+    const bool live = lane < 30 && i0 + lane / 5 < d.n;
+    const int i = live ? i0 + lane / 5 : min(i0, d.n - 1);
+    const double2 *pos = reinterpret_cast<const double2 *>(d.pos);   // (x, y), (z, speed)
+    const double2 xyi = pos[2 * (size_t)i];
+    const double xi = xyi.x, yi = xyi.y, zi = pos[2 * (size_t)i + 1].x;
+    const double qi = d.q[5 * (size_t)i + r];
+    double qmax = qi, qmin = qi, sx = 0.0, sy = 0.0, sz = 0.0, min_delt = 1.0;
+    const int nb = d.nbhs[i];
+    const int32_t *cn = d.conn + (size_t)MAX_CONN * i;
+    for (int j0 = 0; j0 < nb; j0 += QD_BATCH) {
+        int k[QD_BATCH];
+        double2 xy[QD_BATCH], zs[QD_BATCH];
+        double q[QD_BATCH];
+#pragma unroll
+        for (int b = 0; b < QD_BATCH; ++b) k[b] = j0 + b < nb ? cn[j0 + b] : i;
+#pragma unroll
+        for (int b = 0; b < QD_BATCH; ++b) {
+            xy[b] = pos[2 * (size_t)k[b]];
+            zs[b] = pos[2 * (size_t)k[b] + 1];
+            q[b] = d.q[5 * (size_t)k[b] + r];
+        }
+        // the lane's own neighbour of the batch
+        double2 xym = xy[0], zsm = zs[0];
+#pragma unroll
+        for (int b = 1; b < QD_BATCH; ++b) {
+            xym = r == b ? xy[b] : xym;
+            zsm = r == b ? zs[b] : zsm;
+        }
+#pragma unroll
+        for (int b = 0; b < QD_BATCH; ++b) {
+            if (j0 + b < nb) {
+                const double w = d.wq ? d.wq[(size_t)MAX_CONN * i + j0 + b] : 1.0;
+                const double delx = xy[b].x - xi, dely = xy[b].y - yi, delz = zs[b].x - zi;
+                const double t = q[b] - qi;
+                if (q[b] > qmax) qmax = q[b];
+                if (q[b] < qmin) qmin = q[b];
+                sx = sx + w * delx * t;
+                sy = sy + w * dely * t;
+                sz = sz + w * delz * t;
+            }
+        }
+        if (j0 + r < nb) {
+            const double delx = xym.x - xi, dely = xym.y - yi, delz = zsm.x - zi;
+            const double dist = sqrt(delx * delx + dely * dely + delz * delz);
+            const double delt = d.cfl * dist / zsm.y;       // timestep_delt.f90:235-253
+            if (delt < min_delt) min_delt = delt;
+        }
+    }
+    static_assert(QD_BATCH == 5, "a batch deals one neighbour to each lane of a point");
+#pragma unroll
+    for (int b = 1; b < 5; ++b) {
+        const double o = __shfl_sync(FULL, min_delt, lane - r + (r + b) % 5);
+        if (o < min_delt) min_delt = o;
+    }
+    if (!live) return;
+    const double *g = d.qgeo + QGEO_STRIDE * (size_t)i;
+    const double one_by_det = g[6];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) d.dq[15 * (size_t)i + 3 * r + a] = cramer_num(a, g, sx, sy, sz) * one_by_det;
+    d.qm[10 * (size_t)i + 2 * r + 0] = qmax;
+    d.qm[10 * (size_t)i + 2 * r + 1] = qmin;
+    if (r == 0) d.delt[i] = min_delt;
 }
 
 // eval_flux_residual (flux_residual.f90:40-81): one warp per point.  Lanes
@@ -388,95 +435,181 @@ __device__ __forceinline__ void sweep_inputs_warp(const DevCloud &d, int i, int 
 // then 30 lanes (list, component) sum the list terms in list order and solve
 // the 3x3 least-squares system with the precomputed moments.
 //
-// FUSED (chain schedule): the warps also produce the points' sweep inputs
-// (D_inv, fluxes of prim in the shared frame, the fixed increment of an
-// unswept point) and mark the hand-off words.
-//
 // R: the type of the reconstruction, limiter and flux arithmetic (float in
 // mixed precision); the offsets, weights, list sums and 3x3 solves are double.
-// RS: the type of the sweep inputs' fluxes (float whenever the sweeps run in
-// FP32, so that a sweep differences fluxes evaluated the same way).
-// Blocks of the flux kernel per SM the compiler must fit: four for the FP64
-// evaluation (128 registers, 16 warps per SM).
+// One end j of a neighbour pair in straight-line code (reconstruct, flux_pre,
+// axis_terms); ok is cleared where an argument is out of its range.
+__device__ __forceinline__ void end_core(const DevCloud &d, int j, double delx, double dely, double delz, const Frame &F,
+                                         FluxPreT<double> &P, AxisTermsT<double> A[3], bool &ok) {
+    const double *qj = d.q + 5 * (size_t)j, *dqj = d.dq + 15 * (size_t)j, *qmj = d.qm + 10 * (size_t)j;
+    const double eps2 = d.eps2[j];
+    double qt[5], prim[5], yspb;
+#pragma unroll
+    for (int r = 0; r < 5; ++r) {
+        const double q = qj[r];
+        const double temp = delx * dqj[3 * r] + dely * dqj[3 * r + 1] + delz * dqj[3 * r + 2];
+        qt[r] = q - 0.5 * limiter_core(q, temp, qmj[2 * r], qmj[2 * r + 1], eps2, ok) * temp;
+    }
+    prim_core(qt, prim, ok);
+    pre_core(prim, F, P, yspb, ok);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) axis_core(P.ut(a), P.sb, P.spb, yspb, A[a], ok);
+}
 template <typename R>
-constexpr int flux_min_blocks() { return sizeof(R) == 8 ? 4 : 1; }
+__device__ __forceinline__ void end_general(const DevCloud &d, int j, R delx, R dely, R delz, const FrameT<R> &F,
+                                            FluxPreT<R> &P, AxisTermsT<R> A[3]) {
+    R prim[5];
+    reconstruct<R>(d, j, delx, dely, delz, prim);
+    flux_pre(prim, F, P);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) axis_terms(P, a, A[a]);
+}
 
-template <bool FUSED, typename R, typename RS = R>
-__global__ void __launch_bounds__(FLUX_WARPS * 32, flux_min_blocks<R>()) k_flux(DevCloud d) {
+// One end's fluxes for every list the slot is in, into T[(list * 32 + lane) * 5
+// + component]: the first end's, then the second's less the first's.
+template <typename R>
+__device__ __forceinline__ void end_terms(int cls, int mask, int lane, const FluxPreT<R> &P, const AxisTermsT<R> A[3],
+                                          bool second, double *T) {
+    const bool wall = cls == CLS_WALL, octant = cls != CLS_INTERIOR;
+    const R A3 = wall ? A[2].An : A[2].Ap, B3 = wall ? -A[2].B : A[2].B;
+    for (; __any_sync(FULL, mask != 0); mask = mask_rest(mask)) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const int both = (mask >> (2 * a)) & 3;
+            const bool pos = (both & 1) != 0;
+            R f[5];
+            axis_flux(octant && a < 2, a, pos, P, A[a], A3, B3, f);
+            double *t = T + ((2 * a + (pos ? 0 : 1)) * MAX_SLOTS + lane) * 5;
+            if (both) {
+#pragma unroll
+                for (int c = 0; c < 5; ++c) t[c] = second ? (double)(f[c] - (R)t[c]) : (double)f[c];
+            }
+        }
+    }
+}
+
+// The terms with the operators, where an end's arguments left the range of the
+// straight-line code.
+__device__ __noinline__ void end_terms_general(const DevCloud &d, int p, int j, double delx, double dely, double delz,
+                                               int cls, int mask, int lane, bool second, double *T) {
+    Frame F;
+    load_frame(d.frame + 9 * (size_t)p, F);
+    FluxPre P;
+    AxisTerms A[3];
+    end_general<double>(d, j, delx, dely, delz, F, P, A);
+    end_terms<double>(cls, mask, lane, P, A, second, T);
+}
+
+// Bound by the FP64 pipe (47% busy) and the latency of the ends' gathers at 16
+// warps per SM.  Blocks per SM the compiler must fit: four in FP64 (128
+// registers; 1.1M points: three are 20% slower, five 6%), five in FP32 (62,400
+// points: 0.25 ms against 0.32 with four).  The pair's ends go through one copy
+// of the code: with both ends' code in a row the loop overran the instruction
+// cache (1.1M points: 9.4 against 7.9 ms).  With the branch-free functions and
+// storage order, 1.1M points take 5.95 ms against 10.7 ms before.
+template <typename R>
+constexpr int flux_blocks() { return sizeof(R) == 8 ? 4 : 5; }
+
+//
+// RS other than void (chain schedule): the first ceil(n / 128) blocks instead
+// evaluate the sweep inputs, a thread per point (point_inputs<RS>), after
+// marking their points' hand-off words DU_PENDING.
+template <typename R, typename RS>
+__global__ void __launch_bounds__(FLUX_WARPS * 32, flux_blocks<R>()) k_flux(const __grid_constant__ DevCloud d) {
     extern __shared__ double smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int first = 0;
+    if constexpr (!std::is_void<RS>::value) {
+        constexpr int PTS = FLUX_WARPS * 32;
+        first = (d.n + PTS - 1) / PTS;
+        if ((int)blockIdx.x < first) {
+            const size_t i0 = (size_t)blockIdx.x * PTS, i1 = min(i0 + PTS, (size_t)d.n);
+            const double pend = __longlong_as_double((long long)DU_PENDING);
+            if (d.shared_frame)
+                for (size_t w = DG_STRIDE * i0 + threadIdx.x; w < DG_STRIDE * i1; w += PTS) d.dgf[w] = d.dgb[w] = pend;
+            for (size_t w = 5 * i0 + threadIdx.x; w < 5 * i1; w += PTS)
+                if (d.swept[w / 5]) d.dUp[w] = d.dUn[w] = pend;
+            __syncthreads();              // before the fixed increments over the marks
+            // the fluxes' rows through shared memory, for whole-line stores
+            // (an odd stride: no bank conflicts)
+            constexpr int ROW = 31;
+            static_assert(PTS * ROW <= FLUX_WARPS * FLUX_SMEM_PER_WARP, "rows fit the flux warps' memory");
+            if (i0 + threadIdx.x < i1) point_inputs<RS>(d, (int)(i0 + threadIdx.x), smem + ROW * threadIdx.x);
+            __syncthreads();
+            if (d.shared_frame)
+                for (int w = threadIdx.x; w < 30 * (int)(i1 - i0); w += PTS)
+                    d.gold[30 * i0 + w] = smem[w / 30 * ROW + w % 30];
+            return;
+        }
+    }
     double *T = smem + warp * FLUX_SMEM_PER_WARP;     // T[(dir*32 + slot)*5 + c]
     double *W = T + NDIR * MAX_SLOTS * 5;             // W[slot*3 + axis]
-    for (int p = blockIdx.x * FLUX_WARPS + warp; p < d.n; p += gridDim.x * FLUX_WARPS) {
+    const int dd = lane / 5, c = lane - 5 * (lane / 5);
+    for (int p = (blockIdx.x - first) * FLUX_WARPS + warp; p < d.n; p += (gridDim.x - first) * FLUX_WARPS) {
         const int cls = d.cls[p];
         if (cls <= 2) {
-            const int ns = d.nslot[p];
-            if (lane < ns) {
-                const int k = d.slot_nbr[(size_t)p * MAX_SLOTS + lane];
-                const int mask = d.slot_mask[(size_t)p * MAX_SLOTS + lane];
-                Frame F;
-                load_frame(d.frame + 9 * (size_t)p, F);
-                FrameT<R> FR;
+            // lanes without a slot take the point itself and no list
+            const bool have = lane < d.nslot[p];
+            const int k = have ? d.slot_nbr[(size_t)p * MAX_SLOTS + lane] : p;
+            const int mask = have ? d.slot_mask[(size_t)p * MAX_SLOTS + lane] : 0;
+            // the lane's list (up to 27 entries of a byte, 28 apart)
+            const int cnt = lane < 30 ? d.list_cnt[(size_t)p * NDIR + dd] : 0;
+            const uint32_t *ent = reinterpret_cast<const uint32_t *>(d.list_ent + ((size_t)p * NDIR + (lane < 30 ? dd : 0)) * LIST_STRIDE);
+            Frame F;
+            load_frame(d.frame + 9 * (size_t)p, F);
+            const double delx = d.pos[4 * (size_t)k] - d.pos[4 * (size_t)p], dely = d.pos[4 * (size_t)k + 1] - d.pos[4 * (size_t)p + 1],
+                         delz = d.pos[4 * (size_t)k + 2] - d.pos[4 * (size_t)p + 2];
+            // dels*weights, delt*weights, deln*weights (weights 1 for power 0)
+            const double w = d.wf ? d.wf[(size_t)MAX_SLOTS * p + lane] : 1.0;
+            W[lane * 3 + 0] = (delx * F.t1[0] + dely * F.t1[1] + delz * F.t1[2]) * w;
+            W[lane * 3 + 1] = (delx * F.t2[0] + dely * F.t2[1] + delz * F.t2[2]) * w;
+            W[lane * 3 + 2] = (delx * F.n[0] + dely * F.n[1] + delz * F.n[2]) * w;
+#pragma unroll 1
+            for (int e = 0; e < 2; ++e) {
+                const int j = e ? k : p;
+                FluxPreT<R> P;
+                AxisTermsT<R> A[3];
+                if constexpr (sizeof(R) == 8) {
+                    bool ok = true;
+                    end_core(d, j, delx, dely, delz, F, P, A, ok);
+                    if (__all_sync(FULL, ok || !have)) end_terms<double>(cls, mask, lane, P, A, e != 0, T);
+                    else end_terms_general(d, p, j, delx, dely, delz, cls, mask, lane, e != 0, T);
+                } else {
+                    FrameT<R> FR;
 #pragma unroll
-                for (int r = 0; r < 3; ++r) { FR.t1[r] = (R)F.t1[r]; FR.t2[r] = (R)F.t2[r]; FR.n[r] = (R)F.n[r]; }
-                const double delx = d.x[k] - d.x[p], dely = d.y[k] - d.y[p], delz = d.z[k] - d.z[p];
-                // dels*weights, delt*weights, deln*weights (weights 1 for power 0)
-                const double w = d.wf ? d.wf[(size_t)MAX_SLOTS * p + lane] : 1.0;
-                W[lane * 3 + 0] = (delx * F.t1[0] + dely * F.t1[1] + delz * F.t1[2]) * w;
-                W[lane * 3 + 1] = (delx * F.t2[0] + dely * F.t2[1] + delz * F.t2[2]) * w;
-                W[lane * 3 + 2] = (delx * F.n[0] + dely * F.n[1] + delz * F.n[2]) * w;
-                int axes = 0;
-#pragma unroll
-                for (int dd = 0; dd < NDIR; ++dd)
-                    if (mask & (1 << dd)) axes |= kind_axes(flux_kind(cls, dd));
-                R prim[5];
-                FluxPreT<R> Pi, Pk;
-                AxisTermsT<R> Ai[3], Ak[3];
-                reconstruct<R>(d, p, (R)delx, (R)dely, (R)delz, prim);
-                flux_pre(prim, FR, Pi);
-                reconstruct<R>(d, k, (R)delx, (R)dely, (R)delz, prim);
-                flux_pre(prim, FR, Pk);
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    if (axes & (1 << a)) {
-                        axis_terms(Pi, a, Ai[a]);
-                        axis_terms(Pk, a, Ak[a]);
-                    }
-                }
-                for (int dd = 0; dd < NDIR; ++dd) {
-                    if (!(mask & (1 << dd))) continue;
-                    const int kind = flux_kind(cls, dd);
-#pragma unroll
-                    for (int c = 0; c < 5; ++c) {
-                        const R gi = flux_component(kind, c, Pi, Ai);
-                        const R gk = flux_component(kind, c, Pk, Ak);
-                        T[(dd * MAX_SLOTS + lane) * 5 + c] = (double)(gk - gi);
-                    }
+                    for (int r = 0; r < 3; ++r) { FR.t1[r] = (R)F.t1[r]; FR.t2[r] = (R)F.t2[r]; FR.n[r] = (R)F.n[r]; }
+                    end_general<R>(d, j, (R)delx, (R)dely, (R)delz, FR, P, A);
+                    end_terms<R>(cls, mask, lane, P, A, e != 0, T);
                 }
             }
             __syncwarp();
             double G = 0.0;
             if (lane < 30) {
-                const int dd = lane / 5, c = lane - 5 * dd;
-                const int cnt = d.list_cnt[(size_t)p * NDIR + dd];
-                const uint8_t *ent = d.list_ent + ((size_t)p * NDIR + dd) * LIST_STRIDE;
                 double sx = 0.0, sy = 0.0, sz = 0.0;
-#pragma unroll 4
-                for (int j = 0; j < cnt; ++j) {
-                    const int s = ent[j];
-                    const double t = T[(dd * MAX_SLOTS + s) * 5 + c];
-                    sx = sx + t * W[s * 3 + 0];
-                    sy = sy + t * W[s * 3 + 1];
-                    sz = sz + t * W[s * 3 + 2];
+                const double *t = T + dd * MAX_SLOTS * 5 + c;
+                for (int j = 0; j < cnt; j += 4) {
+                    const uint32_t e4 = ent[j >> 2];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        if (j + q < cnt) {
+                            const int s = (e4 >> (8 * q)) & 255;
+                            const double v = t[s * 5];
+                            sx = sx + v * W[s * 3 + 0];
+                            sy = sy + v * W[s * 3 + 1];
+                            sz = sz + v * W[s * 3 + 2];
+                        }
+                    }
                 }
                 const double *g = d.geo + (size_t)p * GEO_STRIDE + dd * 8;
-                const double num = cramer_num(dd >> 1, g, sx, sy, sz);
+                const double num = cramer_select(dd >> 1, g, sx, sy, sz), det = g[G_DET];
                 // outer_flux_dG*.f90:118-124 multiply by 1/det; the others divide
-                G = (cls == CLS_OUTER) ? num * (1.0 / g[G_DET]) : num / g[G_DET];
+                const double y = rcp_rn(det);
+                if (ieee_ok(fabs(det)) && ieee_num_ok(num)) G = (cls == CLS_OUTER) ? num * y : quot_rn(num, det, y);
+                else G = (cls == CLS_OUTER) ? num * (1.0 / det) : num / det;
             }
             double gd[NDIR];
 #pragma unroll
-            for (int dd = 0; dd < NDIR; ++dd) gd[dd] = __shfl_sync(FULL, G, dd * 5 + (lane % 5));
+            for (int e = 0; e < NDIR; ++e) gd[e] = __shfl_sync(FULL, G, e * 5 + (lane % 5));
             if (lane < 5) {
                 double r;
                 if (cls == CLS_INTERIOR) r = gd[0] + gd[1] + gd[2] + gd[3] + gd[4] + gd[5];
@@ -485,7 +618,6 @@ __global__ void __launch_bounds__(FLUX_WARPS * 32, flux_min_blocks<R>()) k_flux(
                 d.flux_res[5 * (size_t)p + lane] = r;
             }
         }
-        if (FUSED) sweep_inputs_warp<RS>(d, p, lane);
         __syncwarp();
     }
 }
@@ -1117,6 +1249,7 @@ __global__ void k_update(DevCloud d, double *U_next, double *q_next) {
         for (int r = 0; r < 5; ++r) p[r] = d.prim[5 * (size_t)i + r];
     }
     d.res_sqr[i] = res;
+    d.pos[4 * (size_t)i + 3] = signal_speed(p);
     double Un[5], qn[5];
     primitive_to_rotated_conserved(p, F, Un);
     primitive_to_q(p, qn);
@@ -1144,6 +1277,7 @@ __global__ void k_update_ss(DevCloud d, double *U_next, double *q_next) {
             p[r] = src >= 0 ? d.prim[5 * (size_t)src + r] : 0.0;
             d.prim[5 * (size_t)k + r] = p[r];
         }
+        d.pos[4 * (size_t)k + 3] = signal_speed(p);
         Frame F;
         load_frame(d.frame + 9 * (size_t)k, F);
         double Un[5], qn[5];
@@ -1352,14 +1486,13 @@ static void set_attributes(int device) {
     static bool done[256] = {false};
     std::lock_guard<std::mutex> lock(mu);
     if (device < 0 || device >= 256 || done[device]) return;
-    cudaFuncSetAttribute(k_flux<false, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         FLUX_WARPS * FLUX_SMEM_PER_WARP * 8);
-    cudaFuncSetAttribute(k_flux<true, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         FLUX_WARPS * FLUX_SMEM_PER_WARP * 8);
-    cudaFuncSetAttribute(k_flux<true, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         FLUX_WARPS * FLUX_SMEM_PER_WARP * 8);
-    cudaFuncSetAttribute(k_flux<true, double, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         FLUX_WARPS * FLUX_SMEM_PER_WARP * 8);
+    auto flux = [](auto *kern) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FLUX_WARPS * FLUX_SMEM_PER_WARP * 8);
+    };
+    flux(k_flux<double, void>);
+    flux(k_flux<double, double>);
+    flux(k_flux<double, float>);
+    flux(k_flux<float, float>);
     cudaFuncSetAttribute(k_sweep_levels, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          SWEEP_WARPS * SWEEP_SMEM_BYTES);
     cudaFuncSetAttribute(k_sweep_df, cudaFuncAttributeMaxDynamicSharedMemorySize, DF_WARPS * SWEEP_SMEM_BYTES);
@@ -1489,6 +1622,11 @@ cudaError_t launch_rows(const double *src, double *dst, const int32_t *perm, int
     return cudaGetLastError();
 }
 
+cudaError_t launch_qgeo(const DevCloud &d, double *qgeo, cudaStream_t s) {
+    k_qgeo<<<(d.n + 127) / 128, 128, 0, s>>>(d, qgeo);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_conserved_q(const DevCloud &d, cudaStream_t s) {
     k_conserved_q<<<(d.n + 127) / 128, 128, 0, s>>>(d);
     return cudaGetLastError();
@@ -1568,7 +1706,7 @@ cudaError_t launch_iteration(const DevCloud &d, int iter_slot, const IterStreams
     // supersonic copies may read a neighbour's increment from before the
     // sweeps, which k_pending is about to mark
     if (d.dU_old) cudaMemcpyAsync(d.dU_old, d.dUn, sizeof(double) * 5 * (size_t)n, cudaMemcpyDeviceToDevice, s);
-    k_qderiv<<<(n + 127) / 128, 128, 0, s>>>(d);
+    k_qderiv<<<(n + QD_POINTS - 1) / QD_POINTS, QD_THREADS, 0, s>>>(d);
     for (int j = 0; j < d.inner_iterations; ++j) {
         k_qinner<<<(n + 127) / 128, 128, 0, s>>>(d, d.dq, d.dq_tmp);
         cudaMemcpyAsync(d.dq, d.dq_tmp, sizeof(double) * 15 * (size_t)n, cudaMemcpyDeviceToDevice, s);
@@ -1581,17 +1719,16 @@ cudaError_t launch_iteration(const DevCloud &d, int iter_slot, const IterStreams
         else k_g0<double><<<gb, 128, 0, s>>>(d);
     }
     if (chains) {
-        // the flux residual, the sweep inputs and the hand-off marks; before the
-        // sweeps, whose teams leave no room beside them (1.1M points: 37.0 ms
-        // per iteration against 39.5 to 112 with the flux residual beside the
-        // forward sweep; 62k: 7.0 against 6.9)
+        // before the sweeps, whose teams leave no room beside them (1.1M points:
+        // 37.0 ms per iteration against 39.5 to 112 with the flux residual
+        // beside the forward sweep; 62k: 7.0 against 6.9)
         const size_t fsm = FLUX_WARPS * FLUX_SMEM_PER_WARP * 8;
         // a smaller grid walks the same order with its warps striding through it
         const int fgrid = d.flux_grid > 0 && d.flux_grid < fblocks ? d.flux_grid : fblocks;
-        auto flux = [&](auto *kern) { launch_prio(kern, fgrid, FLUX_WARPS * 32, fsm, s, false, d); };
-        if (dc) flux(k_flux<true, double, float>);
-        else if (mixed) flux(k_flux<true, float>);
-        else flux(k_flux<true, double>);
+        const int grid = fgrid + (n + FLUX_WARPS * 32 - 1) / (FLUX_WARPS * 32);
+        if (dc) launch_prio(k_flux<double, float>, grid, FLUX_WARPS * 32, fsm, s, false, d);
+        else if (mixed) launch_prio(k_flux<float, float>, grid, FLUX_WARPS * 32, fsm, s, false, d);
+        else launch_prio(k_flux<double, double>, grid, FLUX_WARPS * 32, fsm, s, false, d);
         mark(2, s);
         mark(3, s);
         if (part == ITER_PRE) {
@@ -1601,7 +1738,7 @@ cudaError_t launch_iteration(const DevCloud &d, int iter_slot, const IterStreams
         sweep(1);
         mark(4, s);
     } else {
-        k_flux<false, double><<<fblocks, FLUX_WARPS * 32, FLUX_WARPS * FLUX_SMEM_PER_WARP * 8, s>>>(d);
+        k_flux<double, void><<<fblocks, FLUX_WARPS * 32, FLUX_WARPS * FLUX_SMEM_PER_WARP * 8, s>>>(d);
         mark(2, s);
         k_pending<<<sms * 8, 256, 0, s>>>(d);
         k_dinv_gold<<<(n + 127) / 128, 128, 0, s>>>(d);

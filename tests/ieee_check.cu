@@ -27,7 +27,7 @@ __device__ uint64_t significand(uint64_t r) {
     case 0: return m & 0xff;
     case 1: return (one - (m & 0xff)) & one;
     case 2: return (m & (one << 26)) & one;
-    case 3: return ((m & (one << 26)) + (m & 7)) & one;
+    case 3: return (r >> 3 & 1) ? one : ((m & (one << 26)) + (m & 7)) & one;
     default: return m;
     }
 }
