@@ -832,6 +832,9 @@ int attach_state(mfcfd_handle *h) {
 #undef AL
     d.U = h->U_buf[0];
     d.q = h->q_buf[0];
+    d.frame0_axes = 1;
+    for (int r = 0; r < 9; ++r)
+        if (d.frame0[r] != (r % 4 == 0 ? 1.0 : 0.0) || std::signbit(d.frame0[r])) d.frame0_axes = 0;
     if (h->dry) return MFCFD_OK;
     CK(cudaMemsetAsync(d.sweep_counter, 0, sizeof(int) * 2, h->stream));
     CK(cudaMemsetAsync(d.err, 0, sizeof(int), h->stream));

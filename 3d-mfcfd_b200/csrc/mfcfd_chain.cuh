@@ -12,10 +12,12 @@
  * arithmetic of one point (remaining sums, solve, own flux) and a
  * shared-memory hand-off, not the fetches around it.  Measured (B200, FP64,
  * both sweeps of an iteration; before: one warp per chain, which did all of a
- * point's work in turn): 62,400 points 13.6 -> 6.2 ms (1.7 us per level),
- * 1.1M points 49.6 -> 23.9 ms, mixed precision at 62,400 11.4 -> 5.1 ms.  Of a
- * point's cycles on the dependent path, its own flux takes about 1,160, the
- * sums after the ring term 120, the solve 155, the rest of dU 165.
+ * point's work in turn): 62,400 points 13.6 -> 5.05 ms (1.4 us per level),
+ * 1.1M points 49.6 -> 20.6 ms, mixed precision at 62,400 11.4 -> 3.8 ms.  On
+ * the critical path of the 62,400-point sweep three hops in four are from a
+ * chain's point to its next (1.0 us: its own flux about 1,100 cycles, the sums
+ * after the ring term 150, the solve 150, the rest of dU 165), one in four to
+ * another chain through L2 (1.8 us), one in thirty to a wall point (3.6 us).
  *
  * Ring.  The team's last increments lie in a shared ring of TEAM_RING slots of
  * 32 words (lane l's component), one per position (a team of one warp:
@@ -184,6 +186,10 @@ __device__ __forceinline__ void lds_if(unsigned long long &v, unsigned a, bool t
                  : "+l"(v)
                  : "r"(a), "r"((int)take));
 }
+__device__ __forceinline__ bool pending_word(unsigned long long v) {
+    // no increment, flux or D_inv has this upper half (a signalling NaN)
+    return (unsigned)(v >> 32) == (unsigned)(DU_PENDING >> 32);
+}
 // The ring word at `a` once its position has written it (every lane calls; a
 // lane without `need` does not wait).
 __device__ __forceinline__ double ring_word(const DevCloud &d, unsigned a, bool need) {
@@ -192,14 +198,10 @@ __device__ __forceinline__ double ring_word(const DevCloud &d, unsigned a, bool 
     bool wait;
     do {
         t = lds_relaxed(a);
-        wait = need && is_pending(t);
+        wait = need && pending_word((unsigned long long)__double_as_longlong(t));
         if (wait && !team_spin_continue(spins, d)) wait = false;
     } while (__any_sync(FULL, wait));
     return t;
-}
-__device__ __forceinline__ bool pending_word(unsigned long long v) {
-    // no increment, flux or D_inv has this upper half (a signalling NaN)
-    return (unsigned)(v >> 32) == (unsigned)(DU_PENDING >> 32);
 }
 
 // s += term x weight, in the list's order; a no-op unless `in`.
@@ -229,7 +231,7 @@ struct Sums {
 // the terms before it are added, and the products of the AFTER terms after
 // it formed, before the wait for its word.  Straight-line code with predicated
 // loads and sums: a divergent branch per term costs more than the term.
-constexpr int AFTER = 6;
+constexpr int AFTER = 8;
 template <bool FOLD>
 __device__ __forceinline__ void shared_sums(const DevCloud &d, const SweepEntry *E, int n, const double *src,
                                             unsigned tl, unsigned rl, const Team &team, int pos, Sums<FOLD> &s) {
@@ -320,88 +322,6 @@ __device__ __forceinline__ void shared_sums(const DevCloud &d, const SweepEntry 
     }
 }
 
-// The operators' form of a point whose arguments were out of the range of the
-// branch-free ones: dU and the point's flux in the shared frame (component c of
-// list dd) from its list sums.
-struct PointOut {
-    double dnew, flux;
-};
-template <typename R, bool FOLD>
-__device__ __noinline__ PointOut point_general(const double *frame0, const SweepStage *st, bool forward, int dd, int c,
-                                               double sx, double sy, double sz, double dinv, double base5) {
-    double G = sx;
-    if constexpr (!FOLD) {
-        const double *g = st->geo + dd * 8;
-        G = cramer_select(dd >> 1, g, sx, sy, sz) / g[6];
-    }
-    double gd[NDIR];
-#pragma unroll
-    for (int e = 0; e < NDIR; ++e) gd[e] = __shfl_sync(FULL, G, e * 5 + c);
-    const double lu = gd[0] + gd[1] + gd[2] + gd[3] + gd[4] + gd[5];
-    PointOut o;
-    o.dnew = forward ? -(dinv * (base5 + lu)) : base5 - dinv * lu;
-    R U[5];
-#pragma unroll
-    for (int r = 0; r < 5; ++r) U[r] = (R)(__shfl_sync(FULL, o.dnew, r) + st->U[r]);
-    FrameT<R> F0;
-    load_frame(frame0, F0);
-    o.flux = (double)state_flux_general<R>(dd, c, U, F0, F0);
-    return o;
-}
-
-// A point in the shared frame: the sweep's common case, kept apart from the
-// others so that its code is short and free of their branches.
-template <typename R, bool FOLD>
-__device__ __forceinline__ void shared_point(const DevCloud &d, const ChainItem &it, const SweepStage *st, bool forward,
-                                             int lane, int word, int dd, int c, double *T, const Team &team, int pos) {
-    const int p = it.p;
-    const bool hold = p + 1 == d.withhold1;           // failure-detection hook: publish nothing
-    const double gold = st->gold[word], dinv = st->dinv[0], base5 = st->base[c];
-    double U[5];
-#pragma unroll
-    for (int r = 0; r < 5; ++r) U[r] = st->U[r];
-    const int lo = count_sum(it.cnt & ((1u << (5 * dd)) - 1u)), n = item_count(it.cnt, dd);
-    double g[7] = {0, 0, 0, 0, 0, 0, 1.0};
-    double ydet = 0.0;
-    bool ok = true;
-    if constexpr (!FOLD) {
-#pragma unroll
-        for (int r = 0; r < 7; ++r) g[r] = st->geo[dd * 8 + r];
-        ok = ieee_ok(fabs(g[6]));
-        ydet = rcp_rn(g[6]);
-    }
-    double *out = (forward ? d.dgf : d.dgb) + (DG_LIST * dd + c);
-    Sums<FOLD> s;
-    shared_sums<FOLD>(d, st->ent + lo, n, out, smem_addr(T + lane), smem_addr(team.ring + word), team, pos, s);
-    double G = s.x;
-    if constexpr (!FOLD) {
-        const double num = cramer_select(dd >> 1, g, s.x, s.y, s.z);
-        ok = ok && ieee_num_ok(num);
-        G = quot_rn(num, g[6], ydet);
-    }
-    double gd[NDIR];
-#pragma unroll
-    for (int e = 0; e < NDIR; ++e) gd[e] = __shfl_sync(FULL, G, e * 5 + c);
-    const double lu = gd[0] + gd[1] + gd[2] + gd[3] + gd[4] + gd[5];
-    double dnew = forward ? -(dinv * (base5 + lu)) : base5 - dinv * lu;
-    R Un[5];
-#pragma unroll
-    for (int r = 0; r < 5; ++r) Un[r] = (R)(__shfl_sync(FULL, dnew, r) + U[r]);
-    FrameT<R> F0;
-    load_frame(d.frame0, F0);
-    double flux = (double)state_flux(dd, c, Un, F0, F0, ok);
-    if (!__all_sync(FULL, ok)) {
-        const PointOut o = point_general<R, FOLD>(d.frame0, st, forward, dd, c, s.x, s.y, s.z, dinv, base5);
-        dnew = o.dnew;
-        flux = o.flux;
-    }
-    const double v = sizeof(R) == 8 ? flux - gold : (double)((R)flux - (R)gold);
-    sts_relaxed(smem_addr(team.ring + ring_slot(team, pos, 0) * 32 + lane), v);
-    if (lane < 30 && (it.info & CI_PUBLISH) && !hold) st_relaxed_f64(out + DG_STRIDE * (size_t)p, v);
-    if (lane < 5 && !hold) st_relaxed_f64((forward ? d.dUp : d.dUn) + 5 * (size_t)p + lane, dnew);
-    team_leave(team, pos, lane);
-}
-
 // A wall or interior point's slot: its fluxes along the three axes, less what T
 // holds, into T.  The sign of each axis's list is selected, not branched on.
 template <typename R>
@@ -423,12 +343,23 @@ __device__ __forceinline__ void slot_fluxes(bool wall, int mask, const FluxPreT<
     }
 }
 
+// The state of a slot's neighbour (conserved U in frame Fk) in the point's
+// frame with the operators, where it left the range of the straight-line code.
+template <typename R>
+__device__ __noinline__ void slot_state_general(const R U[5], const FrameT<R> &Fk, const FrameT<R> &Fp, FluxPreT<R> &P,
+                                                AxisTermsT<R> A[3]) {
+    R pn[5];
+    conserved_to_primitive(U, Fk, pn);
+    flux_pre(pn, Fp, P);
+    for (int a = 0; a < 3; ++a) axis_terms(P, a, A[a]);
+}
+
 // Term fluxes of a point outside the shared frame, lane per neighbour slot,
 // into T[(list * MAX_SLOTS + slot) * 5 + component] (phases A and B of
 // sweep_point).
 template <typename R>
-__device__ __forceinline__ void unshared_terms(const DevCloud &d, const ChainItem &it, const SweepStage *st, int cls,
-                                               const FrameT<R> &Fp, bool forward, int lane, double *T, bool g0_newer) {
+__device__ __noinline__ void unshared_terms(const DevCloud &d, ChainItem it, const SweepStage *st, int cls, bool forward,
+                                            int lane, double *T, bool g0_newer) {
     const bool mine = (st->need >> lane) & 1u;
     const bool g0 = (it.info & CI_G0) != 0;
     const int k_slot = mine ? st->slot_nbr[lane] : it.p;
@@ -437,8 +368,9 @@ __device__ __forceinline__ void unshared_terms(const DevCloud &d, const ChainIte
     double Uk[5];
 #pragma unroll
     for (int r = 0; r < 5; ++r) Uk[r] = d.U[5 * (size_t)k_slot + r];
-    FrameT<R> Fk;
+    FrameT<R> Fk, Fp;
     load_frame(d.frame + 9 * (size_t)k_slot, Fk);
+    load_frame(st->frame, Fp);
     if (mine && !g0) neighbour_fluxes<R>(d, cls, Fp, k_slot, mask_slot, lane, T);
     unsigned long long v[5] = {0, 0, 0, 0, 0};
     {
@@ -459,19 +391,19 @@ __device__ __forceinline__ void unshared_terms(const DevCloud &d, const ChainIte
     FluxPreT<R> P;
     AxisTermsT<R> A[3];
     bool ok = true;
-    if constexpr (sizeof(R) == 8) {
-        double yspb;
-        state_core(U, Fk, Fp, P, yspb, ok);
+    R yspb;
+    state_core(U, Fk, Fp, P, yspb, ok);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) axis_core(P.ut(a), P.sb, P.spb, yspb, A[a], ok);
-    }
-    ok = ok || !mine;
-    if (sizeof(R) == 4 || !__all_sync(FULL, ok)) {
-        R pn[5];
-        conserved_to_primitive(U, Fk, pn);
-        flux_pre(pn, Fp, P);
+    for (int a = 0; a < 3; ++a) axis_core(P.ut(a), P.sb, P.spb, yspb, A[a], ok);
+    if (!__all_sync(FULL, ok || !mine)) {
+        R Uc[5] = {U[0], U[1], U[2], U[3], U[4]};
+        FrameT<R> Fkc = Fk, Fpc = Fp;
+        FluxPreT<R> Pc;
+        AxisTermsT<R> Ac[3];
+        slot_state_general<R>(Uc, Fkc, Fpc, Pc, Ac);
+        P = Pc;
 #pragma unroll
-        for (int a = 0; a < 3; ++a) axis_terms(P, a, A[a]);
+        for (int a = 0; a < 3; ++a) A[a] = Ac[a];
     }
     if (g0) {
         // the copied phase-A fluxes: every lane's copies have landed
@@ -493,6 +425,119 @@ __device__ __forceinline__ void unshared_terms(const DevCloud &d, const ChainIte
         }
     }
     __syncwarp();
+}
+
+// The operators' form of a point whose arguments were out of the range of the
+// branch-free ones: dU and the point's flux in the shared frame (component c of
+// list dd) from its list sums.
+struct PointOut {
+    double dnew, flux;
+};
+__device__ __forceinline__ double list_total(bool wall, const double gd[NDIR]) {
+    const double x = gd[0] + gd[1] + gd[2] + gd[3] + (wall ? gd[5] : gd[4]);
+    return wall ? 2.0 * x : x + gd[5];
+}
+template <typename R, bool FOLD>
+__device__ __noinline__ PointOut point_general(const double *frame0, const SweepStage *st, bool wall, bool forward, int dd,
+                                               int c, double sx, double sy, double sz, double dinv, double base5) {
+    double G = sx;
+    if constexpr (!FOLD) {
+        const double *g = st->geo + dd * 8;
+        G = cramer_select(dd >> 1, g, sx, sy, sz) / g[6];
+    }
+    double gd[NDIR];
+#pragma unroll
+    for (int e = 0; e < NDIR; ++e) gd[e] = __shfl_sync(FULL, G, e * 5 + c);
+    const double lu = list_total(wall, gd);
+    PointOut o;
+    o.dnew = forward ? -(dinv * (base5 + lu)) : base5 - dinv * lu;
+    R U[5];
+#pragma unroll
+    for (int r = 0; r < 5; ++r) U[r] = (R)(__shfl_sync(FULL, o.dnew, r) + st->U[r]);
+    FrameT<R> F0, F;
+    load_frame(frame0, F0);
+    load_frame(st->frame, F);
+    o.flux = (double)state_flux_general<R>(dd, c, U, F, F0);
+    return o;
+}
+
+// A point in the shared frame, or a wall point, of a cloud with a shared frame
+// under the alias driver: the sweep's common cases, kept apart from the others
+// so that their code is short, free of the others' branches and, beyond the
+// sums, the same for both (a wall point's own code is seldom in the
+// instruction cache).
+template <typename R, bool FOLD>
+__device__ __forceinline__ void common_point(const DevCloud &d, const ChainItem &it, const SweepStage *st, bool forward,
+                                             int lane, int word, int dd, int c, double *T, const Team &team, int pos,
+                                             bool g0_newer) {
+    const int p = it.p;
+    const bool hold = p + 1 == d.withhold1;           // failure-detection hook: publish nothing
+    const bool wall = (it.info & CI_WALL) != 0;
+    const double gold = st->gold[word], dinv = st->dinv[0], base5 = st->base[c];
+    const double Uc = st->U[c];
+    const int lo = count_sum(it.cnt & ((1u << (5 * dd)) - 1u)), n = item_count(it.cnt, dd);
+    double g[7] = {0, 0, 0, 0, 0, 0, 1.0};
+    double ydet = 0.0;
+    bool ok = d.frame0_axes != 0;
+    if constexpr (!FOLD) {
+#pragma unroll
+        for (int r = 0; r < 7; ++r) g[r] = st->geo[dd * 8 + r];
+        if (wall && dd == 4) g[6] = 1.0;              // a list walls do not have
+        ok = ok && ieee_ok(fabs(g[6]));
+        ydet = rcp_rn(g[6]);
+    }
+    double *out = (forward ? d.dgf : d.dgb) + (DG_LIST * dd + c);
+    Sums<FOLD> s;
+    const SweepEntry *E = st->ent + lo;
+    if (wall) {
+        unshared_terms<R>(d, it, st, CLS_WALL, forward, lane, T, g0_newer);
+        const double *Tl = T + dd * MAX_SLOTS * 5 + c;
+        const int nmax = (int)__reduce_max_sync(FULL, (unsigned)n);
+        for (int j = 0; j < nmax; j += 4) {
+            // past the list's end: its first terms, unused
+            double t[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) t[q] = Tl[((E[j + q < n ? j + q : 0].pad >> 8) & (MAX_SLOTS - 1)) * 5];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) s.term(j + q < n, t[q], E[j + q < n ? j + q : 0]);
+        }
+    } else {
+        shared_sums<FOLD>(d, E, n, out, smem_addr(T + lane), smem_addr(team.ring + word), team, pos, s);
+    }
+    double G = s.x;
+    if constexpr (!FOLD) {
+        const double num = cramer_select(dd >> 1, g, s.x, s.y, s.z);
+        ok = ok && ieee_num_ok(num);
+        G = quot_rn(num, g[6], ydet);
+    }
+    double gd[NDIR];
+#pragma unroll
+    for (int e = 0; e < NDIR; ++e) gd[e] = __shfl_sync(FULL, G, e * 5 + c);
+    const double lu = list_total(wall, gd);
+    double dnew = forward ? -(dinv * (base5 + lu)) : base5 - dinv * lu;
+    const double un = dnew + Uc;
+    R Un[5];
+#pragma unroll
+    for (int r = 0; r < 5; ++r) Un[r] = (R)__shfl_sync(FULL, un, r);
+    if (wall) {
+        // back from the point's frame (conserved_to_primitive)
+        FrameT<R> F;
+        load_frame(st->frame, F);
+        const R m1 = Un[1], m2 = Un[2], m3 = Un[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) Un[1 + r] = F.t1[r] * m1 + F.t2[r] * m2 + F.n[r] * m3;
+    }
+    double flux = (double)state_flux(dd, c, Un, ok);
+    if (!__all_sync(FULL, ok)) {
+        const PointOut o = point_general<R, FOLD>(d.frame0, st, wall, forward, dd, c, s.x, s.y, s.z, dinv, base5);
+        dnew = o.dnew;
+        flux = o.flux;
+    }
+    const double v = sizeof(R) == 8 ? flux - gold : (double)((R)flux - (R)gold);
+    sts_relaxed(smem_addr(team.ring + ring_slot(team, pos, 0) * 32 + lane), v);
+    if (lane < 30 && (it.info & CI_PUBLISH) && !hold) st_relaxed_f64(out + DG_STRIDE * (size_t)p, v);
+    if (lane < 5 && !hold) st_relaxed_f64((forward ? d.dUp : d.dUn) + 5 * (size_t)p + lane, dnew);
+    team_leave(team, pos, lane);
 }
 
 // One point of the forward (LdelU) or backward (UdelU) sweep by one warp of
@@ -542,7 +587,7 @@ __device__ __noinline__ void general_point(const DevCloud &d, ChainItem it, cons
         const bool shared = (it.info & CI_SHARED) != 0;   // backup driver
         if (!shared) {
             const int cls = wall ? CLS_WALL : (outer ? CLS_OUTER : CLS_INTERIOR);
-            unshared_terms<R>(d, it, st, cls, Fp, forward, lane, T, g0_newer);
+            unshared_terms<R>(d, it, st, cls, forward, lane, T, g0_newer);
         }
         double sx = 0.0, sy = 0.0, sz = 0.0;
 #pragma unroll 4
@@ -661,8 +706,8 @@ __device__ __forceinline__ void chain_sweep(const DevCloud &d, int forward, int 
             }
             const ChainItem after = pos + 2 * size < len ? items[pos + 2 * size] : nxt;
             team_enter(d, team, pos, lane);
-            if ((cur.info & (CI_SHARED | CI_COPY | CI_OUTER | CI_WALL)) == CI_SHARED && !d.dg_old)
-                shared_point<R, FOLD>(d, cur, &stg[s], forward != 0, lane, word, dd, c, T, team, pos);
+            if ((cur.info & (CI_SHARED | CI_WALL)) && d.shared_frame && !d.dg_old)
+                common_point<R, FOLD>(d, cur, &stg[s], forward != 0, lane, word, dd, c, T, team, pos, more);
             else
                 general_point<R, FOLD>(d, cur, &stg[s], forward != 0, lane, T, team, pos, more);
             cur = nxt;

@@ -313,6 +313,7 @@ struct DevCloud {
     int n;
     int shared_frame;
     double frame0[9];
+    int frame0_axes;              // frame0 is exactly the global axes
     double power, cfl;
     int inner_iterations;         // second-order q-derivative passes
     int update_variant;           // MFCFD_UPDATE_*

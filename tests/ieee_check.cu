@@ -1,8 +1,10 @@
-// Compares mfcfd_ieee.cuh with the FP64 operators on the GPU: random
+// Compares mfcfd_ieee.cuh with the operators on the GPU.  FP64: random
 // arguments over the range ieee_ok admits, and arguments next to rounding
 // boundaries (quotients and roots whose exact value lies close to a midpoint
-// of two doubles, significands next to a power of two).  Prints the number of
-// arguments and of results whose bits differ.
+// of two doubles, significands next to a power of two).  FP32: every
+// significand for the reciprocal and (both parities of the exponent) the root,
+// random pairs for the quotient.  Prints the number of arguments and of
+// results whose bits differ.
 #include <cstdio>
 #include <cstdint>
 #include <cstdlib>
@@ -74,6 +76,35 @@ __global__ void check(uint64_t seed, int rounds, unsigned long long *bad) {
     atomicAdd(bad + 3, seen);
 }
 
+__global__ void check_f32(uint64_t seed, int rounds, unsigned long long *bad) {
+    const uint64_t id = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, all = gridDim.x * (uint64_t)blockDim.x;
+    unsigned long long wrong[3] = {0, 0, 0}, seen = 0;
+    auto differ = [](float a, float b) { return __float_as_int(a) != __float_as_int(b); };
+    for (uint64_t m = id; m < (1ull << 24); m += all) {
+        // all significands in two neighbouring binades, at a random exponent
+        const int e = 68 + 2 * (int)(mix(seed ^ m) % 59);
+        const float b = __int_as_float((int)((uint32_t)(e << 23) + (uint32_t)m));
+        if (!ieee_ok(b)) continue;
+        ++seen;
+        const float y = rcp_rn(b);
+        if (differ(y, 1.0f / b)) ++wrong[0];
+        if (differ(sqrt_rn(b), sqrtf(b))) ++wrong[2];
+        for (int k = 0; k < rounds; ++k) {
+            const uint64_t r = mix(seed + 64 * m + (uint64_t)k);
+            float a = __int_as_float((int)(((uint32_t)(67 + r % 119) << 23) | (uint32_t)(r >> 40 & 0x7fffff)));
+            if (k & 1) {                  // next to a midpoint
+                const float q = __int_as_float((int)((127u << 23) | (uint32_t)(r >> 40 & 0x7fffff)));
+                a = __fmaf_rn(q, b, 0x1p-24f * b);
+                if (!ieee_ok(a)) continue;
+            }
+            if (differ(quot_nz(a, b, y), a / b)) ++wrong[1];
+        }
+    }
+    for (int w = 0; w < 3; ++w)
+        if (wrong[w]) atomicAdd(bad + w, wrong[w]);
+    atomicAdd(bad + 3, seen);
+}
+
 int main(int argc, char **argv) {
     const int rounds = argc > 1 ? std::atoi(argv[1]) : 256;
     unsigned long long *bad = nullptr, h[4] = {0, 0, 0, 0};
@@ -81,6 +112,12 @@ int main(int argc, char **argv) {
     check<<<148 * 8, 256>>>(20240607ull, rounds, bad);
     if (cudaMemcpy(h, bad, sizeof h, cudaMemcpyDeviceToHost) != cudaSuccess) return 2;
     std::printf("arguments %llu wrong: reciprocal %llu quotient %llu root %llu\n", h[3], h[0], h[1], h[2]);
+    unsigned long long f[4] = {0, 0, 0, 0};
+    if (cudaMemset(bad, 0, sizeof h) != cudaSuccess) return 2;
+    check_f32<<<148 * 8, 256>>>(20240608ull, 16, bad);
+    if (cudaMemcpy(f, bad, sizeof f, cudaMemcpyDeviceToHost) != cudaSuccess) return 2;
+    std::printf("FP32 arguments %llu wrong: reciprocal %llu quotient %llu root %llu\n", f[3], f[0], f[1], f[2]);
     cudaFree(bad);
+    if (f[0] || f[1] || f[2] || !f[3]) return 1;
     return h[0] || h[1] || h[2] || !h[3] ? 1 : 0;
 }
