@@ -16,8 +16,10 @@
  *    keys' order is the order of discovery, which a prefix sum over the key
  *    space turns into alias numbers.  Point 1's first neighbour takes alias
  *    1 and is never a parent, as in the reference.
- *  - levels: the longest-path depth over a sweep's dependencies, by Kahn's
- *    layering (a point joins level L+1 when its last dependency leaves
+ *  - levels: the longest-path depth over a sweep's dependencies: for the
+ *    device-resident set-up in the sweep's own order, a point's level as soon
+ *    as its producers' are known (k_levels_flow); for the host set-up by
+ *    Kahn's layering (a point joins level L+1 when its last dependency leaves
  *    level L), with one kernel per level queued without host round trips.
  */
 #include <cuda_runtime.h>
@@ -778,83 +780,49 @@ __global__ void k_ent_fill(int nsw, bool forward, const int32_t *order, const in
     }
 }
 
-// levels by Kahn's layering over the sweep terms whose producer is swept
-__global__ void k_dep_count(int nsw, const int32_t *order, const int32_t *off, const SweepEntry *ent,
-                            const uint8_t *swept, int32_t *indeg, int32_t *rcnt) {
-    GRID_STRIDE(t, (size_t)nsw) {
-        const int p = order[t];
-        int c = 0;
-        for (int e = off[p]; e < off[p + 1]; ++e) {
-            const int k = ent[e].k;
-            if (!swept[k]) continue;
-            ++c;
-            atomicAdd(&rcnt[k], 1);
-        }
-        indeg[p] = c;
-    }
-}
-
-__global__ void k_dep_fill(int nsw, const int32_t *order, const int32_t *off, const SweepEntry *ent,
-                           const uint8_t *swept, const int32_t *roff, int32_t *rcur, int32_t *rlist) {
-    GRID_STRIDE(t, (size_t)nsw) {
-        const int p = order[t];
-        for (int e = off[p]; e < off[p + 1]; ++e) {
-            const int k = ent[e].k;
-            if (swept[k]) rlist[roff[k] + atomicAdd(&rcur[k], 1)] = p;
-        }
-    }
-}
-
-__global__ void k_level_keys(int nsw, const int32_t *order, const int32_t *level, uint32_t *key, int32_t *hist,
-                             int *cycle) {
+__global__ void k_level_keys(int nsw, const int32_t *order, const int32_t *level, uint32_t *key, int32_t *hist) {
     GRID_STRIDE(t, (size_t)nsw) {
         const int lv = level[order[t]];
-        if (lv < 0) {
-            atomicExch(cycle, 1);
-            key[t] = 0;
-            continue;
-        }
         key[t] = (uint32_t)lv;
         atomicAdd(&hist[lv], 1);
     }
 }
 
-// Kahn's layering in one block: the frontier of level L (count0[0] points
-// in front, from k_lv_roots) releases the dependents whose last producer it
-// holds into level L+1; a warp takes a frontier point and its lanes its
-// dependents.  The loop ends when a level releases nothing; it runs at most
-// nsw levels.
-__global__ void __launch_bounds__(1024) k_levels_block(int nsw, int32_t *front, int32_t *next, const int32_t *count0,
-                                                       const int32_t *roff, const int32_t *rlist, int32_t *indeg,
-                                                       int32_t *level) {
-    __shared__ int m, m_next;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    if (threadIdx.x == 0) {
-        m = count0[0];
-        m_next = 0;
-    }
-    __syncthreads();
-    for (int L = 0; L < nsw && m > 0; ++L) {
-        for (int f = warp; f < m; f += warps) {
-            const int p = front[f];
-            const int e1 = roff[p + 1];
-            for (int e = roff[p] + lane; e < e1; e += 32) {
-                const int q = rlist[e];
-                if (atomicSub(&indeg[q], 1) == 1) {
-                    level[q] = L + 1;
-                    next[atomicAdd(&m_next, 1)] = q;
+// level[p] = 1 + the deepest of the swept neighbours p's sweep reads (-1: none),
+// in the sweep's own order: a warp takes the order's next point and its lanes
+// poll the levels (-1: not yet known) of the point's slots.  A producer comes
+// earlier in the order, so a running warp has it and every poll ends; each is
+// bounded anyway.  What bounds the pass is a hop through L2 per level (about 1
+// us), where layering by Kahn's method in one block took 11 us a level: its
+// atomics, one per sweep term, all from one SM (handle of 250,620 points: 100
+// -> 69 ms, of 1.1M points 417 -> 281 ms).
+constexpr int LEVEL_SPINS = 1 << 21;
+__global__ void __launch_bounds__(128) k_levels_flow(int nsw, const int32_t *order, const uint32_t *need,
+                                                     const int32_t *slot_nbr, const uint8_t *swept, int32_t *level,
+                                                     int *counter, int *failed) {
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        int idx = 0;
+        if (lane == 0) idx = atomicAdd(counter, 1);
+        idx = __shfl_sync(0xffffffffu, idx, 0);
+        if (idx >= nsw) return;
+        const int p = order[idx];
+        int k = -1;
+        if (need[p] >> lane & 1u) k = slot_nbr[(size_t)p * MAX_SLOTS + lane];
+        int lv = -1;
+        if (k >= 0 && swept[k]) {
+            for (int spins = 0;; ++spins) {
+                asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(lv) : "l"(level + k) : "memory");
+                if (lv >= 0) break;
+                if (spins > LEVEL_SPINS || ((spins & 1023) == 1023 && *(volatile int *)failed)) {
+                    atomicExch(failed, 1);
+                    lv = 0;
+                    break;
                 }
             }
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            m = m_next;
-            m_next = 0;
-        }
-        int32_t *t = front;
-        front = next;
-        next = t;
-        __syncthreads();
+        const int deepest = __reduce_max_sync(0xffffffffu, lv);
+        if (lane == 0) asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(level + p), "r"(deepest + 1) : "memory");
     }
 }
 
@@ -1289,42 +1257,30 @@ int device_setup(int device, const mfcfd_params &P, Topology &T, const double *x
         }
         dt.n_ent[dir] = ne;
 
-        // levels: the longest path over swept producers (Kahn's layering)
+        // levels: the longest path over swept producers
         DS_KEEP(dt.level[dir], n);
         PREP_CK(cudaMemsetAsync(dt.level[dir], 0xff, 4 * (size_t)n, s));
         DS_KEEP(lpts_dir[dir], nsw);
         std::vector<int32_t> hist;
         if (nsw > 0) {
-            int32_t *indeg, *rcnt, *roff, *rcur, *rlist, *fa, *fb, *count, *hcnt;
+            int32_t *hcnt;
             uint32_t *key, *key_sorted;
-            int *cycle;
-            DS_TMP(indeg, n); DS_TMP(rcnt, (size_t)n + 1); DS_TMP(roff, (size_t)n + 1); DS_TMP(rcur, n);
-            DS_TMP(rlist, ne); DS_TMP(fa, nsw); DS_TMP(fb, nsw); DS_TMP(count, (size_t)nsw + 2);
-            DS_TMP(hcnt, (size_t)nsw + 1); DS_TMP(key, nsw); DS_TMP(key_sorted, nsw); DS_TMP(cycle, 1);
-            PREP_CK(cudaMemsetAsync(rcnt, 0, 4 * ((size_t)n + 1), s));
-            PREP_CK(cudaMemsetAsync(rcur, 0, 4 * (size_t)n, s));
-            PREP_CK(cudaMemsetAsync(count, 0, 4 * ((size_t)nsw + 2), s));
+            int *work;                     // next point of the order, failure
+            DS_TMP(hcnt, (size_t)nsw + 1); DS_TMP(key, nsw); DS_TMP(key_sorted, nsw); DS_TMP(work, 2);
             PREP_CK(cudaMemsetAsync(hcnt, 0, 4 * ((size_t)nsw + 1), s));
-            PREP_CK(cudaMemsetAsync(cycle, 0, sizeof(int), s));
-            k_dep_count<<<gs, PREP_THREADS, 0, s>>>(nsw, order[dir], off_dir[dir], ent_dir[dir], swept, indeg, rcnt);
-            int ndep = 0;
-            if (int rc = scan(rcnt, roff, n + 1, &ndep)) return rc;
-            k_dep_fill<<<gs, PREP_THREADS, 0, s>>>(nsw, order[dir], off_dir[dir], ent_dir[dir], swept, roff, rcur,
-                                                   rlist);
-            // one thread per point of the order (k_lv_roots has no grid-stride loop)
-            k_lv_roots<<<(nsw + PREP_THREADS - 1) / PREP_THREADS, PREP_THREADS, 0, s>>>(order[dir], nsw, indeg,
-                                                                                     dt.level[dir], fa, count);
-            // every level in one block: a barrier per level instead of a launch
-            k_levels_block<<<1, 1024, 0, s>>>(nsw, fa, fb, count, roff, rlist, indeg, dt.level[dir]);
+            PREP_CK(cudaMemsetAsync(work, 0, 2 * sizeof(int), s));
+            const int blocks = std::min((nsw + 3) / 4, 8 * device_sms(device));
+            k_levels_flow<<<blocks, 128, 0, s>>>(nsw, order[dir], need_dir[dir], slot_nbr, swept, dt.level[dir], work,
+                                                 work + 1);
             PREP_CK(cudaGetLastError());
-            k_level_keys<<<gs, PREP_THREADS, 0, s>>>(nsw, order[dir], dt.level[dir], key, hcnt, cycle);
+            k_level_keys<<<gs, PREP_THREADS, 0, s>>>(nsw, order[dir], dt.level[dir], key, hcnt);
             PREP_CK(cudaGetLastError());
-            int h_cycle = 0;
-            PREP_CK(cudaMemcpyAsync(&h_cycle, cycle, sizeof(int), cudaMemcpyDeviceToHost, s));
+            int failed = 0;
+            PREP_CK(cudaMemcpyAsync(&failed, work + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
             PREP_CK(cudaStreamSynchronize(s));
-            if (h_cycle) {
-                err = "sweep dependencies contain a cycle";
-                return MFCFD_ERR_STENCIL;
+            if (failed) {
+                err = "a wait of the level pass ran out";
+                return MFCFD_ERR_TIMEOUT;
             }
             // points of each level in the sweep's order
             if (int rc = sort_pairs(key, key_sorted, order[dir], lpts_dir[dir], nsw, s, tmp, err)) return rc;
