@@ -61,11 +61,12 @@ def test_team_sweeps_equal_the_level_schedule(mfcfd_lib, case, warps):
         s.close()
 
 
-def test_ieee_functions_equal_the_operators(tmp_path):
-    """mfcfd_ieee.cuh against the FP64 operators (tests/ieee_check.cu): no
+@pytest.mark.parametrize("name,args", [("ieee_check", ["128"]), ("flux_check", [])])
+def test_straight_line_functions_equal_the_operators(tmp_path, name, args):
+    """mfcfd_ieee.cuh and state_flux against the operators (tests/NAME.cu): no
     result differs."""
-    exe = str(tmp_path / "ieee_check")
+    exe = str(tmp_path / name)
     subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-fmad=false", "-o", exe,
-                    os.path.join(REPO, "tests", "ieee_check.cu")], check=True)
-    out = subprocess.run([exe, "128"], capture_output=True, text=True)
+                    os.path.join(REPO, "tests", name + ".cu")], check=True)
+    out = subprocess.run([exe] + args, capture_output=True, text=True)
     assert out.returncode == 0, out.stdout + out.stderr
