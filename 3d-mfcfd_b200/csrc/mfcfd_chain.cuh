@@ -393,8 +393,7 @@ __device__ __noinline__ void unshared_terms(const DevCloud &d, ChainItem it, con
     bool ok = true;
     R yspb;
     state_core(U, Fk, Fp, P, yspb, ok);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) axis_core(P.ut(a), P.sb, P.spb, yspb, A[a], ok);
+    axes_core(P, yspb, A, ok);
     if (!__all_sync(FULL, ok || !mine)) {
         R Uc[5] = {U[0], U[1], U[2], U[3], U[4]};
         FrameT<R> Fkc = Fk, Fpc = Fp;
@@ -483,7 +482,7 @@ __device__ __forceinline__ void common_point(const DevCloud &d, const ChainItem 
 #pragma unroll
         for (int r = 0; r < 7; ++r) g[r] = st->geo[dd * 8 + r];
         if (wall && dd == 4) g[6] = 1.0;              // a list walls do not have
-        ok = ok && ieee_ok(fabs(g[6]));
+        ok &= ieee_ok(fabs(g[6]));
         ydet = rcp_rn(g[6]);
     }
     double *out = (forward ? d.dgf : d.dgb) + (DG_LIST * dd + c);
@@ -507,7 +506,7 @@ __device__ __forceinline__ void common_point(const DevCloud &d, const ChainItem 
     double G = s.x;
     if constexpr (!FOLD) {
         const double num = cramer_select(dd >> 1, g, s.x, s.y, s.z);
-        ok = ok && ieee_num_ok(num);
+        ok &= ieee_num_ok(num);
         G = quot_rn(num, g[6], ydet);
     }
     double gd[NDIR];

@@ -452,8 +452,7 @@ __device__ __forceinline__ void end_core(const DevCloud &d, int j, double delx, 
     }
     prim_core(qt, prim, ok);
     pre_core(prim, F, P, yspb, ok);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) axis_core(P.ut(a), P.sb, P.spb, yspb, A[a], ok);
+    axes_core(P, yspb, A, ok);
 }
 template <typename R>
 __device__ __forceinline__ void end_general(const DevCloud &d, int j, R delx, R dely, R delz, const FrameT<R> &F,
@@ -500,13 +499,15 @@ __device__ __noinline__ void end_terms_general(const DevCloud &d, int p, int j, 
     end_terms<double>(cls, mask, lane, P, A, second, T);
 }
 
-// Bound by the FP64 pipe (47% busy) and the latency of the ends' gathers at 16
-// warps per SM.  Blocks per SM the compiler must fit: four in FP64 (128
+// Bound by the FP64 pipe (54% busy) and the latency of the ends' gathers at 16
+// warps per SM (prefetches into L1 for the neighbour's end or the next point
+// gained nothing).  Blocks per SM the compiler must fit: four in FP64 (128
 // registers; 1.1M points: three are 20% slower, five 6%), five in FP32 (62,400
 // points: 0.25 ms against 0.32 with four).  The pair's ends go through one copy
 // of the code: with both ends' code in a row the loop overran the instruction
-// cache (1.1M points: 9.4 against 7.9 ms).  With the branch-free functions and
-// storage order, 1.1M points take 5.95 ms against 10.7 ms before.
+// cache (1.1M points: 9.4 against 7.9 ms).  With the branch-free functions,
+// storage order and the three axes side by side, 1.1M points take 5.35 ms
+// against 10.7 ms before.
 template <typename R>
 constexpr int flux_blocks() { return sizeof(R) == 8 ? 4 : 5; }
 

@@ -2,8 +2,8 @@
  * A point's own flux as the sweep evaluates it (state_flux) against the
  * general form with the operators (state_flux_general), bit for bit, in the
  * global axes: random densities, pressures and directions, Mach numbers from 0
- * to 4 (every piece of erf), and states next to those where it hands over to
- * the general form; and the quotient and root that start from the quotient's
+ * to 4 (every piece of erf up to 3.4); the three axes' half-range terms in other
+ * axes (axes_core); and the quotient and root that start from the quotient's
  * approximation against the operators.  Prints the counts and returns 1 if any
  * differs or too few states were taken.
  */
@@ -52,6 +52,21 @@ __global__ void check(int n, unsigned long long *out) {
     }
     atomicAdd(out, (unsigned long long)taken);
     if (wrong) atomicAdd(out + 1, (unsigned long long)wrong);
+    // the three axes' terms in turned axes
+    FrameT<R> H;
+    for (int r = 0; r < 3; ++r) { H.t1[r] = (R)(r == 1 ? 0.6 : r == 2 ? 0.8 : 0); H.t2[r] = r == 0; H.n[r] = (R)(r == 1 ? 0.8 : r == 2 ? -0.6 : 0); }
+    const R prim[5] = {(R)rho, (R)v[0], (R)v[1], (R)v[2], (R)p};
+    FluxPreT<R> P, Q;
+    AxisTermsT<R> A[3], B[3];
+    R ysp;
+    bool ok = true;
+    pre_core(prim, H, P, ysp, ok);
+    axes_core(P, ysp, A, ok);
+    flux_pre(prim, H, Q);
+    for (int a = 0; a < 3; ++a) {
+        axis_terms(Q, a, B[a]);
+        if (!ok || !same(A[a].B, B[a].B) || !same(A[a].Ap, B[a].Ap) || !same(A[a].An, B[a].An)) atomicAdd(out + 1, 1ull);
+    }
     if constexpr (sizeof(R) == 8) {
         double q0;
         const double q = quot_seed(0.5 * rho, p, q0), x = MF_PI * q;
