@@ -36,3 +36,18 @@ def test_knn_device_rejects_duplicates(mfcfd_lib):
     x = np.array([0.0, 1.0, 1.0, 2.0, 3.0])
     with pytest.raises(MfcfdError, match="coincide"):
         cloud.knn(x, np.zeros(5), np.zeros(5), 2, device=0)
+
+
+@pytest.mark.parametrize("n", [2, 28, 32, 33, 65, 256, 257, 2049, 16385])
+def test_knn_device_equals_host_at_leaf_and_node_edges(mfcfd_lib, n):
+    # a leaf is 32 points, a node 8 leaves or nodes; clustered points make the
+    # leaves' boxes overlap, equal distances are broken by index
+    rng = np.random.default_rng(n)
+    p = rng.standard_normal((n, 3)) * 10.0 ** rng.integers(-3, 2, (n, 1))
+    p[::3] = np.round(p[::3], 2) + np.arange(0, n, 3)[:, None]
+    for k in (1, 5, 26, 27):
+        if k >= n:
+            continue
+        h, d = _both(*p.T.copy(), k)
+        for a, b in zip(h, d):
+            assert np.array_equal(a, b), k
