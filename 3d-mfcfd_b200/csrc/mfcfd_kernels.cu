@@ -439,16 +439,17 @@ __global__ void __launch_bounds__(QD_THREADS) k_qderiv(const __grid_constant__ D
 // mixed precision); the offsets, weights, list sums and 3x3 solves are double.
 // One end j of a neighbour pair in straight-line code (reconstruct, flux_pre,
 // axis_terms); ok is cleared where an argument is out of its range.
-__device__ __forceinline__ void end_core(const DevCloud &d, int j, double delx, double dely, double delz, const Frame &F,
-                                         FluxPreT<double> &P, AxisTermsT<double> A[3], bool &ok) {
+template <typename R>
+__device__ __forceinline__ void end_core(const DevCloud &d, int j, R delx, R dely, R delz, const FrameT<R> &F, FluxPreT<R> &P,
+                                         AxisTermsT<R> A[3], bool &ok) {
     const double *qj = d.q + 5 * (size_t)j, *dqj = d.dq + 15 * (size_t)j, *qmj = d.qm + 10 * (size_t)j;
-    const double eps2 = d.eps2[j];
-    double qt[5], prim[5], yspb;
+    const R eps2 = (R)d.eps2[j];
+    R qt[5], prim[5], yspb;
 #pragma unroll
     for (int r = 0; r < 5; ++r) {
-        const double q = qj[r];
-        const double temp = delx * dqj[3 * r] + dely * dqj[3 * r + 1] + delz * dqj[3 * r + 2];
-        qt[r] = q - 0.5 * limiter_core(q, temp, qmj[2 * r], qmj[2 * r + 1], eps2, ok) * temp;
+        const R q = (R)qj[r];
+        const R temp = delx * (R)dqj[3 * r] + dely * (R)dqj[3 * r + 1] + delz * (R)dqj[3 * r + 2];
+        qt[r] = q - R(0.5) * limiter_core(q, temp, (R)qmj[2 * r], (R)qmj[2 * r + 1], eps2, ok) * temp;
     }
     prim_core(qt, prim, ok);
     pre_core(prim, F, P, yspb, ok);
@@ -489,25 +490,27 @@ __device__ __forceinline__ void end_terms(int cls, int mask, int lane, const Flu
 
 // The terms with the operators, where an end's arguments left the range of the
 // straight-line code.
-__device__ __noinline__ void end_terms_general(const DevCloud &d, int p, int j, double delx, double dely, double delz,
-                                               int cls, int mask, int lane, bool second, double *T) {
-    Frame F;
+template <typename R>
+__device__ __noinline__ void end_terms_general(const DevCloud &d, int p, int j, R delx, R dely, R delz, int cls, int mask,
+                                               int lane, bool second, double *T) {
+    FrameT<R> F;
     load_frame(d.frame + 9 * (size_t)p, F);
-    FluxPre P;
-    AxisTerms A[3];
-    end_general<double>(d, j, delx, dely, delz, F, P, A);
-    end_terms<double>(cls, mask, lane, P, A, second, T);
+    FluxPreT<R> P;
+    AxisTermsT<R> A[3];
+    end_general<R>(d, j, delx, dely, delz, F, P, A);
+    end_terms<R>(cls, mask, lane, P, A, second, T);
 }
 
-// Bound by the FP64 pipe (54% busy) and the latency of the ends' gathers at 16
+// Bound by the FP64 pipe (58% busy) and the latency of the ends' gathers at 16
 // warps per SM (prefetches into L1 for the neighbour's end or the next point
 // gained nothing).  Blocks per SM the compiler must fit: four in FP64 (128
 // registers; 1.1M points: three are 20% slower, five 6%), five in FP32 (62,400
-// points: 0.25 ms against 0.32 with four).  The pair's ends go through one copy
-// of the code: with both ends' code in a row the loop overran the instruction
-// cache (1.1M points: 9.4 against 7.9 ms).  With the branch-free functions,
-// storage order and the three axes side by side, 1.1M points take 5.35 ms
-// against 10.7 ms before.
+// points: 0.26 ms against 0.28 with four and 0.26 with six).  The pair's ends go
+// through one copy of the code: with both ends' code in a row the loop overran
+// the instruction cache (1.1M points: 9.4 against 7.9 ms).  With the branch-free
+// functions, storage order, the three axes side by side and the list's entries
+// and moments read before the sums, 1.1M points take 5.0 ms against 10.7 ms
+// before; 250k points in FP32 0.97 ms.
 template <typename R>
 constexpr int flux_blocks() { return sizeof(R) == 8 ? 4 : 5; }
 
@@ -547,15 +550,14 @@ __global__ void __launch_bounds__(FLUX_WARPS * 32, flux_blocks<R>()) k_flux(cons
     double *W = T + NDIR * MAX_SLOTS * 5;             // W[slot*3 + axis]
     const int dd = lane / 5, c = lane - 5 * (lane / 5);
     for (int p = (blockIdx.x - first) * FLUX_WARPS + warp; p < d.n; p += (gridDim.x - first) * FLUX_WARPS) {
-        const int cls = d.cls[p];
+        // read together: each would be a round trip of its own
+        const int cls = d.cls[p], slots = d.nslot[p];
+        const int slot_k = d.slot_nbr[(size_t)p * MAX_SLOTS + lane], slot_m = d.slot_mask[(size_t)p * MAX_SLOTS + lane];
         if (cls <= 2) {
             // lanes without a slot take the point itself and no list
-            const bool have = lane < d.nslot[p];
-            const int k = have ? d.slot_nbr[(size_t)p * MAX_SLOTS + lane] : p;
-            const int mask = have ? d.slot_mask[(size_t)p * MAX_SLOTS + lane] : 0;
-            // the lane's list (up to 27 entries of a byte, 28 apart)
-            const int cnt = lane < 30 ? d.list_cnt[(size_t)p * NDIR + dd] : 0;
-            const uint32_t *ent = reinterpret_cast<const uint32_t *>(d.list_ent + ((size_t)p * NDIR + (lane < 30 ? dd : 0)) * LIST_STRIDE);
+            const bool have = lane < slots;
+            const int k = have ? slot_k : p;
+            const int mask = have ? slot_m : 0;
             Frame F;
             load_frame(d.frame + 9 * (size_t)p, F);
             const double delx = d.pos[4 * (size_t)k] - d.pos[4 * (size_t)p], dely = d.pos[4 * (size_t)k + 1] - d.pos[4 * (size_t)p + 1],
@@ -570,38 +572,46 @@ __global__ void __launch_bounds__(FLUX_WARPS * 32, flux_blocks<R>()) k_flux(cons
                 const int j = e ? k : p;
                 FluxPreT<R> P;
                 AxisTermsT<R> A[3];
-                if constexpr (sizeof(R) == 8) {
-                    bool ok = true;
-                    end_core(d, j, delx, dely, delz, F, P, A, ok);
-                    if (__all_sync(FULL, ok || !have)) end_terms<double>(cls, mask, lane, P, A, e != 0, T);
-                    else end_terms_general(d, p, j, delx, dely, delz, cls, mask, lane, e != 0, T);
-                } else {
-                    FrameT<R> FR;
+                FrameT<R> FR;
 #pragma unroll
-                    for (int r = 0; r < 3; ++r) { FR.t1[r] = (R)F.t1[r]; FR.t2[r] = (R)F.t2[r]; FR.n[r] = (R)F.n[r]; }
-                    end_general<R>(d, j, (R)delx, (R)dely, (R)delz, FR, P, A);
-                    end_terms<R>(cls, mask, lane, P, A, e != 0, T);
-                }
+                for (int r = 0; r < 3; ++r) { FR.t1[r] = (R)F.t1[r]; FR.t2[r] = (R)F.t2[r]; FR.n[r] = (R)F.n[r]; }
+                bool ok = true;
+                end_core<R>(d, j, (R)delx, (R)dely, (R)delz, FR, P, A, ok);
+                if (__all_sync(FULL, ok || !have)) end_terms<R>(cls, mask, lane, P, A, e != 0, T);
+                else end_terms_general<R>(d, p, j, (R)delx, (R)dely, (R)delz, cls, mask, lane, e != 0, T);
             }
+            // the lane's list (up to 27 entries of a byte, 28 apart), its first
+            // entries and its moments, all before the sums that wait for them
+            const int dl = lane < 30 ? dd : 0;
+            const int cnt = lane < 30 ? d.list_cnt[(size_t)p * NDIR + dl] : 0;
+            const uint32_t *ent = reinterpret_cast<const uint32_t *>(d.list_ent + ((size_t)p * NDIR + dl) * LIST_STRIDE);
+            uint32_t e4[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) e4[q] = ent[q];
+            const double *gp = d.geo + (size_t)p * GEO_STRIDE + dl * 8;
+            double g[7];
+#pragma unroll
+            for (int r = 0; r < 7; ++r) g[r] = gp[r];
             __syncwarp();
             double G = 0.0;
             if (lane < 30) {
                 double sx = 0.0, sy = 0.0, sz = 0.0;
                 const double *t = T + dd * MAX_SLOTS * 5 + c;
-                for (int j = 0; j < cnt; j += 4) {
-                    const uint32_t e4 = ent[j >> 2];
+                auto add = [&](uint32_t w, int j) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         if (j + q < cnt) {
-                            const int s = (e4 >> (8 * q)) & 255;
+                            const int s = (w >> (8 * q)) & 255;
                             const double v = t[s * 5];
                             sx = sx + v * W[s * 3 + 0];
                             sy = sy + v * W[s * 3 + 1];
                             sz = sz + v * W[s * 3 + 2];
                         }
                     }
-                }
-                const double *g = d.geo + (size_t)p * GEO_STRIDE + dd * 8;
+                };
+#pragma unroll
+                for (int q = 0; q < 4; ++q) add(e4[q], 4 * q);
+                for (int j = 16; j < cnt; j += 4) add(ent[j >> 2], j);
                 const double num = cramer_select(dd >> 1, g, sx, sy, sz), det = g[G_DET];
                 // outer_flux_dG*.f90:118-124 multiply by 1/det; the others divide
                 const double y = rcp_rn(det);
@@ -1169,8 +1179,8 @@ namespace mfcfd {
 // blocks of the chain sweeps running at once have to fit the device together.
 // They are counted in slots of a sixth of an SM: a 4-warp block takes 2 in
 // mixed precision (three per SM: at most 168 registers and 76 KB of shared
-// memory), 3 in FP64 (two per SM: 234 registers, no spills), or 2 in the dense
-// FP64 build (168 registers, 20 bytes spilled), which a cloud takes whose teams
+// memory), 3 in FP64 (two per SM: 254 registers, no spills), or 2 in the dense
+// FP64 build (168 registers, 100 bytes spilled), which a cloud takes whose teams
 // need more than two blocks per SM (1.1M points, 376 teams of four: 37.0 ms
 // per iteration against 41.5 as teams of two on more chains).  The sweeps at
 // once take at most 6 * (SMs - CH_FREE_SMS) slots; the other SMs' room is for

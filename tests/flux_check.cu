@@ -3,7 +3,8 @@
  * general form with the operators (state_flux_general), bit for bit, in the
  * global axes: random densities, pressures and directions, Mach numbers from 0
  * to 4 (every piece of erf up to 3.4); the three axes' half-range terms in other
- * axes (axes_core); and the quotient and root that start from the quotient's
+ * axes (axes_core); the reconstruction's limiter and primitive state; and the
+ * quotient and root that start from the quotient's
  * approximation against the operators.  Prints the counts and returns 1 if any
  * differs or too few states were taken.
  */
@@ -67,10 +68,34 @@ __global__ void check(int n, unsigned long long *out) {
         axis_terms(Q, a, B[a]);
         if (!ok || !same(A[a].B, B[a].B) || !same(A[a].Ap, B[a].Ap) || !same(A[a].An, B[a].An)) atomicAdd(out + 1, 1ull);
     }
+    // q -> primitive, and the limiter near its threshold and its ratio of one
+    const double be = 0.5 * rho / p;
+    const R qt[5] = {(R)(log(rho) + 2.5 * log(be) - be * u * u), (R)(2 * be * v[0]), (R)(2 * be * v[1]), (R)(2 * be * v[2]),
+                     (R)(-2 * be)};
+    R pa[5], pb[5];
+    ok = true;
+    prim_core(qt, pa, ok);
+    qtilde_to_primitive(qt, pb);
+    for (int r = 0; ok && r < 5; ++r)
+        if (r && !same(pa[r], pb[r]) || !same(pa[0], pb[0])) atomicAdd(out + 1, 1ull);
+    const R q = qt[0], temp = (R)(exp2(-30 * rnd(s)) * (rnd(s) < 0.5 ? -1 : 1)), eps2 = (R)(1e-6 * rnd(s));
+    const R hi = (R)(q + (rnd(s) < 0.2 ? 0 : exp2(-25 * rnd(s)))), lo = (R)(q - (rnd(s) < 0.2 ? 0 : exp2(-25 * rnd(s))));
+    ok = true;
+    const R phi = limiter_core(q, temp, hi, lo, eps2, ok);
+    const R neg = (q - R(0.5) * temp) - q, pos = neg > R(0) ? hi - q : lo - q;
+    R want = R(1);
+    if (!(r_abs(neg) <= R(MF_LIM_EPS))) {
+        R num = (pos * pos) + eps2, den = pos * pos + R(2) * neg * neg;
+        num = num * neg + R(2) * neg * neg * pos;
+        den = den + neg * pos + eps2;
+        den = den * neg;
+        want = num / den < R(1) ? num / den : R(1);
+    }
+    if (ok && !same(phi, want)) atomicAdd(out + 1, 1ull);
     if constexpr (sizeof(R) == 8) {
         double q0;
-        const double q = quot_seed(0.5 * rho, p, q0), x = MF_PI * q;
-        if (!same(q, 0.5 * rho / p) || !same(sqrt_from(q, rsqrt_seed(q0)), sqrt(q)) ||
+        const double qb = quot_seed(0.5 * rho, p, q0), x = MF_PI * qb;
+        if (!same(qb, 0.5 * rho / p) || !same(sqrt_from(qb, rsqrt_seed(q0)), sqrt(qb)) ||
             !same(sqrt_from(x, rsqrt_seed(MF_PI * q0)), sqrt(x)))
             atomicAdd(out + 2, 1ull);
         // all-ones denominators, and numerators next to a quotient's midpoint
