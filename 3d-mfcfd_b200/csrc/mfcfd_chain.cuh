@@ -12,12 +12,12 @@
  * arithmetic of one point (remaining sums, solve, own flux) and a
  * shared-memory hand-off, not the fetches around it.  Measured (B200, FP64,
  * both sweeps of an iteration; before: one warp per chain, which did all of a
- * point's work in turn): 62,400 points 13.6 -> 5.05 ms (1.4 us per level),
- * 1.1M points 49.6 -> 20.6 ms, mixed precision at 62,400 11.4 -> 3.8 ms.  On
- * the critical path of the 62,400-point sweep three hops in four are from a
- * chain's point to its next (1.0 us: its own flux about 1,100 cycles, the sums
+ * point's work in turn): 62,400 points 13.6 -> 4.6 ms (1.25 us per level),
+ * 1.1M points 49.6 -> 19.4 ms, mixed precision at 62,400 11.4 -> 3.5 ms.  On
+ * the critical path of the 62,400-point sweep seven hops in ten are from a
+ * chain's point to its next (0.86 us: its own flux about 855 cycles, the sums
  * after the ring term 150, the solve 150, the rest of dU 165), one in four to
- * another chain through L2 (1.8 us), one in thirty to a wall point (3.6 us).
+ * another chain through L2 (1.9 us), one in thirteen at a wall point (3.5 us).
  *
  * Ring.  The team's last increments lie in a shared ring of TEAM_RING slots of
  * 32 words (lane l's component), one per position (a team of one warp:
@@ -231,6 +231,9 @@ struct Sums {
 // the terms before it are added, and the products of the AFTER terms after
 // it formed, before the wait for its word.  Straight-line code with predicated
 // loads and sums: a divergent branch per term costs more than the term.
+// (GATHER, AFTER) measured at 62,400 points, ms per iteration: (16, 8) 4.99,
+// (12, 8) 5.25, (8, 8) 6.40, (20, 8) 5.13, (16, 6) 5.11, (16, 10) 4.99 (1.1M
+// points: 25.9 against 25.4).
 constexpr int AFTER = 8;
 template <bool FOLD>
 __device__ __forceinline__ void shared_sums(const DevCloud &d, const SweepEntry *E, int n, const double *src,

@@ -151,12 +151,12 @@ constexpr int CHAIN_RING = 8;           // increments a warp keeps in shared mem
 constexpr int DG_STRIDE = 36;
 constexpr int DG_LIST = 6;
 
-// Static warp assignment of the sweep points for the chain schedule: warp
-// lists (CSR, each in topological order), the owner warp of every point and
-// the per-point records, per direction.  A point goes to the warp that just
-// processed its deepest dependency when that warp is free to continue, so
-// critical chains stay inside one warp; otherwise to the warp idle the
-// longest.  The builder also marks each term of T's entry lists with where
+// Static assignment of the sweep points to the chain schedule's chains: their
+// lists (CSR, each in topological order), the owner chain of every point and
+// the per-point records, per direction.  A point goes to the chain that just
+// processed its deepest dependency when that chain is free to continue, so
+// critical paths stay inside one team of warps; otherwise to the chain idle
+// the longest.  The builder also marks each term of T's entry lists with where
 // its producer's increment comes from (ENT_* bits).
 struct ChainSchedule {
     int warps = 0;

@@ -1644,8 +1644,8 @@ cudaError_t launch_conserved_q(const DevCloud &d, cudaStream_t s) {
 }
 
 // A launch with an explicit scheduling priority.  The chain sweep must have
-// its blocks placed before those of the flux kernel beside it (which never
-// waits, so it cannot hold the sweep up for good); the priority travels with
+// its blocks placed before those of other handles' flux kernels (which never
+// wait, so they cannot hold the sweep up for good); the priority travels with
 // the launch, so it holds in a captured graph as on a stream.
 template <typename... Args, typename... Act>
 static cudaError_t launch_prio(void (*kern)(Args...), int grid, int block, size_t smem, cudaStream_t s, bool high,
