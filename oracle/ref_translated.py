@@ -43,7 +43,7 @@ def build(reference_dir: str = None) -> bool:
     reference is absent and nothing was built before."""
     if reference_dir is None:
         reference_dir = os.environ.get(REF_DIR_ENV, "")
-    if not reference_dir or not os.path.isdir(reference_dir):
+    if not reference_dir or not os.path.isdir(reference_dir) or not os.listdir(reference_dir):
         return all(os.path.exists(p) for p in _LIBS.values())
     out_c = os.path.join(_HERE, "_ref", "ref_translated.c")
     subprocess.run(["python", os.path.join(_HERE, "f2c_ref.py"), reference_dir, out_c],
