@@ -7,7 +7,6 @@
  */
 #include <algorithm>
 #include <chrono>
-#include <condition_variable>
 #include <deque>
 #include <thread>
 #include <cmath>
@@ -22,6 +21,27 @@
 #include "mfcfd_internal.h"
 
 using namespace mfcfd;
+
+// The slots of a running chunk, held until the stream that runs it is idle: an
+// error or an exception on the way does not free them under its sweeps.
+struct ChunkSlots {
+    SlotPool::Lease lease;
+    cudaStream_t stream = nullptr;
+    ChunkSlots() = default;
+    ChunkSlots(SlotPool::Lease &&l, cudaStream_t s) : lease(std::move(l)), stream(s) {}
+    ChunkSlots(ChunkSlots &&) = default;
+    ChunkSlots &operator=(ChunkSlots &&o) {
+        end();
+        lease = std::move(o.lease);
+        stream = o.stream;
+        return *this;
+    }
+    ~ChunkSlots() { end(); }
+    void end() {
+        if (lease) cudaStreamSynchronize(stream);
+        lease = SlotPool::Lease();
+    }
+};
 
 struct mfcfd_handle {
     mfcfd_params P;
@@ -68,7 +88,7 @@ struct mfcfd_handle {
     int graph_next = 0;
     cudaEvent_t batch_ev = nullptr;        // end of the handle's chunk in mfcfd_run_batch / mfcfd_launch
     int pending_chunk = 0;                 // mfcfd_launch: iterations not yet completed
-    int held = 0, held_budget = 0;         // slots of the running chunk, and its budget of them
+    ChunkSlots pending_slots;              // ... and their slots
     // chain schedule: the warps it may hold beside other handles' (in blocks
     // of ch_wpb); DevCloud::ch_shape is the shape of the running chunk
     int ch_budget = 0, ch_wpb = 0;
@@ -189,14 +209,10 @@ void drop_graphs(mfcfd_handle *h) {
     }
 }
 
-void give_slots(mfcfd_handle *h);
-
 void release(mfcfd_handle *h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
-    if (h->pending_chunk) {                // launched and never completed
-        give_slots(h);
-        h->pending_chunk = 0;
-    }
+    h->pending_slots.end();                // launched and never completed
+    h->pending_chunk = 0;
     drop_graphs(h);
     for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
     h->ev.clear();
@@ -240,70 +256,23 @@ int launch_one(mfcfd_handle *h, int j) {
     return MFCFD_OK;
 }
 
-// Slots of a device's chain sweeps in use (chain_slot_capacity), over every
-// handle and thread of the process.  A run holds at least its handles'
-// budgets (mfcfd_info.chain_slots), whose sum over concurrent runs is the
-// callers' to bound; a run of mfcfd_run, mfcfd_run_batch, mfcfd_run_group or
-// the request server may hold more while nobody needs it, for one chunk of
-// iterations at a time, and whoever does not find room for its budget beside
-// such a run waits for that chunk.
-struct SlotPool {
-    std::mutex mu;
-    std::condition_variable freed;
-    int used = 0, excess = 0;
-};
-SlotPool g_slots[256];
+SlotPool g_slots[256];                     // per device
 constexpr int EXCESS_CHUNK = 64;           // iterations a run beyond its budget lasts at most
 
-// Take slots for handles of these chain counts: the shape of their sweeps in
-// *shape (the largest teams within max(budget, min(want, what is free))).
-// Returns the slots held; -1, with `wait` false, instead of waiting (for a
-// caller that itself holds more than its budgets).
-int take_slots(int dev, const int *chains, int count, int precision, int spread, int budget, int want, bool wait,
-               ChainShape *shape) {
-    SlotPool &p = g_slots[dev & 255];
-    const int capacity = chain_slot_capacity(dev);
-    std::unique_lock<std::mutex> lock(p.mu);
-    auto room = [&] { return p.used + budget <= capacity || p.excess == 0; };
-    if (!wait && !room()) return -1;
-    p.freed.wait(lock, room);
-    *shape = chain_fit(chains, count, precision, spread, std::max(budget, std::min(want, capacity - p.used)));
-    int hold = 0;
-    for (int i = 0; i < count; ++i) hold += chain_slots(chains[i], *shape, precision);
-    hold = std::max(hold, budget);
-    p.used += hold;
-    p.excess += hold - budget;
-    return hold;
-}
-void give_slots(int dev, int budget, int hold) {
-    SlotPool &p = g_slots[dev & 255];
-    {
-        std::lock_guard<std::mutex> lock(p.mu);
-        p.used -= hold;
-        p.excess -= hold - budget;
-    }
-    p.freed.notify_all();
-}
 int budget_slots(const mfcfd_handle *h) {
     return h->d.sweep_mode == MFCFD_SWEEP_CHAINS
                ? chain_budget_slots(h->ch_budget, h->ch_wpb, h->d.precision, h->P.chain_spread)
                : 0;
 }
-// Slots of one handle's chunk (h->held; 0 for the other schedules), its shape
+// Slots for one handle's next chunk (none for the other schedules), its shape
 // set; false if it would have to wait.
-bool take_slots(mfcfd_handle *h, int want, bool wait) {
-    h->held = h->held_budget = 0;
+bool take_slots(mfcfd_handle *h, int want, bool wait, SlotPool::Lease *l) {
     if (h->d.sweep_mode != MFCFD_SWEEP_CHAINS) return true;
-    h->held_budget = budget_slots(h);
-    h->held = take_slots(h->P.device, &h->d.ch_chains, 1, h->d.precision, h->P.chain_spread, h->held_budget, want, wait,
-                         &h->d.ch_shape);
-    if (h->held >= 0) return true;
-    h->held = 0;
-    return false;
-}
-void give_slots(mfcfd_handle *h) {
-    if (h->held > 0) give_slots(h->P.device, h->held_budget, h->held);
-    h->held = 0;
+    const SlotAsk a{&h->d.ch_chains, 1, h->d.precision, h->P.chain_spread, budget_slots(h), want};
+    *l = g_slots[h->P.device & 255].take(chain_slot_capacity(h->P.device), a, wait);
+    if (!*l) return false;
+    h->d.ch_shape = l->shape();
+    return true;
 }
 
 // Launch the iterations of one chunk (slots 0 .. chunk-1).  With graphs, the
@@ -472,13 +441,12 @@ int run_iterations(mfcfd_handle *h, int32_t t0, int32_t iters, double *res_hist)
     if (!h->have_state) return fail(h, MFCFD_ERR_ARG, "no state: call mfcfd_set_prim first");
     int status = MFCFD_OK;
     for (int32_t done = 0; done < iters;) {
-        take_slots(h, 1 << 20, true);
+        ChunkSlots slots{SlotPool::Lease(), h->stream};
+        take_slots(h, 1 << 20, true, &slots.lease);
         int chunk = std::min<int32_t>(iters - done, h->res_cap);
-        if (h->held > h->held_budget) chunk = std::min(chunk, EXCESS_CHUNK);
+        if (slots.lease.lent()) chunk = std::min(chunk, EXCESS_CHUNK);
         int rc = launch_chunk(h, chunk, false);
-        if (rc) cudaStreamSynchronize(h->stream);
         if (!rc) rc = finish_chunk(h, t0 + done, chunk, res_hist ? res_hist + 2 * (size_t)done : nullptr, &status);
-        give_slots(h);
         if (rc) return rc;
         done += chunk;
     }
@@ -1057,18 +1025,14 @@ extern "C++" int mfcfd::launch_within(mfcfd_handle *h, int32_t t0, int32_t iters
         if (iters > h->res_cap) return fail(h, MFCFD_ERR_ARG, "at most 1024 iterations per launch");
         CK(cudaSetDevice(h->P.device));
         if (!h->batch_ev) CK(cudaEventCreateWithFlags(&h->batch_ev, cudaEventDisableTiming));
-        if (!take_slots(h, slots, wait)) return MFCFD_ERR_BUSY;
-        int rc = launch_chunk(h, iters, true);
-        const cudaError_t e = rc ? cudaSuccess : cudaEventRecord(h->batch_ev, h->stream);
-        if (e != cudaSuccess) rc = cuda_fail(h, e, "cudaEventRecord");
-        if (rc) {
-            cudaStreamSynchronize(h->stream);
-            give_slots(h);
-            return rc;
-        }
+        ChunkSlots taken{SlotPool::Lease(), h->stream};
+        if (!take_slots(h, slots, wait, &taken.lease)) return MFCFD_ERR_BUSY;
+        if (int rc = launch_chunk(h, iters, true)) return rc;
+        CK(cudaEventRecord(h->batch_ev, h->stream));
+        if (held) *held = taken.lease.slots();
+        h->pending_slots = std::move(taken);
         h->pending_chunk = iters;
         h->pending_t0 = t0;
-        if (held) *held = h->held;
         return MFCFD_OK;
     });
 }
@@ -1088,8 +1052,8 @@ int mfcfd_complete(mfcfd_handle *h, int32_t wait, double *res_hist, int32_t *don
         int st = MFCFD_OK;
         const int chunk = h->pending_chunk;
         h->pending_chunk = 0;
+        const ChunkSlots slots(std::move(h->pending_slots));
         int rc = finish_chunk(h, h->pending_t0, chunk, res_hist, &st);
-        give_slots(h);
         *done = 1;
         return rc ? rc : st;
     });
@@ -1273,6 +1237,14 @@ int mfcfd_debug_digest(mfcfd_handle *h, const char *name, uint64_t *digest, int6
     });
 }
 
+int mfcfd_debug_slots(int32_t device, int32_t *held) {
+    return host_guard(nullptr, [&]() -> int {
+        if (device < 0 || device > 255 || !held) return MFCFD_ERR_ARG;
+        *held = g_slots[device].held();
+        return MFCFD_OK;
+    });
+}
+
 int mfcfd_get_info(mfcfd_handle *h, mfcfd_info *info) {
     return host_guard(h ? &h->err : nullptr, [&]() -> int {
         if (!h || !info) return MFCFD_ERR_ARG;
@@ -1416,8 +1388,13 @@ int mfcfd_run_batch(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
         std::vector<int32_t> done(count, 0);
         std::vector<int> chunk_of(count, 0);
         std::deque<int32_t> ready;
+        // every launched chunk ends (and its slots return) before an error
+        // leaves the call
+        std::vector<ChunkSlots> slots(count);
         std::vector<int32_t> running;
+        running.reserve(count);
         for (int32_t i = 0; i < count; ++i) {
+            slots[i].stream = hs[i]->stream;
             if (iters > 0) ready.push_back(i);
             if (!hs[i]->batch_ev && cudaEventCreateWithFlags(&hs[i]->batch_ev, cudaEventDisableTiming) != cudaSuccess)
                 return cuda_fail(hs[i], cudaGetLastError(), "cudaEventCreateWithFlags");
@@ -1425,15 +1402,6 @@ int mfcfd_run_batch(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
         // each handle's share of the device, by its budget
         long budgets = 0;
         for (int32_t i = 0; i < count; ++i) budgets += budget_slots(hs[i]);
-        // every launched chunk ends (and its slots return) before an error
-        // leaves the call
-        auto drain = [&](int rc) {
-            for (const int32_t i : running) {
-                cudaStreamSynchronize(hs[i]->stream);
-                give_slots(hs[i]);
-            }
-            return rc;
-        };
         int used = 0;
         while (!ready.empty() || !running.empty()) {
             while (!ready.empty()) {
@@ -1441,16 +1409,16 @@ int mfcfd_run_batch(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
                 mfcfd_handle *h = hs[i];
                 if (!running.empty() && used + budget_slots(h) > capacity) break;
                 const int share = (int)std::min<long>(capacity, (long)capacity * budget_slots(h) / std::max(budgets, 1l));
-                if (!take_slots(h, share, running.empty())) break;
+                if (!take_slots(h, share, running.empty(), &slots[i].lease)) break;
                 ready.pop_front();
                 const int chunk = std::min<int32_t>(iters - done[i], std::max(h->res_cap, 1));
                 int rc = launch_chunk(h, chunk, true);
                 const cudaError_t e = rc ? cudaSuccess : cudaEventRecord(h->batch_ev, h->stream);
                 if (e != cudaSuccess) rc = cuda_fail(h, e, "cudaEventRecord");
+                if (rc) return rc;
                 running.push_back(i);
-                if (rc) return drain(rc);
                 chunk_of[i] = chunk;
-                used += h->held;
+                used += slots[i].lease.slots();
             }
             // wait for the first of the running chunks to complete
             int found = -1;
@@ -1458,17 +1426,17 @@ int mfcfd_run_batch(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
                 for (size_t r = 0; r < running.size() && found < 0; ++r) {
                     const cudaError_t q = cudaEventQuery(hs[running[r]]->batch_ev);
                     if (q == cudaSuccess) found = (int)r;
-                    else if (q != cudaErrorNotReady) return drain(cuda_fail(hs[running[r]], q, "cudaEventQuery"));
+                    else if (q != cudaErrorNotReady) return cuda_fail(hs[running[r]], q, "cudaEventQuery");
                 }
                 if (found < 0) std::this_thread::sleep_for(std::chrono::microseconds(20));
             }
             const int32_t i = running[found];
             running.erase(running.begin() + found);
-            used -= hs[i]->held;
+            used -= slots[i].lease.slots();
             int st = MFCFD_OK;
             double *rh = res_hist ? res_hist + 2 * ((size_t)i * iters + done[i]) : nullptr;
             int rc = finish_chunk(hs[i], t0[i] + done[i], chunk_of[i], rh, &st);
-            give_slots(hs[i]);
+            slots[i].end();
             if (!rc) rc = st;
             if (status && rc && status[i] == MFCFD_OK) status[i] = rc;
             if (rc && first_err == MFCFD_OK) first_err = rc;
@@ -1604,18 +1572,14 @@ int mfcfd_run_group(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
             graphs = graphs && hs[i]->P.graphs >= 1 && !hs[i]->graphs_off;
         }
         int first_err = MFCFD_OK;
-        // the group's slots for one chunk, returned on every path
-        struct Held {
-            int dev, budget, slots;
-            ~Held() { give_slots(dev, budget, slots); }
-        };
+        const SlotAsk ask{chains.data(), count, d0.precision, h0->P.chain_spread, slots, 1 << 20};
         for (int32_t done = 0; done < iters;) {
-            const Held held{dev, slots, take_slots(dev, chains.data(), count, d0.precision, h0->P.chain_spread, slots,
-                                                   1 << 20, true, &gr.shape)};
+            const ChunkSlots held(g_slots[dev & 255].take(chain_slot_capacity(dev), ask, true), gr.s);
+            gr.shape = held.lease.shape();
             G->block_start[0] = 0;
             for (int32_t i = 0; i < count; ++i)
                 G->block_start[i + 1] = G->block_start[i] + chain_blocks(chains[i], gr.shape);
-            const int chunk = std::min<int32_t>(iters - done, held.slots > slots ? std::min(res_cap, EXCESS_CHUNK) : res_cap);
+            const int chunk = std::min<int32_t>(iters - done, held.lease.lent() ? std::min(res_cap, EXCESS_CHUNK) : res_cap);
             for (int32_t i = 0; i < count; ++i) hs[i]->res_valid = false;
             std::vector<int> cur(count), last(count);
             for (int32_t i = 0; i < count; ++i) cur[i] = hs[i]->cur, last[i] = hs[i]->last;

@@ -38,7 +38,6 @@ namespace mfcfd {
 
 constexpr int TEAM_RING = 24;
 static_assert(TEAM_RING >= 3 * CHAIN_RING, "ring slots outlive their readers");
-constexpr int CH_WPB = 4;                // warps per block
 constexpr int GATHER = 16;               // terms of a list gathered at a time
 // ring slots of a team: a warp alone reads a slot before it writes it again
 __host__ __device__ constexpr int ring_slots(int team) { return team == 1 ? CHAIN_RING : TEAM_RING; }

@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/mfcfd.h"
+#include "mfcfd_slots.h"
 
 namespace mfcfd {
 
@@ -298,16 +299,6 @@ int build_topology(const mfcfd_params &P, int n, const int32_t *status, const do
                    const double *nor, const int32_t *nbhs, const int32_t *conn,
                    const double *min_dist, Topology &T, std::string &err);
 
-// Launch shape of a chain sweep: the warps that walk a chain together (1, 2 or
-// 4), the FP64 build for three blocks per SM instead of two, one block per SM
-// (mfcfd_params.chain_spread).
-struct ChainShape {
-    int team, dense, spread;
-};
-inline bool operator==(const ChainShape &a, const ChainShape &b) {
-    return a.team == b.team && a.dense == b.dense && a.spread == b.spread;
-}
-
 // Device-side views (plain pointers, passed to kernels by value).
 struct DevCloud {
     int n;
@@ -433,12 +424,6 @@ int chain_budget_slots(int budget, int wpb, int precision, int spread);
 // twice and 6.93 with once), at most what the device holds as teams of four
 // unless that is below 0.85 times the level, and at most the budget.
 int chain_count(int device, int budget, int width, int spread);
-// Blocks and slots of a chain sweep.
-int chain_blocks(int chains, const ChainShape &c);
-int chain_slots(int chains, const ChainShape &c, int precision);
-// The largest teams with which the sweeps of these chain counts fit `slots`
-// together; teams of one (which fit their budgets) if none does.
-ChainShape chain_fit(const int *chains, int count, int precision, int spread, int slots);
 // Whether the chain kernels hold the blocks per SM that the slots count on.
 bool chain_fits(int device, bool group);
 // Per-device launch set-up (kernel attributes), done before a stream capture.

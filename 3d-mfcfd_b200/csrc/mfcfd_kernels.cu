@@ -1583,30 +1583,6 @@ int chain_count(int device, int budget, int width, int spread) {
     return c < 1 ? 1 : c;
 }
 
-int chain_blocks(int chains, const ChainShape &c) { return (chains * c.team + CH_WPB - 1) / CH_WPB; }
-
-int chain_slots(int chains, const ChainShape &c, int precision) {
-    const int each = c.spread ? 6 : (precision != MFCFD_PRECISION_FP64 || c.dense ? 2 : 3);
-    return chain_blocks(chains, c) * each;
-}
-
-ChainShape chain_fit(const int *chains, int count, int precision, int spread, int slots) {
-    ChainShape c{};
-    c.spread = spread;
-    c.team = spread ? 1 : CH_WPB;
-    for (;; c.team /= 2) {
-        for (c.dense = 0; c.dense < 2; ++c.dense) {
-            int sum = 0;
-            for (int i = 0; i < count; ++i) sum += chain_slots(chains[i], c, precision);
-            if (sum <= slots) return c;
-            if (precision != MFCFD_PRECISION_FP64) break;
-        }
-        if (c.team == 1) break;
-    }
-    c.dense = 0;
-    return c;
-}
-
 // Rows [a, a + rows) of width w between the reference's index order and
 // the storage order: scatter puts row i of src (a transfer buffer in index
 // order) at storage row perm[a + i] of dst; gather does the reverse.

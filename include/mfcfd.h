@@ -338,6 +338,11 @@ int mfcfd_knn(int32_t device, int32_t n, const double *x, const double *y, const
  * the device. */
 int mfcfd_debug_digest(mfcfd_handle *h, const char *name, uint64_t *digest, int64_t *bytes);
 
+/* Diagnostics: the slots (mfcfd_info.chain_slots) that running chain sweeps of
+ * this process hold on a device; 0 once every run has returned and every
+ * launch is completed or its handle destroyed. */
+int mfcfd_debug_slots(int32_t device, int32_t *held);
+
 int mfcfd_get_info(mfcfd_handle *h, mfcfd_info *info);
 
 /* The CUDA stream (cudaStream_t) all of the handle's work runs on, so a

@@ -1,0 +1,58 @@
+"""Slots of chain sweeps (mfcfd_debug_slots): held while a chunk runs, all
+returned when every call is over, however it ended."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _held():
+    from mfcfd import _lib
+    v = ctypes.c_int32(-1)
+    assert _lib.lib().mfcfd_debug_slots(0, ctypes.byref(v)) == 0
+    return v.value
+
+
+def _solvers(cloud, count, **kw):
+    from mfcfd.solver import Solver
+    ss = [Solver(cloud, 0.5, 1.0, **kw) for _ in range(count)]
+    for s in ss:
+        s.initial_conditions()
+    return ss
+
+
+def test_run_between_launch_and_complete_keeps_the_count(mfcfd_lib, small_cloud):
+    from mfcfd import batch
+    ss = _solvers(small_cloud, 2)
+    budget = ss[0].info()["chain_slots"]
+    ss[0].launch(1, 3)
+    assert _held() == budget
+    ss[0].q_lskum(2, t0=4)                 # its own slots; the launch keeps its
+    assert _held() == budget
+    batch.run_batch(ss, 2)
+    assert _held() == budget
+    ss[0].complete()
+    assert _held() == 0
+    ss[1].launch(3, 2)                     # never completed
+    assert _held() == budget
+    for s in ss:
+        s.close()
+    assert _held() == 0
+
+
+def test_failed_runs_return_their_slots(mfcfd_lib, small_cloud):
+    from mfcfd import batch
+    from mfcfd._lib import MfcfdError
+    ss = _solvers(small_cloud, 2)
+    prim = ss[0].get(mfcfd_lib.FIELD_PRIM)
+    prim[7, 4] = np.nan                    # a residual that is not finite
+    for run in (lambda: ss[0].q_lskum(2), lambda: batch.run_batch(ss, 2), lambda: batch.run_group(ss, 2)):
+        for s in ss:
+            s.initial_conditions(prim)
+        with pytest.raises(MfcfdError):
+            run()
+        assert _held() == 0
+    for s in ss:
+        s.close()
