@@ -37,8 +37,8 @@ struct ChunkSlots {
         return *this;
     }
     ~ChunkSlots() { end(); }
-    void end() {
-        if (lease) cudaStreamSynchronize(stream);
+    void end(bool idle = false) {
+        if (lease && !idle) cudaStreamSynchronize(stream);
         lease = SlotPool::Lease();
     }
 };
@@ -264,15 +264,30 @@ int budget_slots(const mfcfd_handle *h) {
                ? chain_budget_slots(h->ch_budget, h->ch_wpb, h->d.precision, h->P.chain_spread)
                : 0;
 }
-// Slots for one handle's next chunk (none for the other schedules), its shape
-// set; false if it would have to wait.
-bool take_slots(mfcfd_handle *h, int want, bool wait, SlotPool::Lease *l) {
-    if (h->d.sweep_mode != MFCFD_SWEEP_CHAINS) return true;
+// Slots for the next chunk on stream s; `wait` as in SlotPool::take.
+int take_slots(mfcfd_handle *h, const SlotAsk &a, bool wait, cudaStream_t s, SlotPool::Lease *l) {
+    cudaError_t e = cudaSuccess;
+    *l = g_slots[h->P.device & 255].take(chain_slot_capacity(h->P.device), a, wait, [&](void *end) {
+        e = cudaStreamWaitEvent(s, (cudaEvent_t)end, 0);
+        return e == cudaSuccess;
+    });
+    CK(e);
+    return *l ? MFCFD_OK : MFCFD_ERR_BUSY;
+}
+// ... of one handle (none for the other schedules), its shape set; the chunk's
+// end is recorded in batch_ev.
+int take_slots(mfcfd_handle *h, int want, bool wait, SlotPool::Lease *l) {
+    if (!h->batch_ev) CK(cudaEventCreateWithFlags(&h->batch_ev, cudaEventDisableTiming));
+    if (h->d.sweep_mode != MFCFD_SWEEP_CHAINS) return MFCFD_OK;
     const SlotAsk a{&h->d.ch_chains, 1, h->d.precision, h->P.chain_spread, budget_slots(h), want};
-    *l = g_slots[h->P.device & 255].take(chain_slot_capacity(h->P.device), a, wait);
-    if (!*l) return false;
+    if (int rc = take_slots(h, a, wait, h->stream, l)) return rc;
     h->d.ch_shape = l->shape();
-    return true;
+    return MFCFD_OK;
+}
+int chunk_launched(mfcfd_handle *h, SlotPool::Lease *l) {
+    CK(cudaEventRecord(h->batch_ev, h->stream));
+    l->launched(h->batch_ev);
+    return MFCFD_OK;
 }
 
 // Launch the iterations of one chunk (slots 0 .. chunk-1).  With graphs, the
@@ -442,12 +457,14 @@ int run_iterations(mfcfd_handle *h, int32_t t0, int32_t iters, double *res_hist)
     int status = MFCFD_OK;
     for (int32_t done = 0; done < iters;) {
         ChunkSlots slots{SlotPool::Lease(), h->stream};
-        take_slots(h, 1 << 20, true, &slots.lease);
+        if (int rc = take_slots(h, SLOTS_EVEN, true, &slots.lease)) return rc;
         int chunk = std::min<int32_t>(iters - done, h->res_cap);
         if (slots.lease.lent()) chunk = std::min(chunk, EXCESS_CHUNK);
         int rc = launch_chunk(h, chunk, false);
+        if (!rc) rc = chunk_launched(h, &slots.lease);
         if (!rc) rc = finish_chunk(h, t0 + done, chunk, res_hist ? res_hist + 2 * (size_t)done : nullptr, &status);
         if (rc) return rc;
+        slots.end(true);
         done += chunk;
     }
     return status;
@@ -1024,11 +1041,10 @@ extern "C++" int mfcfd::launch_within(mfcfd_handle *h, int32_t t0, int32_t iters
         if (h->pending_chunk) return fail(h, MFCFD_ERR_ARG, "a launch is already pending on this handle");
         if (iters > h->res_cap) return fail(h, MFCFD_ERR_ARG, "at most 1024 iterations per launch");
         CK(cudaSetDevice(h->P.device));
-        if (!h->batch_ev) CK(cudaEventCreateWithFlags(&h->batch_ev, cudaEventDisableTiming));
         ChunkSlots taken{SlotPool::Lease(), h->stream};
-        if (!take_slots(h, slots, wait, &taken.lease)) return MFCFD_ERR_BUSY;
+        if (int rc = take_slots(h, slots, wait, &taken.lease)) return rc;
         if (int rc = launch_chunk(h, iters, true)) return rc;
-        CK(cudaEventRecord(h->batch_ev, h->stream));
+        if (int rc = chunk_launched(h, &taken.lease)) return rc;
         if (held) *held = taken.lease.slots();
         h->pending_slots = std::move(taken);
         h->pending_chunk = iters;
@@ -1396,8 +1412,6 @@ int mfcfd_run_batch(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
         for (int32_t i = 0; i < count; ++i) {
             slots[i].stream = hs[i]->stream;
             if (iters > 0) ready.push_back(i);
-            if (!hs[i]->batch_ev && cudaEventCreateWithFlags(&hs[i]->batch_ev, cudaEventDisableTiming) != cudaSuccess)
-                return cuda_fail(hs[i], cudaGetLastError(), "cudaEventCreateWithFlags");
         }
         // each handle's share of the device, by its budget
         long budgets = 0;
@@ -1409,12 +1423,12 @@ int mfcfd_run_batch(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
                 mfcfd_handle *h = hs[i];
                 if (!running.empty() && used + budget_slots(h) > capacity) break;
                 const int share = (int)std::min<long>(capacity, (long)capacity * budget_slots(h) / std::max(budgets, 1l));
-                if (!take_slots(h, share, running.empty(), &slots[i].lease)) break;
+                int rc = take_slots(h, share, running.empty(), &slots[i].lease);
+                if (rc == MFCFD_ERR_BUSY) break;
                 ready.pop_front();
                 const int chunk = std::min<int32_t>(iters - done[i], std::max(h->res_cap, 1));
-                int rc = launch_chunk(h, chunk, true);
-                const cudaError_t e = rc ? cudaSuccess : cudaEventRecord(h->batch_ev, h->stream);
-                if (e != cudaSuccess) rc = cuda_fail(h, e, "cudaEventRecord");
+                if (!rc) rc = launch_chunk(h, chunk, true);
+                if (!rc) rc = chunk_launched(h, &slots[i].lease);
                 if (rc) return rc;
                 running.push_back(i);
                 chunk_of[i] = chunk;
@@ -1453,7 +1467,7 @@ namespace {
 struct GroupRun {
     ChainShape shape{};
     cudaStream_t s = nullptr;
-    cudaEvent_t start = nullptr, bwd = nullptr;
+    cudaEvent_t start = nullptr, bwd = nullptr, end = nullptr;
     struct Graph {
         int chunk;
         std::vector<int> cur;
@@ -1466,6 +1480,7 @@ struct GroupRun {
         for (auto &g : graphs) cudaGraphExecDestroy(g.exec);
         if (start) cudaEventDestroy(start);
         if (bwd) cudaEventDestroy(bwd);
+        if (end) cudaEventDestroy(end);
         if (s) cudaStreamDestroy(s);
     }
 };
@@ -1565,6 +1580,7 @@ int mfcfd_run_group(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
         CK(cudaStreamCreateWithPriority(&gr.s, cudaStreamNonBlocking, hi));
         CK(cudaEventCreateWithFlags(&gr.start, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&gr.bwd, cudaEventDisableTiming));
+        CK(cudaEventCreateWithFlags(&gr.end, cudaEventDisableTiming));
         int res_cap = 1 << 30;
         bool graphs = true;
         for (int32_t i = 0; i < count; ++i) {
@@ -1572,9 +1588,10 @@ int mfcfd_run_group(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
             graphs = graphs && hs[i]->P.graphs >= 1 && !hs[i]->graphs_off;
         }
         int first_err = MFCFD_OK;
-        const SlotAsk ask{chains.data(), count, d0.precision, h0->P.chain_spread, slots, 1 << 20};
+        const SlotAsk ask{chains.data(), count, d0.precision, h0->P.chain_spread, slots, SLOTS_EVEN};
         for (int32_t done = 0; done < iters;) {
-            const ChunkSlots held(g_slots[dev & 255].take(chain_slot_capacity(dev), ask, true), gr.s);
+            ChunkSlots held{SlotPool::Lease(), gr.s};
+            if (int rc = take_slots(h0, ask, true, gr.s, &held.lease)) return rc;
             gr.shape = held.lease.shape();
             G->block_start[0] = 0;
             for (int32_t i = 0; i < count; ++i)
@@ -1615,6 +1632,8 @@ int mfcfd_run_group(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
             } else {
                 CK(launch_group_chunk(hs, count, chunk, gr, *G));
             }
+            CK(cudaEventRecord(gr.end, gr.s));
+            held.lease.launched(gr.end);
             CK(cudaStreamSynchronize(gr.s));
             for (int32_t i = 0; i < count; ++i) {
                 int st = MFCFD_OK;

@@ -12,6 +12,7 @@
 #include <condition_variable>
 #include <mutex>
 #include <utility>
+#include <vector>
 
 #include "../../include/mfcfd.h"
 
@@ -57,19 +58,27 @@ inline ChainShape chain_fit(const int *chains, int count, int precision, int spr
 }
 
 // A run's claim: its handles' chain counts, the slots of their budgets, and the
-// slots it would use if they were free.
+// slots it would use if they were free (SLOTS_EVEN: an even share with the runs
+// that hold slots).
 struct SlotAsk {
     const int *chains;
     int count, precision, spread, budget, want;
 };
+constexpr int SLOTS_EVEN = -1;
 
 // Slots of a device's chain sweeps in use (chain_slot_capacity), over every
-// handle and thread of the process.  A run holds at least its handles'
-// budgets (mfcfd_info.chain_slots), whose sum over concurrent runs is the
-// callers' to bound; a run of mfcfd_run, mfcfd_run_batch, mfcfd_run_group or
-// the request server may hold more while nobody needs it, for one chunk of
-// iterations at a time, and whoever does not find room for its budget beside
-// such a run waits for that chunk.
+// handle and thread of the process.  A run takes slots for one chunk of
+// iterations at a time: its handles' budgets (mfcfd_info.chain_slots) at once,
+// and more while they are free.  Where its budget does not fit beside the
+// chunks that hold slots, its own chunk waits on the device for some of them
+// to end (those that hold more than their budgets first, the oldest first): a
+// host thread waits for another's launch calls at most, never for its
+// iterations.  What a run holds counts from the moment it asks, so the others'
+// next chunks leave it room.
+//
+// The sweeps on the device at any time fit it together: of those running, the
+// one that asked last had, when it asked, room beside all others that it did
+// not wait for.
 class SlotPool {
 public:
     // Slots taken, given back when the object goes: on every path, so with an
@@ -84,63 +93,109 @@ public:
             return *this;
         }
         ~Lease() {
-            if (pool_) pool_->give(budget_, slots_);
+            if (pool_) pool_->give(id_);
         }
         explicit operator bool() const { return pool_ != nullptr; }
         int slots() const { return slots_; }
-        bool lent() const { return slots_ > budget_; }       // beyond the budget
+        bool lent() const { return lent_; }                  // beyond the budget
         const ChainShape &shape() const { return shape_; }
+        // The chunk is launched; `end` is recorded behind it, and stays
+        // recorded until the slots are given back.
+        void launched(void *end) {
+            if (pool_) pool_->mark(id_, end);
+        }
 
     private:
         friend class SlotPool;
         void swap(Lease &o) noexcept {
             std::swap(pool_, o.pool_);
-            std::swap(budget_, o.budget_);
+            std::swap(id_, o.id_);
             std::swap(slots_, o.slots_);
+            std::swap(lent_, o.lent_);
             std::swap(shape_, o.shape_);
         }
         SlotPool *pool_ = nullptr;
-        int budget_ = 0, slots_ = 0;
+        long id_ = 0;
+        int slots_ = 0;
+        bool lent_ = false;
         ChainShape shape_{};
     };
 
-    // The largest teams within max(budget, min(want, what is free)); empty, with
-    // `wait` false, instead of waiting (for a caller that itself holds more
-    // than its budgets).
-    Lease take(int capacity, const SlotAsk &a, bool wait) {
-        std::unique_lock<std::mutex> lock(mu_);
-        auto room = [&] { return used_ + a.budget <= capacity || excess_ == 0; };
+    // Slots with the largest teams within max(budget, min(want, what is free)).
+    // after(end): has the chunk about to be launched wait for another's; false
+    // if that fails.  Empty if it failed or, with `wait` false, instead of any
+    // such wait (for a caller with chunks of its own to attend to).
+    template <typename After>
+    Lease take(int capacity, const SlotAsk &a, bool wait, After after) {
         Lease l;
-        if (!wait && !room()) return l;
-        freed_.wait(lock, room);
-        l.shape_ = chain_fit(a.chains, a.count, a.precision, a.spread, std::max(a.budget, std::min(a.want, capacity - used_)));
+        std::unique_lock<std::mutex> lock(mu_);
+        int used = 0;
+        for (const Held &h : held_) used += h.slots;
+        const int want = a.want == SLOTS_EVEN ? capacity / ((int)held_.size() + 1) : a.want;
+        l.shape_ = chain_fit(a.chains, a.count, a.precision, a.spread, std::max(a.budget, std::min(want, capacity - used)));
         for (int i = 0; i < a.count; ++i) l.slots_ += chain_slots(a.chains[i], l.shape_, a.precision);
         l.slots_ = std::max(l.slots_, a.budget);
-        l.budget_ = a.budget;
+        l.lent_ = l.slots_ > a.budget;
+        std::vector<long> ids;
+        for (int lent = 1; lent >= 0; --lent)
+            for (const Held &h : held_)
+                if (h.lent == (lent != 0) && used + l.slots_ > capacity) {
+                    used -= h.slots;
+                    ids.push_back(h.id);
+                }
+        if (!ids.empty() && !wait) return Lease();
+        held_.push_back({next_, l.slots_, l.lent_, false, nullptr});
+        l.id_ = next_++;
         l.pool_ = this;
-        used_ += l.slots_;
-        excess_ += l.slots_ - l.budget_;
+        // each was taken before this one, so no two wait for each other
+        for (const long id : ids) {
+            const Held *h;
+            launched_.wait(lock, [&] { return !(h = find(id)) || h->launched; });
+            if (h && !after(h->end)) return Lease();         // and l goes back
+        }
         return l;
     }
 
     // Slots held now.
     int held() {
         std::lock_guard<std::mutex> lock(mu_);
-        return used_;
+        int used = 0;
+        for (const Held &h : held_) used += h.slots;
+        return used;
     }
 
 private:
-    void give(int budget, int slots) {
+    struct Held {
+        long id;
+        int slots;
+        bool lent, launched;
+        void *end;
+    };
+    Held *find(long id) {
+        for (Held &h : held_)
+            if (h.id == id) return &h;
+        return nullptr;
+    }
+    void mark(long id, void *end) {
         {
             std::lock_guard<std::mutex> lock(mu_);
-            used_ -= slots;
-            excess_ -= slots - budget;
+            Held *h = find(id);
+            h->launched = true;
+            h->end = end;
         }
-        freed_.notify_all();
+        launched_.notify_all();
+    }
+    void give(long id) {
+        {
+            std::lock_guard<std::mutex> lock(mu_);
+            held_.erase(held_.begin() + (find(id) - held_.data()));
+        }
+        launched_.notify_all();
     }
     std::mutex mu_;
-    std::condition_variable freed_;
-    int used_ = 0, excess_ = 0;
+    std::condition_variable launched_;
+    std::vector<Held> held_;                                 // by age
+    long next_ = 0;
 };
 
 }  // namespace mfcfd

@@ -253,8 +253,10 @@ int mfcfd_fpi_step(mfcfd_handle *h, int32_t t, double *res_new, double *residue)
  * then reports whether they have finished (*done), or waits for them with
  * wait != 0, and on completion fills res_hist (2*iters, may be NULL) as
  * mfcfd_run does.  One launch may be pending per handle.  Chain sweeps of
- * handles running at once must fit the device together: the launches'
- * mfcfd_info.chain_slots may add up to chain_slot_capacity at most.
+ * handles running at once fit the device together: launches whose
+ * mfcfd_info.chain_slots add up to chain_slot_capacity at most run side by
+ * side, others (and any beside a run that holds more than its chain_slots)
+ * wait on the device, not in the call, for chunks launched before to end.
  */
 int mfcfd_launch(mfcfd_handle *h, int32_t t0, int32_t iters);
 int mfcfd_complete(mfcfd_handle *h, int32_t wait, double *res_hist, int32_t *done);
@@ -290,10 +292,9 @@ int mfcfd_run_batch(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
  * mfcfd_run gives it.  A group waits each iteration for its slowest sweep,
  * so handles of similar size group best.  res_hist and status as in
  * mfcfd_run_batch.  Calls on disjoint handles may run from separate host
- * threads at once; as with mfcfd_launch, the chain sweeps running at the
- * same time must then fit the device together (their chain_slots add up to
- * chain_slot_capacity at most), or their bounded waits may run out
- * (MFCFD_ERR_TIMEOUT).
+ * threads at once; as with mfcfd_launch, those run side by side whose chain
+ * sweeps fit the device together (their chain_slots add up to
+ * chain_slot_capacity at most), the others' iterations wait on the device.
  */
 #define MFCFD_GROUP_MAX_CLOUDS 32
 int mfcfd_run_group(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, int32_t iters,

@@ -56,3 +56,36 @@ def test_failed_runs_return_their_slots(mfcfd_lib, small_cloud):
         assert _held() == 0
     for s in ss:
         s.close()
+
+
+def test_runs_from_two_threads_give_the_bits_of_runs_alone(mfcfd_lib):
+    import threading
+    from mfcfd import batch, cloud
+    from mfcfd.solver import Solver
+    clouds = [cloud.shell_cloud(26, 361, seed=s, knn_device=0) for s in (1, 2, 3)]
+    ref = [Solver(c, 0.5, 1.0) for c in clouds]
+    ss = [Solver(c, 0.5, 1.0) for c in clouds]
+    for s in ref + ss:
+        s.initial_conditions()
+    want = [s.q_lskum(70) for s in ref]
+    got = [None] * 3
+
+    def run():
+        got[0] = ss[0].q_lskum(70)
+
+    def group():
+        got[1] = batch.run_group(ss[1:2], 70)[0]
+
+    threads = [threading.Thread(target=run), threading.Thread(target=group)]
+    for t in threads:
+        t.start()
+    ss[2].launch(1, 70)
+    got[2] = ss[2].complete()
+    for t in threads:
+        t.join()
+    for s, r, g, w in zip(ss, ref, got, want):
+        assert np.array_equal(g, w)
+        assert np.array_equal(s.get(mfcfd_lib.FIELD_PRIM), r.get(mfcfd_lib.FIELD_PRIM))
+    assert _held() == 0
+    for s in ss + ref:
+        s.close()
