@@ -1183,8 +1183,9 @@ namespace mfcfd {
 // FP64 build (168 registers, 100 bytes spilled), which a cloud takes whose teams
 // need more than two blocks per SM (1.1M points, 376 teams of four: 37.0 ms
 // per iteration against 41.5 as teams of two on more chains).  The sweeps at
-// once take at most 6 * (SMs - CH_FREE_SMS) slots; the other SMs' room is for
-// the kernels of other handles between their sweeps.
+// once take at most 6 * (SMs - CH_FREE_SMS) slots, or 4 of each of these SMs
+// where their blocks differ in size (SlotPool); the other SMs' room is for the
+// kernels of other handles between their sweeps.
 constexpr int CH_FREE_SMS = 16;
 
 template <typename R, bool FOLD, bool DENSE>

@@ -31,30 +31,13 @@ inline bool operator==(const ChainShape &a, const ChainShape &b) {
     return a.team == b.team && a.dense == b.dense && a.spread == b.spread;
 }
 
-// Blocks and slots of a chain sweep.
+// Blocks of a chain sweep, the slots of one, and of all.
 inline int chain_blocks(int chains, const ChainShape &c) { return (chains * c.team + CH_WPB - 1) / CH_WPB; }
-inline int chain_slots(int chains, const ChainShape &c, int precision) {
-    const int each = c.spread ? 6 : (precision != MFCFD_PRECISION_FP64 || c.dense ? 2 : 3);
-    return chain_blocks(chains, c) * each;
+inline int chain_block_slots(const ChainShape &c, int precision) {
+    return c.spread ? 6 : (precision != MFCFD_PRECISION_FP64 || c.dense ? 2 : 3);
 }
-
-// The largest teams with which the sweeps of these chain counts fit `slots`
-// together; teams of one (which fit their budgets) if none does.
-inline ChainShape chain_fit(const int *chains, int count, int precision, int spread, int slots) {
-    ChainShape c{};
-    c.spread = spread;
-    c.team = spread ? 1 : CH_WPB;
-    for (;; c.team /= 2) {
-        for (c.dense = 0; c.dense < 2; ++c.dense) {
-            int sum = 0;
-            for (int i = 0; i < count; ++i) sum += chain_slots(chains[i], c, precision);
-            if (sum <= slots) return c;
-            if (precision != MFCFD_PRECISION_FP64) break;
-        }
-        if (c.team == 1) break;
-    }
-    c.dense = 0;
-    return c;
+inline int chain_slots(int chains, const ChainShape &c, int precision) {
+    return chain_blocks(chains, c) * chain_block_slots(c, precision);
 }
 
 // A run's claim: its handles' chain counts, the slots of their budgets, and the
@@ -79,6 +62,13 @@ constexpr int SLOTS_EVEN = -1;
 // The sweeps on the device at any time fit it together: of those running, the
 // one that asked last had, when it asked, room beside all others that it did
 // not wait for.
+//
+// Blocks of one size fill SMs without a remainder: they may take all slots.
+// Where sizes differ, an SM that holds four slots may have no room for one
+// more block (two blocks of two slots beside one of three, or beside a spread
+// one, which needs half of the SM's shared memory): together they may take
+// four slots of each SM.  A handle in FP64 has a build of either size, so it
+// usually joins the size that is running.
 class SlotPool {
 public:
     // Slots taken, given back when the object goes: on every path, so with an
@@ -121,7 +111,8 @@ public:
         ChainShape shape_{};
     };
 
-    // Slots with the largest teams within max(budget, min(want, what is free)).
+    // Slots with the largest teams within max(budget, want) that have room now,
+    // or else with the shape within the budget that waits for the fewest chunks.
     // after(end): has the chunk about to be launched wait for another's; false
     // if that fails.  Empty if it failed or, with `wait` false, instead of any
     // such wait (for a caller with chunks of its own to attend to).
@@ -129,22 +120,36 @@ public:
     Lease take(int capacity, const SlotAsk &a, bool wait, After after) {
         Lease l;
         std::unique_lock<std::mutex> lock(mu_);
-        int used = 0;
-        for (const Held &h : held_) used += h.slots;
         const int want = a.want == SLOTS_EVEN ? capacity / ((int)held_.size() + 1) : a.want;
-        l.shape_ = chain_fit(a.chains, a.count, a.precision, a.spread, std::max(a.budget, std::min(want, capacity - used)));
-        for (int i = 0; i < a.count; ++i) l.slots_ += chain_slots(a.chains[i], l.shape_, a.precision);
-        l.slots_ = std::max(l.slots_, a.budget);
-        l.lent_ = l.slots_ > a.budget;
-        std::vector<long> ids;
+        // the order in which chunks are waited for
+        std::vector<const Held *> order;
         for (int lent = 1; lent >= 0; --lent)
             for (const Held &h : held_)
-                if (h.lent == (lent != 0) && used + l.slots_ > capacity) {
-                    used -= h.slots;
-                    ids.push_back(h.id);
-                }
-        if (!ids.empty() && !wait) return Lease();
-        held_.push_back({next_, l.slots_, l.lent_, false, nullptr});
+                if (h.lent == (lent != 0)) order.push_back(&h);
+        size_t waits = order.size() + 1;
+        int block = 0;
+        for (ChainShape c{a.spread ? 1 : CH_WPB, 0, a.spread};;) {
+            int slots = 0;
+            for (int i = 0; i < a.count; ++i) slots += chain_slots(a.chains[i], c, a.precision);
+            slots = std::max(slots, a.budget);
+            const bool last = c.team == 1 && (c.dense || c.spread || a.precision != MFCFD_PRECISION_FP64);
+            const size_t w = waits_for(order, capacity, slots, chain_block_slots(c, a.precision));
+            const bool own = slots <= a.budget || (c.team == 1 && !c.dense);   // (teams of one fit their budget)
+            if (w < waits && (own || (w == 0 && slots <= want))) {
+                waits = w;
+                block = chain_block_slots(c, a.precision);
+                l.shape_ = c;
+                l.slots_ = slots;
+            }
+            if (waits == 0 || last) break;
+            if (a.precision != MFCFD_PRECISION_FP64 || c.dense) c.team /= 2, c.dense = 0;
+            else c.dense = 1;
+        }
+        if (waits > 0 && !wait) return Lease();
+        l.lent_ = l.slots_ > a.budget;
+        std::vector<long> ids;
+        for (size_t k = 0; k < waits; ++k) ids.push_back(order[k]->id);
+        held_.push_back({next_, l.slots_, block, l.lent_, false, nullptr});
         l.id_ = next_++;
         l.pool_ = this;
         // each was taken before this one, so no two wait for each other
@@ -167,10 +172,24 @@ public:
 private:
     struct Held {
         long id;
-        int slots;
+        int slots, block;                                    // of them, slots of a block
         bool lent, launched;
         void *end;
     };
+    // How many of the chunks in `order` have to end before `slots` in blocks of
+    // `block` have room beside the others.
+    static size_t waits_for(const std::vector<const Held *> &order, int capacity, int slots, int block) {
+        for (size_t w = 0; w < order.size(); ++w) {
+            int sum = slots;
+            bool same = true;
+            for (size_t k = w; k < order.size(); ++k) {
+                sum += order[k]->slots;
+                same = same && order[k]->block == block;
+            }
+            if (sum <= (same ? capacity : capacity / 6 * 4)) return w;
+        }
+        return order.size();
+    }
     Held *find(long id) {
         for (Held &h : held_)
             if (h.id == id) return &h;

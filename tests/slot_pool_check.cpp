@@ -94,18 +94,18 @@ struct Chunk {
 // room.
 int launch_beside_a_run() {
     SlotPool p;
-    const int chains = 396;
+    const int chains = 264;
     int end = 0;
     std::vector<void *> waited;
     auto after = [&](void *e) { return waited.push_back(e), true; };
-    SlotPool::Lease run = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 180, SLOTS_EVEN), true, no_wait);
+    SlotPool::Lease run = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 198, SLOTS_EVEN), true, no_wait);
     REQUIRE(run.lent() && run.slots() == CAP);
     run.launched(&end);
     REQUIRE(!p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 300, 0), false, after) && waited.empty());
     SlotPool::Lease launch = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 300, 0), true, after);
     REQUIRE(launch && !launch.lent() && launch.slots() == 300 && waited == std::vector<void *>{&end});
     run = SlotPool::Lease();
-    run = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 180, SLOTS_EVEN), true, no_wait);
+    run = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 198, SLOTS_EVEN), true, no_wait);
     REQUIRE(run && run.slots() <= CAP - 300);
     // a chunk whose wait cannot be queued does not run, and holds nothing
     const int before = p.held();
@@ -128,7 +128,7 @@ int threads_share() {
         std::vector<std::thread> pool;
         for (int k = 0; k < threads; ++k)
             pool.emplace_back([&, k] {
-                const int chains = 396, budget = 180;      // 4 of 5 fit
+                const int chains = 240, budget = 180;      // 4 of 5 fit
                 while (!stop) {
                     all[k].emplace_back(new Chunk());
                     Chunk *c = all[k].back().get();
@@ -158,6 +158,102 @@ int threads_share() {
     return 0;
 }
 
+// Shapes of a block, and an SM's room for them: registers (168 a thread where
+// three blocks share an SM, else 256) and kilobytes of shared memory.
+struct Block {
+    int slots, regs, smem;
+};
+constexpr Block BLOCKS[] = {{2, 168 * 128, 76}, {3, 256 * 128, 76}, {6, 256 * 128, 117}, {6, 168 * 128, 117}};
+bool fits_sm(const int n[4]) {
+    int regs = 0, smem = 0;
+    for (int b = 0; b < 4; ++b) regs += n[b] * BLOCKS[b].regs, smem += n[b] * BLOCKS[b].smem;
+    return regs <= 65536 && smem <= 228;
+}
+
+// The fewest slots that blocks of the kinds in `have` can hold on an SM without
+// room for another block of kind b.
+int fewest_without_room(const bool have[4], int b) {
+    int least = 1 << 20;
+    int n[4];
+    for (n[0] = 0; n[0] <= (have[0] ? 3 : 0); ++n[0])
+        for (n[1] = 0; n[1] <= (have[1] ? 3 : 0); ++n[1])
+            for (n[2] = 0; n[2] <= (have[2] ? 2 : 0); ++n[2])
+                for (n[3] = 0; n[3] <= (have[3] ? 2 : 0); ++n[3]) {
+                    if (!fits_sm(n)) continue;
+                    ++n[b];
+                    const bool room = fits_sm(n);
+                    --n[b];
+                    if (room) continue;
+                    int slots = 0;
+                    for (int k = 0; k < 4; ++k) slots += n[k] * BLOCKS[k].slots;
+                    least = std::min(least, slots);
+                }
+    return least;
+}
+
+// Blocks of different sizes leave parts of SMs that no other block fits, so
+// counting slots is not enough: the sweeps that the pool lets run at once are
+// all resident together, in whatever order their blocks were placed.
+int block_sizes() {
+    unsigned seed = 1;
+    auto rnd = [&](int n) { return (int)((seed = seed * 1664525u + 1013904223u) >> 8) % n; };
+    int mixed_sizes = 0;
+    for (int round = 0; round < 20000; ++round) {
+        SlotPool p;
+        std::vector<SlotPool::Lease> running;
+        std::vector<int> kinds;
+        const int share = rnd(3) ? 1 + rnd(CAP) : SLOTS_EVEN;
+        for (int k = 0; k < 12; ++k) {
+            const int precision = rnd(2) ? MFCFD_PRECISION_FP64 : MFCFD_PRECISION_MIXED, spread = rnd(8) == 0;
+            const int chains = 1 + rnd(spread ? 100 : 264);
+            const int budget = (chains + 3) / 4 * (spread ? 6 : precision == MFCFD_PRECISION_FP64 ? 3 : 2);
+            const SlotAsk a{&chains, 1, precision, spread, budget, share};
+            SlotPool::Lease l = p.take(CAP, a, false, no_wait);
+            if (!l) continue;
+            const ChainShape c = l.shape();
+            kinds.push_back(spread ? (precision == MFCFD_PRECISION_FP64 ? 2 : 3)
+                                   : (precision == MFCFD_PRECISION_FP64 && !c.dense ? 1 : 0));
+            REQUIRE(l.slots() >= chain_slots(chains, c, precision) && (l.lent() || l.slots() == budget));
+            running.push_back(std::move(l));
+        }
+        bool have[4] = {false, false, false, false};
+        for (const int k : kinds) have[k] = true;
+        mixed_sizes += have[0] + have[1] + (have[2] || have[3]) > 1;
+        for (int b = 0; b < 4; ++b)
+            if (have[b] && !(p.held() - BLOCKS[b].slots < 148 * fewest_without_room(have, b))) {
+                std::printf("%d slots in use, a block of kind %d has no room where every SM holds %d\n", p.held(), b,
+                            fewest_without_room(have, b));
+                return 1;
+            }
+    }
+    REQUIRE(mixed_sizes > 1000);
+    return 0;
+}
+
+// What the pool gives sweeps that differ in block size: the FP64 build of the
+// size that is running, and the device to one size after the other where
+// neither fits beside the other.
+int block_size_choice() {
+    SlotPool p;
+    const int few = 88, many = 264;
+    int end = 0;
+    std::vector<void *> waited;
+    auto after = [&](void *e) { return waited.push_back(e), true; };
+    SlotPool::Lease mixed = p.take(CAP, ask(many, MFCFD_PRECISION_MIXED, 132, 528), true, no_wait);
+    REQUIRE(mixed.slots() == 528 && mixed.shape().team == 4);
+    mixed.launched(&end);
+    SlotPool::Lease f64 = p.take(CAP, ask(few, MFCFD_PRECISION_FP64, 66, 264), true, no_wait);
+    REQUIRE(f64 && f64.shape().dense == 1 && f64.shape().team == 4 && f64.slots() == 176);
+    f64 = SlotPool::Lease();
+    mixed = SlotPool::Lease();
+    f64 = p.take(CAP, ask(many, MFCFD_PRECISION_FP64, 198, CAP), true, no_wait);
+    REQUIRE(f64.shape().dense == 0 && f64.slots() == CAP);
+    f64.launched(&end);
+    mixed = p.take(CAP, ask(many, MFCFD_PRECISION_MIXED, 132, 0), true, after);
+    REQUIRE(mixed && !mixed.lent() && waited == std::vector<void *>{&end});
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -166,6 +262,8 @@ int main(int argc, char **argv) {
         if (!std::strcmp(argv[i], "leases")) bad = leases();
         else if (!std::strcmp(argv[i], "launch_beside_a_run")) bad = launch_beside_a_run();
         else if (!std::strcmp(argv[i], "threads_share")) bad = threads_share();
+        else if (!std::strcmp(argv[i], "block_sizes")) bad = block_sizes();
+        else if (!std::strcmp(argv[i], "block_size_choice")) bad = block_size_choice();
         else bad = 1;
     }
     if (!bad) std::printf("ok\n");

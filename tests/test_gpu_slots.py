@@ -89,3 +89,22 @@ def test_runs_from_two_threads_give_the_bits_of_runs_alone(mfcfd_lib):
     assert _held() == 0
     for s in ss + ref:
         s.close()
+
+
+def test_batch_of_different_block_sizes_gives_the_bits_of_runs_alone(mfcfd_lib):
+    from mfcfd import batch, cloud
+    from mfcfd.solver import Solver
+    c = cloud.shell_cloud(26, 361, seed=4, knn_device=0)
+    kinds = [{}, {"precision": 1}, {"precision": 2}, {"chain_spread": 1}, {"chain_warps": 40}] * 3
+    ref = [Solver(c, 0.5, 1.0, **k) for k in kinds[:5]]
+    ss = [Solver(c, 0.5, 1.0, **k) for k in kinds]
+    for s in ref + ss:
+        s.initial_conditions()
+    want = [s.q_lskum(6) for s in ref]
+    got = batch.run_batch(ss, 6)
+    for i, s in enumerate(ss):
+        assert np.array_equal(got[i], want[i % 5])
+        assert np.array_equal(s.get(mfcfd_lib.FIELD_PRIM), ref[i % 5].get(mfcfd_lib.FIELD_PRIM))
+    assert _held() == 0
+    for s in ss + ref:
+        s.close()

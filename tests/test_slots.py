@@ -20,7 +20,7 @@ def checker(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("check", ["leases", "launch_beside_a_run", "threads_share"])
+@pytest.mark.parametrize("check", ["leases", "launch_beside_a_run", "threads_share", "block_sizes", "block_size_choice"])
 def test_slot_pool(checker, check):
     out = subprocess.run([checker, check], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0 and out.stdout == "ok\n", out.stdout + out.stderr
