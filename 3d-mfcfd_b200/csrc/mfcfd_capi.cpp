@@ -257,7 +257,6 @@ int launch_one(mfcfd_handle *h, int j) {
 }
 
 SlotPool g_slots[256];                     // per device
-constexpr int EXCESS_CHUNK = 64;           // iterations a run beyond its budget lasts at most
 
 int budget_slots(const mfcfd_handle *h) {
     return h->d.sweep_mode == MFCFD_SWEEP_CHAINS
@@ -458,8 +457,7 @@ int run_iterations(mfcfd_handle *h, int32_t t0, int32_t iters, double *res_hist)
     for (int32_t done = 0; done < iters;) {
         ChunkSlots slots{SlotPool::Lease(), h->stream};
         if (int rc = take_slots(h, SLOTS_EVEN, true, &slots.lease)) return rc;
-        int chunk = std::min<int32_t>(iters - done, h->res_cap);
-        if (slots.lease.lent()) chunk = std::min(chunk, EXCESS_CHUNK);
+        const int chunk = slots.lease.chunk(std::min<int32_t>(iters - done, h->res_cap));
         int rc = launch_chunk(h, chunk, false);
         if (!rc) rc = chunk_launched(h, &slots.lease);
         if (!rc) rc = finish_chunk(h, t0 + done, chunk, res_hist ? res_hist + 2 * (size_t)done : nullptr, &status);
@@ -1033,7 +1031,7 @@ int mfcfd_fpi_step(mfcfd_handle *h, int32_t t, double *res_new, double *residue)
     });
 }
 
-extern "C++" int mfcfd::launch_within(mfcfd_handle *h, int32_t t0, int32_t iters, int slots, bool wait, int *held) {
+extern "C++" int mfcfd::launch_within(mfcfd_handle *h, int32_t t0, int32_t iters, int slots, bool wait, int *held, int *launched) {
     return host_guard(h ? &h->err : nullptr, [&]() -> int {
         if (!h || iters < 1) return MFCFD_ERR_ARG;
         if (!h->stream) return fail(h, MFCFD_ERR_ARG, "handle was not created successfully");
@@ -1043,6 +1041,7 @@ extern "C++" int mfcfd::launch_within(mfcfd_handle *h, int32_t t0, int32_t iters
         CK(cudaSetDevice(h->P.device));
         ChunkSlots taken{SlotPool::Lease(), h->stream};
         if (int rc = take_slots(h, slots, wait, &taken.lease)) return rc;
+        if (launched) *launched = iters = taken.lease.chunk(iters);
         if (int rc = launch_chunk(h, iters, true)) return rc;
         if (int rc = chunk_launched(h, &taken.lease)) return rc;
         if (held) *held = taken.lease.slots();
@@ -1053,7 +1052,7 @@ extern "C++" int mfcfd::launch_within(mfcfd_handle *h, int32_t t0, int32_t iters
     });
 }
 
-int mfcfd_launch(mfcfd_handle *h, int32_t t0, int32_t iters) { return mfcfd::launch_within(h, t0, iters, 0, true, nullptr); }
+int mfcfd_launch(mfcfd_handle *h, int32_t t0, int32_t iters) { return mfcfd::launch_within(h, t0, iters, 0, true, nullptr, nullptr); }
 
 int mfcfd_complete(mfcfd_handle *h, int32_t wait, double *res_hist, int32_t *done) {
     return host_guard(h ? &h->err : nullptr, [&]() -> int {
@@ -1426,7 +1425,7 @@ int mfcfd_run_batch(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
                 int rc = take_slots(h, share, running.empty(), &slots[i].lease);
                 if (rc == MFCFD_ERR_BUSY) break;
                 ready.pop_front();
-                const int chunk = std::min<int32_t>(iters - done[i], std::max(h->res_cap, 1));
+                const int chunk = slots[i].lease.chunk(std::min<int32_t>(iters - done[i], std::max(h->res_cap, 1)));
                 if (!rc) rc = launch_chunk(h, chunk, true);
                 if (!rc) rc = chunk_launched(h, &slots[i].lease);
                 if (rc) return rc;
@@ -1596,7 +1595,7 @@ int mfcfd_run_group(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
             G->block_start[0] = 0;
             for (int32_t i = 0; i < count; ++i)
                 G->block_start[i + 1] = G->block_start[i] + chain_blocks(chains[i], gr.shape);
-            const int chunk = std::min<int32_t>(iters - done, held.lease.lent() ? std::min(res_cap, EXCESS_CHUNK) : res_cap);
+            const int chunk = held.lease.chunk(std::min<int32_t>(iters - done, res_cap));
             for (int32_t i = 0; i < count; ++i) hs[i]->res_valid = false;
             std::vector<int> cur(count), last(count);
             for (int32_t i = 0; i < count; ++i) cur[i] = hs[i]->cur, last[i] = hs[i]->last;

@@ -457,8 +457,9 @@ cudaError_t launch_fold_terms(const DevCloud &d, double *const saved[2], bool fo
 // mfcfd_launch holding up to `slots` slots (its budget if that is more); *held
 // (may be null) receives the slots it holds until mfcfd_complete.  With `wait`
 // false, MFCFD_ERR_BUSY where the chunk would have to wait on the device for
-// chunks that hold slots now.
-int launch_within(mfcfd_handle *h, int32_t t0, int32_t iters, int slots, bool wait, int *held);
+// chunks that hold slots now.  *launched (null: all) receives the iterations
+// launched, LENT_CHUNK at most beyond the budget.
+int launch_within(mfcfd_handle *h, int32_t t0, int32_t iters, int slots, bool wait, int *held, int *launched);
 
 // Allocation-free residual (mfcfd_residual_noalloc); the current device must
 // be the handle's.

@@ -53,7 +53,9 @@ struct Request {
     std::string err;
     bool done = false;
     int slots = 0;                    // SM slots of its chain sweep (mfcfd_info)
-    int held = 0;                     // ... of its running chunk
+    int held = 0;                     // ... of its running part of a chunk
+    int part = 0, part_of = 0;        // its iterations, and those of the chunk done before it
+    int chunk_rc = MFCFD_OK;          // first error of the chunk
     int slot_capacity = 0;            // the device's chain slots (mfcfd_info)
     bool running = false;             // a chunk is launched and not yet completed
     double t_launch = 0.0;            // server clock at its running chunk's launch
@@ -387,7 +389,7 @@ void mfcfd_server::scheduler_loop() {
                 if (r->running || r->retiring) continue;
                 if (running > 0 && used + r->slots > capacity) continue;
                 const int share = std::min(capacity / std::max(active, 1), capacity - used);
-                const int rc = mfcfd::launch_within(r->h, r->t, chunk, share, running == 0, &r->held);
+                const int rc = mfcfd::launch_within(r->h, r->t, chunk - r->part_of, share, running == 0, &r->held, &r->part);
                 if (rc == MFCFD_ERR_BUSY) continue;
                 progress = true;
                 if (rc) {
@@ -406,7 +408,7 @@ void mfcfd_server::scheduler_loop() {
             for (const RequestPtr &r : live) {
                 if (!r->running) continue;
                 int32_t done = 0;
-                const int rc = mfcfd_complete(r->h, 0, hist.data(), &done);
+                int rc = mfcfd_complete(r->h, 0, hist.data(), &done);
                 if (!done && rc == MFCFD_OK) continue;
                 progress = true;
                 account();
@@ -414,15 +416,20 @@ void mfcfd_server::scheduler_loop() {
                 r->running = false;
                 used -= r->held;
                 --running;
+                r->t += r->part;
+                r->res.iters += r->part;
+                r->res.res_new = hist[2 * (size_t)(r->part - 1)];
+                r->res.residue = hist[2 * (size_t)(r->part - 1) + 1];
+                r->part_of += r->part;
+                if (r->chunk_rc == MFCFD_OK) r->chunk_rc = rc;
+                rc = r->chunk_rc;
                 {
                     std::lock_guard<std::mutex> lk(mu);
-                    ++st.rounds;
-                    st.iterations += chunk;
+                    st.rounds += r->part_of == chunk;
+                    st.iterations += r->part;
                 }
-                r->t += chunk;
-                r->res.iters += chunk;
-                r->res.res_new = hist[2 * (size_t)(chunk - 1)];
-                r->res.residue = hist[2 * (size_t)(chunk - 1) + 1];
+                if (r->part_of < chunk) continue;     // decisions at the chunk's end only
+                r->part_of = 0;
                 r->res.converged = rc == MFCFD_OK && r->t - 1 > 2 && r->res.residue <= r->target;
                 if (rc != MFCFD_OK) r->fail = rc;
                 if (rc != MFCFD_OK || r->res.converged || r->res.iters >= r->max_iters) r->retiring = true;

@@ -48,6 +48,9 @@ struct SlotAsk {
     int count, precision, spread, budget, want;
 };
 constexpr int SLOTS_EVEN = -1;
+// Iterations that a chunk beyond its run's budget lasts at most, so that whoever
+// asks next does not wait for it long.
+constexpr int LENT_CHUNK = 64;
 
 // Slots of a device's chain sweeps in use (chain_slot_capacity), over every
 // handle and thread of the process.  A run takes slots for one chunk of
@@ -88,6 +91,8 @@ public:
         explicit operator bool() const { return pool_ != nullptr; }
         int slots() const { return slots_; }
         bool lent() const { return lent_; }                  // beyond the budget
+        // Iterations of the next chunk, of `iters` to run.
+        int chunk(int iters) const { return lent_ ? std::min(iters, LENT_CHUNK) : iters; }
         const ChainShape &shape() const { return shape_; }
         // The chunk is launched; `end` is recorded behind it, and stays
         // recorded until the slots are given back.

@@ -103,6 +103,8 @@ int launch_beside_a_run() {
     run.launched(&end);
     REQUIRE(!p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 300, 0), false, after) && waited.empty());
     SlotPool::Lease launch = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 300, 0), true, after);
+    REQUIRE(run.chunk(1000) == LENT_CHUNK && run.chunk(10) == 10);   // not kept waiting for long
+    REQUIRE(launch.chunk(1000) == 1000);
     REQUIRE(launch && !launch.lent() && launch.slots() == 300 && waited == std::vector<void *>{&end});
     run = SlotPool::Lease();
     run = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 198, SLOTS_EVEN), true, no_wait);

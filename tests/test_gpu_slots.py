@@ -108,3 +108,22 @@ def test_batch_of_different_block_sizes_gives_the_bits_of_runs_alone(mfcfd_lib):
     assert _held() == 0
     for s in ss + ref:
         s.close()
+
+
+def test_chunks_beyond_the_budget_are_parts_of_longer_ones(mfcfd_lib, small_cloud):
+    """A batch of 100 iterations and a server's chunks of 100 run in parts of at
+    most 64 where they hold more slots than their budgets: same bits, and a
+    request ends with a whole chunk."""
+    from mfcfd import batch, serve
+    ref, s = _solvers(small_cloud, 2)
+    want = ref.q_lskum(200)
+    for k in (0, 1):
+        assert np.array_equal(batch.run_batch([s], 100)[0], want[100 * k:100 * k + 100])
+    with serve.Server(chunk=100) as srv:
+        r = srv.wait(srv.submit(small_cloud, 0.5, 1.0, max_iters=150, residue_target=-99.0), timeout=120)
+        st = srv.stats()
+    assert r["status"] == 0 and r["iters"] == 200
+    assert np.array_equal(r["prim"], ref.get(mfcfd_lib.FIELD_PRIM)) and r["res_new"] == want[-1, 0]
+    assert st["rounds"] == 2 and st["iterations"] == 200
+    ref.close()
+    s.close()
