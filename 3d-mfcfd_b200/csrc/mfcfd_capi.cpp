@@ -90,8 +90,8 @@ struct mfcfd_handle {
     int pending_chunk = 0;                 // mfcfd_launch: iterations not yet completed
     ChunkSlots pending_slots;              // ... and their slots
     // chain schedule: the warps it may hold beside other handles' (in blocks
-    // of ch_wpb); DevCloud::ch_shape is the shape of the running chunk
-    int ch_budget = 0, ch_wpb = 0;
+    // of ch_wpb), and the warps asked for; DevCloud::ch_shape is the shape of the running chunk
+    int ch_budget = 0, ch_wpb = 0, ch_want = 0;
     int32_t pending_t0 = 0;
     bool graphs_off = false;               // a capture failed: launch one by one
     // device-resident set-up (mfcfd_params.gpu_setup = 1): the topology was
@@ -389,7 +389,7 @@ int apply_chain_schedule(mfcfd_handle *h, int want, int *warps) {
     int wpb = 0;
     const int budget = chain_budget(h->P.device, want, h->P.chain_spread, &wpb);
     if (budget < 1) return fail(h, MFCFD_ERR_CUDA, "chain sweep kernel cannot be resident");
-    const int w = chain_count(h->P.device, budget, h->T.max_level_width, h->P.chain_spread);
+    const int w = chain_count(h->P.device, budget, want, h->T.max_level_width, h->P.chain_spread);
     if (h->dev_setup) {
         DevCloud &d = h->d;
         for (int dir = 0; dir < 2; ++dir) {
@@ -410,6 +410,7 @@ int apply_chain_schedule(mfcfd_handle *h, int want, int *warps) {
             return fail(h, rc, err.empty() ? h->err : err);
         h->ch_budget = budget;
         h->ch_wpb = wpb;
+        h->ch_want = want;
         drop_graphs(h);
         for (int k = 0; k < 3; ++k) h->chain_terms[k] = terms[k];
         *warps = budget;
@@ -441,6 +442,7 @@ int apply_chain_schedule(mfcfd_handle *h, int want, int *warps) {
     d.ch_chains = w;
     h->ch_budget = budget;
     h->ch_wpb = wpb;
+    h->ch_want = want;
     drop_graphs(h);                        // their launches name the old schedule
     h->chain_terms[0] = S.terms_ring;
     h->chain_terms[1] = S.terms_local;
@@ -645,8 +647,9 @@ int stage_host(mfcfd_handle *h, const double *x, const double *y, const double *
         if (P.chain_warps < 0) return fail(h, MFCFD_ERR_ARG, "chain_warps must not be negative");
         const int want = P.chain_warps > 0 ? P.chain_warps : std::max(1, 2 * h->T.max_level_width);
         if (P.chain_spread < 0 || P.chain_spread > 1) return fail(h, MFCFD_ERR_ARG, "chain_spread must be 0 or 1");
+        h->ch_want = want;
         h->ch_budget = chain_budget(P.device, want, P.chain_spread, &h->ch_wpb);
-        st->chains = chain_count(P.device, h->ch_budget, h->T.max_level_width, P.chain_spread);
+        st->chains = chain_count(P.device, h->ch_budget, want, h->T.max_level_width, P.chain_spread);
         if (h->ch_budget < 1 || !chain_fits(P.device, false))
             return fail(h, MFCFD_ERR_CUDA, "chain sweep kernel cannot be resident");
     }
@@ -879,8 +882,9 @@ int create_on_device(mfcfd_handle *h, const double *x, const double *y, const do
     }
     if (P.sweep_mode == MFCFD_SWEEP_CHAINS) {
         const int want = P.chain_warps > 0 ? P.chain_warps : std::max(1, 2 * T.max_level_width);
+        h->ch_want = want;
         h->ch_budget = chain_budget(P.device, want, P.chain_spread, &h->ch_wpb);
-        const int w = chain_count(P.device, h->ch_budget, T.max_level_width, P.chain_spread);
+        const int w = chain_count(P.device, h->ch_budget, want, T.max_level_width, P.chain_spread);
         if (h->ch_budget < 1 || !chain_fits(P.device, false))
             return fail(h, MFCFD_ERR_CUDA, "chain sweep kernel cannot be resident");
         int64_t terms[3];
@@ -1663,10 +1667,11 @@ int mfcfd_set_chain_warps(mfcfd_handle *h, int32_t warps, int32_t *actual) {
         if (!h->staged) return fail(h, MFCFD_ERR_ARG, "handle has no device state");
         // a prepared handle: rebuild the staged schedule before it is attached
         mfcfd_handle::Staged &st = *h->staged;
+        h->ch_want = warps;
         h->ch_budget = chain_budget(h->P.device, warps, h->P.chain_spread, &h->ch_wpb);
         if (h->ch_budget < 1) return fail(h, MFCFD_ERR_CUDA, "chain sweep kernel cannot be resident");
         st.S = ChainSchedule();   // built for these chains at the next dry run or attach
-        st.chains = chain_count(h->P.device, h->ch_budget, h->T.max_level_width, h->P.chain_spread);
+        st.chains = chain_count(h->P.device, h->ch_budget, warps, h->T.max_level_width, h->P.chain_spread);
         if (actual) *actual = h->ch_budget;
         return MFCFD_OK;
     });
@@ -1695,14 +1700,27 @@ int mfcfd_tune_chain(mfcfd_handle *h, const int32_t *candidates, int32_t count, 
         double res_old = 0.0;
         int rc = mfcfd_get_state(h, prim.data(), delu.data(), &res_old);
         if (rc) return rc;
-        const int start = h->ch_budget;
+        const int start = h->ch_want;
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         CK(cudaEventCreate(&e0));
         CK(cudaEventCreate(&e1));
         double best_ms = 0.0;
         int best = start;
+        // candidates of one chain count are one schedule, timed once; the
+        // smallest budget among them is kept
+        std::vector<int> chains(wants.size());
+        std::vector<double> times(wants.size());
         for (size_t c = 0; c < wants.size() && rc == MFCFD_OK; ++c) {
-            int w = 0;
+            int w = 0, wpb = 0;
+            w = chain_budget(h->P.device, wants[c], h->P.chain_spread, &wpb);
+            chains[c] = chain_count(h->P.device, w, wants[c], h->T.max_level_width, h->P.chain_spread);
+            const size_t same = std::find(chains.begin(), chains.begin() + (long)c, chains[c]) - chains.begin();
+            if (same < c) {
+                times[c] = times[same];
+                if (ms) ms[c] = times[c];
+                if (times[c] == best_ms && wants[c] < best) best = wants[c];
+                continue;
+            }
             if ((rc = apply_chain_schedule(h, wants[c], &w))) break;
             // one untimed iteration, then `iters` timed ones, from the saved state
             if ((rc = mfcfd_set_state(h, prim.data(), delu.data(), res_old))) break;
@@ -1715,10 +1733,11 @@ int mfcfd_tune_chain(mfcfd_handle *h, const int32_t *candidates, int32_t count, 
             float t = 0.f;
             cudaEventElapsedTime(&t, e0, e1);
             const double per = t / iters;
+            times[c] = per;
             if (ms) ms[c] = per;
             if (c == 0 || per < best_ms) {
                 best_ms = per;
-                best = w;
+                best = wants[c];
             }
         }
         cudaEventDestroy(e0);

@@ -419,11 +419,16 @@ int device_sms(int device);
 int chain_budget(int device, int want, int spread, int *wpb);
 // Slots of that budget.
 int chain_budget_slots(int budget, int wpb, int precision, int spread);
-// Chains of a schedule: 1.5 times the widest level (one and a half keeps every
-// level's points moving; 62k points: 6.83 ms per iteration against 6.91 with
-// twice and 6.93 with once), at most what the device holds as teams of four
-// unless that is below 0.85 times the level, and at most the budget.
-int chain_count(int device, int budget, int width, int spread);
+// Chains of a schedule for about `want` warps: 1.5 times the widest level for
+// the default of twice the level (one and a half keeps every level's points
+// moving), a third of a chain more or less for each warp more or less, so that
+// mfcfd_tune_chain's candidates differ; at most the budget and, up to the
+// default, what the device holds as teams of four unless that is below 0.85
+// times the level.  FP64, ms per iteration with 1, 1.5 (default), 1.83 and 2.17
+// times the level: 62k points 5.10, 4.97, 4.88, 4.90; 260k 10.00, 9.85, 10.73,
+// 10.84; 1.1M points, whose level is 376, 27.8 with 376 or (default) 396 chains,
+// 39.0 and 47.7 with more than teams of four fit.
+int chain_count(int device, int budget, int want, int width, int spread);
 // Whether the chain kernels hold the blocks per SM that the slots count on.
 bool chain_fits(int device, bool group);
 // Per-device launch set-up (kernel attributes), done before a stream capture.

@@ -1575,13 +1575,13 @@ int chain_budget_slots(int budget, int wpb, int precision, int spread) {
     return (budget + wpb - 1) / wpb * each;
 }
 
-int chain_count(int device, int budget, int width, int spread) {
+int chain_count(int device, int budget, int want, int width, int spread) {
     if (spread) return budget;
-    int c = 3 * width / 2;
+    long c = (2L * want + 5L * width) / 6;
     const int most = 3 * chain_sms(device);          // teams of four the device holds
-    if (c > most && 20 * most >= 17 * width) c = most;
+    if (want <= 2 * width && c > most && 20 * most >= 17 * width) c = most;
     c = c < budget ? c : budget;
-    return c < 1 ? 1 : c;
+    return c < 1 ? 1 : (int)c;
 }
 
 // Rows [a, a + rows) of width w between the reference's index order and

@@ -462,7 +462,9 @@ int mfcfd_forces(mfcfd_handle *h, double wall_area, double ref_area, double *cl,
  * `iters` iterations (after one untimed) of each candidate warp count from
  * the current state, restores that state after each, and keeps the
  * fastest schedule.  candidates NULL with count 0 tries 1.5, 2, 3 and 4
- * times the widest sweep level (the default budget is 2).  *chosen
+ * times the widest sweep level (the default budget is 2); more warps are
+ * more chains, and candidates that give the same chains are timed once and
+ * the smallest budget of them kept.  *chosen
  * receives the kept schedule's budget and ms (count or 4 entries, may be
  * NULL) each candidate's milliseconds per iteration.  The schedule orders
  * the work only: results are the same bits with any choice.

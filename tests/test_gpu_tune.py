@@ -103,3 +103,25 @@ def test_server_chain_percent_keeps_results(mfcfd_lib):
             out.append(srv.wait(srv.submit(c, 0.8, 2.0, max_iters=30, residue_target=-9.0), timeout=120))
     assert out[0]["status"] == 0 and out[1]["status"] == 0
     assert np.array_equal(out[0]["prim"], out[1]["prim"]) and out[0]["res_new"] == out[1]["res_new"]
+
+
+def test_default_candidates_are_different_schedules(mfcfd_lib):
+    from mfcfd import cloud
+    from mfcfd.solver import Solver
+    s = Solver(cloud.shell_cloud(26, 361, seed=2, knn_device=0), 0.5, 1.0)
+    s.initial_conditions()
+    width = s.info()["max_level_width"]
+    kept = s.digest("ch_items0")
+    digests = []
+    for num in (3, 4, 6, 8):
+        s.set_chain_warps(num * width // 2)
+        digests.append(s.digest("ch_items0"))
+    assert len(set(digests)) == 4 and kept == digests[1]
+    # the kept schedule is a timed candidate's, and one asked for twice is timed once
+    chosen, ms = s.tune_chain([4 * width, width, 4 * width], iters=2)
+    assert ms[0] == ms[2]
+    assert s.info()["chain_warps"] == chosen
+    best = 4 * width if ms[0] < ms[1] else width
+    after = s.digest("ch_items0")
+    assert s.set_chain_warps(best) == chosen and s.digest("ch_items0") == after
+    s.close()
