@@ -462,12 +462,31 @@ __device__ __noinline__ PointOut point_general(const double *frame0, const Sweep
     return o;
 }
 
+// A point's own flux where the shared frame is not the global axes: component c
+// of list dd at the conserved state U in frame F.  A kernel of its own (AXES
+// false), since the launch knows the frame: one kernel with both forms had up to
+// 5% slower sweeps in the axes.  62,400 points with a turned frame, ms per
+// iteration: FP64 5.1 (9.0 with the operators after a straight-line form that
+// such a frame always left), mixed precision 4.0 (6.1).
+template <typename R>
+__device__ __forceinline__ R turned_flux(int dd, int c, const R U[5], const FrameT<R> &F, const FrameT<R> &F0, bool &ok) {
+    FluxPreT<R> P;
+    R yspb, e, er;
+    state_core(U, F, F0, P, yspb, ok);
+    const int a = dd >> 1;
+    const bool pos = (dd & 1) == 0;
+    const R ua = pick3(a, P.ut1, P.ut2, P.un);
+    gauss_core(ua * P.sb, e, er, ok);
+    const R B = quot_nz(R(0.5) * e, P.spb, yspb), A = R(0.5) * (R(1.0) + (pos ? er : -er));
+    return split_component(pos, c == a + 1, c, P.rho, P.pr, ua, pick3(c - 1, P.ut1, P.ut2, P.un), P.usq, A, B);
+}
+
 // A point in the shared frame, or a wall point, of a cloud with a shared frame
 // under the alias driver: the sweep's common cases, kept apart from the others
 // so that their code is short, free of the others' branches and, beyond the
 // sums, the same for both (a wall point's own code is seldom in the
-// instruction cache).
-template <typename R, bool FOLD>
+// instruction cache).  AXES: the shared frame is the global axes.
+template <typename R, bool FOLD, bool AXES>
 __device__ __forceinline__ void common_point(const DevCloud &d, const ChainItem &it, const SweepStage *st, bool forward,
                                              int lane, int word, int dd, int c, double *T, const Team &team, int pos,
                                              bool g0_newer) {
@@ -479,7 +498,7 @@ __device__ __forceinline__ void common_point(const DevCloud &d, const ChainItem 
     const int lo = count_sum(it.cnt & ((1u << (5 * dd)) - 1u)), n = item_count(it.cnt, dd);
     double g[7] = {0, 0, 0, 0, 0, 0, 1.0};
     double ydet = 0.0;
-    bool ok = d.frame0_axes != 0;
+    bool ok = !AXES || d.frame0_axes != 0;
     if constexpr (!FOLD) {
 #pragma unroll
         for (int r = 0; r < 7; ++r) g[r] = st->geo[dd * 8 + r];
@@ -520,15 +539,23 @@ __device__ __forceinline__ void common_point(const DevCloud &d, const ChainItem 
     R Un[5];
 #pragma unroll
     for (int r = 0; r < 5; ++r) Un[r] = (R)__shfl_sync(FULL, un, r);
-    if (wall) {
-        // back from the point's frame (conserved_to_primitive)
-        FrameT<R> F;
-        load_frame(st->frame, F);
-        const R m1 = Un[1], m2 = Un[2], m3 = Un[3];
+    double flux;
+    if constexpr (AXES) {
+        if (wall) {
+            // back from the point's frame (conserved_to_primitive)
+            FrameT<R> F;
+            load_frame(st->frame, F);
+            const R m1 = Un[1], m2 = Un[2], m3 = Un[3];
 #pragma unroll
-        for (int r = 0; r < 3; ++r) Un[1 + r] = F.t1[r] * m1 + F.t2[r] * m2 + F.n[r] * m3;
+            for (int r = 0; r < 3; ++r) Un[1 + r] = F.t1[r] * m1 + F.t2[r] * m2 + F.n[r] * m3;
+        }
+        flux = (double)state_flux(dd, c, Un, ok);
+    } else {
+        FrameT<R> F, F0;
+        load_frame(st->frame, F);
+        load_frame(d.frame0, F0);
+        flux = (double)turned_flux(dd, c, Un, F, F0, ok);
     }
-    double flux = (double)state_flux(dd, c, Un, ok);
     if (!__all_sync(FULL, ok)) {
         const PointOut o = point_general<R, FOLD>(d.frame0, st, wall, forward, dd, c, s.x, s.y, s.z, dinv, base5);
         dnew = o.dnew;
@@ -654,7 +681,7 @@ __host__ __device__ constexpr int chain_smem_bytes(int team) {
 
 // One block of a cloud's chain sweep: block `block` of the cloud's
 // chain_blocks(ch_chains, ch_shape).
-template <typename R, bool FOLD>
+template <typename R, bool FOLD, bool AXES>
 __device__ __forceinline__ void chain_sweep(const DevCloud &d, int forward, int block) {
     extern __shared__ double smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -708,7 +735,7 @@ __device__ __forceinline__ void chain_sweep(const DevCloud &d, int forward, int 
             const ChainItem after = pos + 2 * size < len ? items[pos + 2 * size] : nxt;
             team_enter(d, team, pos, lane);
             if ((cur.info & (CI_SHARED | CI_WALL)) && d.shared_frame && !d.dg_old)
-                common_point<R, FOLD>(d, cur, &stg[s], forward != 0, lane, word, dd, c, T, team, pos, more);
+                common_point<R, FOLD, AXES>(d, cur, &stg[s], forward != 0, lane, word, dd, c, T, team, pos, more);
             else
                 general_point<R, FOLD>(d, cur, &stg[s], forward != 0, lane, T, team, pos, more);
             cur = nxt;

@@ -1188,9 +1188,9 @@ namespace mfcfd {
 // kernels of other handles between their sweeps.
 constexpr int CH_FREE_SMS = 16;
 
-template <typename R, bool FOLD, bool DENSE>
+template <typename R, bool FOLD, bool DENSE, bool AXES>
 __global__ void __launch_bounds__(CH_WPB * 32, DENSE ? 3 : 2) k_sweep_chain(const __grid_constant__ DevCloud d, int forward) {
-    chain_sweep<R, FOLD>(d, forward, blockIdx.x);
+    chain_sweep<R, FOLD, AXES>(d, forward, blockIdx.x);
 }
 
 // The chain sweeps of a group of clouds in one launch: blocks
@@ -1198,12 +1198,12 @@ __global__ void __launch_bounds__(CH_WPB * 32, DENSE ? 3 : 2) k_sweep_chain(cons
 // nothing; a block finds its cloud and runs that cloud's schedule as the
 // single-cloud kernel would.  The group lives in the launch's parameters, so
 // every block reads its cloud's pointers from the constant bank.
-template <typename R, bool FOLD, bool DENSE>
+template <typename R, bool FOLD, bool DENSE, bool AXES>
 __global__ void __launch_bounds__(CH_WPB * 32, DENSE ? 3 : 2)
     k_sweep_chain_group(const __grid_constant__ ChainGroup g, int forward) {
     int c = 0;
     while (c + 1 < g.count && (int)blockIdx.x >= g.block_start[c + 1]) ++c;
-    chain_sweep<R, FOLD>(g.cloud[c], forward, (int)blockIdx.x - g.block_start[c]);
+    chain_sweep<R, FOLD, AXES>(g.cloud[c], forward, (int)blockIdx.x - g.block_start[c]);
 }
 
 // three blocks per SM: 228 KB of shared memory, 1 KB of it reserved per block
@@ -1492,6 +1492,18 @@ int residual_noalloc(const DevCloud &d, cudaStream_t s, double *res_new, std::st
     return MFCFD_OK;
 }
 
+// f(kernel, its group form, whether three blocks share an SM) for each form of
+// the chain sweep.
+template <typename F>
+static void each_chain_kernel(F f) {
+    f(k_sweep_chain<double, false, false, true>, k_sweep_chain_group<double, false, false, true>, false);
+    f(k_sweep_chain<double, false, true, true>, k_sweep_chain_group<double, false, true, true>, true);
+    f(k_sweep_chain<float, true, true, true>, k_sweep_chain_group<float, true, true, true>, true);
+    f(k_sweep_chain<double, false, false, false>, k_sweep_chain_group<double, false, false, false>, false);
+    f(k_sweep_chain<double, false, true, false>, k_sweep_chain_group<double, false, true, false>, true);
+    f(k_sweep_chain<float, true, true, false>, k_sweep_chain_group<float, true, true, false>, true);
+}
+
 // Sets the kernels' shared-memory limits once per device.
 static void set_attributes(int device) {
     static std::mutex mu;
@@ -1513,12 +1525,10 @@ static void set_attributes(int device) {
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN_SPREAD_SMEM);
     };
-    chain(k_sweep_chain<double, false, false>);
-    chain(k_sweep_chain<double, false, true>);
-    chain(k_sweep_chain<float, true, true>);
-    chain(k_sweep_chain_group<double, false, false>);
-    chain(k_sweep_chain_group<double, false, true>);
-    chain(k_sweep_chain_group<float, true, true>);
+    each_chain_kernel([&](auto *kern, auto *group, bool) {
+        chain(kern);
+        chain(group);
+    });
     done[device] = true;
 }
 
@@ -1548,13 +1558,10 @@ bool chain_fits(int device, bool group) {
         }
         return true;
     };
-    const bool fits = chain_sms(device) >= 1 &&
-                      (group ? holds(k_sweep_chain_group<double, false, false>, 2) &&
-                                   holds(k_sweep_chain_group<double, false, true>, 3) &&
-                                   holds(k_sweep_chain_group<float, true, true>, 3)
-                             : holds(k_sweep_chain<double, false, false>, 2) &&
-                                   holds(k_sweep_chain<double, false, true>, 3) &&
-                                   holds(k_sweep_chain<float, true, true>, 3));
+    bool fits = chain_sms(device) >= 1;
+    each_chain_kernel([&](auto *kern, auto *grp, bool three) {
+        fits = fits && (group ? holds(grp, three ? 3 : 2) : holds(kern, three ? 3 : 2));
+    });
     k = fits ? 2 : 1;
     return fits;
 }
@@ -1647,12 +1654,27 @@ static cudaError_t launch_prio(void (*kern)(Args...), int grid, int block, size_
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Act>(args)...);
 }
 
+// The kernel of a chain sweep in its group form or not: f(kernel).
+template <typename F>
+static void with_chain_kernel(bool axes, bool mixed, bool dense, F f) {
+    int k = 0;
+    each_chain_kernel([&](auto *kern, auto *group, bool) {
+        if (k++ == (axes ? 0 : 3) + (mixed ? 2 : dense ? 1 : 0)) f(kern, group);
+    });
+}
+// Whether a cloud's sweeps may take the kernels of the global axes (no point
+// of a cloud without a shared frame takes the path in question).
+static bool chain_axes(const DevCloud &d) { return !d.shared_frame || d.frame0_axes; }
+
 cudaError_t launch_chain_group(const ChainGroup &g, const ChainShape &c, int precision, int forward, cudaStream_t s) {
     const int blocks = g.block_start[g.count], smem = chain_smem(c), threads = CH_WPB * 32;
-    if (precision != MFCFD_PRECISION_FP64)
-        return launch_prio(k_sweep_chain_group<float, true, true>, blocks, threads, smem, s, true, g, forward);
-    if (c.dense) return launch_prio(k_sweep_chain_group<double, false, true>, blocks, threads, smem, s, true, g, forward);
-    return launch_prio(k_sweep_chain_group<double, false, false>, blocks, threads, smem, s, true, g, forward);
+    bool axes = true;
+    for (int i = 0; i < g.count; ++i) axes = axes && chain_axes(g.cloud[i]);
+    cudaError_t e = cudaSuccess;
+    with_chain_kernel(axes, precision != MFCFD_PRECISION_FP64, c.dense != 0, [&](auto *, auto *group) {
+        e = launch_prio(group, blocks, threads, smem, s, true, g, forward);
+    });
+    return e;
 }
 
 cudaError_t launch_iteration(const DevCloud &d, int iter_slot, const IterStreams &st, double *U_next,
@@ -1676,9 +1698,9 @@ cudaError_t launch_iteration(const DevCloud &d, int iter_slot, const IterStreams
             const ChainShape &c = d.ch_shape;
             const int blocks = chain_blocks(d.ch_chains, c), smem = chain_smem(c), threads = CH_WPB * 32;
             // MIXED and MIXED_DC: folded weights
-            if (mixed) launch_prio(k_sweep_chain<float, true, true>, blocks, threads, smem, s, true, d, forward);
-            else if (c.dense) launch_prio(k_sweep_chain<double, false, true>, blocks, threads, smem, s, true, d, forward);
-            else launch_prio(k_sweep_chain<double, false, false>, blocks, threads, smem, s, true, d, forward);
+            with_chain_kernel(chain_axes(d), mixed, c.dense != 0, [&](auto *kern, auto *) {
+                launch_prio(kern, blocks, threads, smem, s, true, d, forward);
+            });
         } else if (d.sweep_mode == MFCFD_SWEEP_LEVELS) {
             k_sweep_levels<<<1, SWEEP_THREADS, SWEEP_WARPS * SWEEP_SMEM_BYTES, s>>>(d, forward);
         } else {

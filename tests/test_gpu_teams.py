@@ -70,3 +70,37 @@ def test_straight_line_functions_equal_the_operators(tmp_path, name, args):
                     os.path.join(REPO, "tests", name + ".cu")], check=True)
     out = subprocess.run([exe] + args, capture_output=True, text=True)
     assert out.returncode == 0, out.stdout + out.stderr
+
+
+@pytest.mark.parametrize("iters", [1, 6])
+def test_turned_shared_frame_equals_the_level_schedule(mfcfd_lib, iters):
+    """Interior points that share a frame other than the global axes: its own
+    kernels, in every team size, and in a group beside a cloud in the axes."""
+    from mfcfd import batch, cloud
+    from mfcfd.solver import Solver
+    c = cloud.small_sphere(6, 100, r1=1.5, seed=3)
+    t1, t2, nor = c.tan1.copy(), c.tan2.copy(), c.nor.copy()
+    (ca, sa), (cb, sb) = (np.cos(0.3), np.sin(0.3)), (np.cos(0.5), np.sin(0.5))
+    inner = c.status == 0
+    t1[inner], t2[inner], nor[inner] = (ca, sa, 0.0), (-sa * cb, ca * cb, sb), (sa * sb, -ca * sb, cb)
+    axes = c
+    c = dataclasses.replace(c, tan1=t1, tan2=t2, nor=nor)
+    ss = [Solver(c, 0.5, 1.0, sweep_mode=1)] + [Solver(c, 0.5, 1.0, chain_warps=w) for w in (0, 3, 32, 32)]
+    others = [Solver(axes, 0.5, 1.0, chain_warps=32) for _ in range(2)]
+    for s in ss + others:
+        s.initial_conditions()
+        assert s.info()["shared_frame"] == 1
+    for s in ss[:2]:
+        s.q_lskum(iters)                       # alone: the largest team
+    for s in ss[2:4]:
+        s.launch(1, iters)                     # teams of one and of two
+        s.complete()
+    others[0].q_lskum(iters)
+    batch.run_group([others[1], ss[4]], iters)
+    assert np.array_equal(*[s.get(mfcfd_lib.FIELD_PRIM) for s in others])
+    for f in ("DELUP", "DELUN", "PRIM"):
+        want = ss[0].get(getattr(mfcfd_lib, "FIELD_" + f))
+        for s in ss[1:]:
+            assert np.array_equal(s.get(getattr(mfcfd_lib, "FIELD_" + f)).view(np.uint64), want.view(np.uint64)), f
+    for s in ss + others:
+        s.close()
