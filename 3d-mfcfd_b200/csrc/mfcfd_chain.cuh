@@ -324,6 +324,56 @@ __device__ __forceinline__ void shared_sums(const DevCloud &d, const SweepEntry 
     }
 }
 
+// The same for the backup driver, whose terms may be from before the sweep
+// (ENT_OLD: from `old`): OLD_GATHER terms of each list are read together, then
+// the ring's.  Most of its terms are old, so what counts is how many reads are
+// in flight (62,400 points: 3.4 ms an iteration, 6.4 with a poll per term).
+constexpr int OLD_GATHER = 8;
+template <bool FOLD>
+__device__ __forceinline__ void old_sums(const DevCloud &d, const SweepEntry *E, int n, const double *src, const double *old,
+                                         unsigned rl, const Team &team, int pos, Sums<FOLD> &s) {
+    const int nmax = (int)__reduce_max_sync(FULL, (unsigned)n);
+    for (int base = 0; base < nmax; base += OLD_GATHER, E += OLD_GATHER) {
+        const int m = min(n - base, OLD_GATHER);
+        const double *at[OLD_GATHER];
+        unsigned long long v[OLD_GATHER];
+        unsigned rm = 0;               // this list's ring terms
+#pragma unroll
+        for (int q = 0; q < OLD_GATHER; ++q) {
+            const int2 kp = *reinterpret_cast<const int2 *>(&E[q]);
+            const bool in = q < m, ring = (kp.y & ENT_RING) != 0;
+            at[q] = ((kp.y & ENT_OLD) ? old : src) + DG_STRIDE * (long long)(in ? kp.x : 0);
+            rm |= in && ring ? 1u << q : 0u;
+            v[q] = 0;
+            ldg_if(v[q], at[q], in && !ring);
+        }
+        int spins = 0;
+        for (;;) {
+            bool pend = false;
+#pragma unroll
+            for (int q = 0; q < OLD_GATHER; ++q) pend = pend || pending_word(v[q]);
+            if (!__any_sync(FULL, pend)) break;
+            if (pend && !spin_continue(spins, d)) {
+                // the wait ran out (d.err is set): the terms stay unset
+#pragma unroll
+                for (int q = 0; q < OLD_GATHER; ++q) v[q] = pending_word(v[q]) ? 0 : v[q];
+            }
+#pragma unroll
+            for (int q = 0; q < OLD_GATHER; ++q) ldg_if(v[q], at[q], pending_word(v[q]));
+        }
+#pragma unroll
+        for (int q = 0; q < OLD_GATHER; ++q) {
+            const bool ring = (rm >> q) & 1u;
+            if (__any_sync(FULL, ring)) {
+                const int dist = ring ? ((pos - 1 - (E[q].pad >> ENT_RING_SHIFT)) & (CHAIN_RING - 1)) + 1 : 1;
+                const double t = ring_word(d, rl + ring_slot(team, pos, dist) * 256, ring);
+                if (ring) v[q] = (unsigned long long)__double_as_longlong(t);
+            }
+            s.term(q < m, __longlong_as_double((long long)v[q]), E[q]);
+        }
+    }
+}
+
 // A wall or interior point's slot: its fluxes along the three axes, less what T
 // holds, into T.  The sign of each axis's list is selected, not branched on.
 template <typename R>
@@ -485,7 +535,8 @@ __device__ __forceinline__ R turned_flux(int dd, int c, const R U[5], const Fram
 // under the alias driver: the sweep's common cases, kept apart from the others
 // so that their code is short, free of the others' branches and, beyond the
 // sums, the same for both (a wall point's own code is seldom in the
-// instruction cache).  AXES: the shared frame is the global axes.
+// instruction cache).  AXES: the shared frame is the global axes, and the driver
+// the alias one.
 template <typename R, bool FOLD, bool AXES>
 __device__ __forceinline__ void common_point(const DevCloud &d, const ChainItem &it, const SweepStage *st, bool forward,
                                              int lane, int word, int dd, int c, double *T, const Team &team, int pos,
@@ -579,7 +630,8 @@ __device__ __forceinline__ void common_point(const DevCloud &d, const ChainItem 
 // (folded when the handle is attached), so the sums are the derivatives;
 // otherwise the three weighted moments are summed in FP64 and solved, as the
 // reference does.
-template <typename R, bool FOLD>
+// OLD: points of the backup driver in the shared frame are among them.
+template <typename R, bool FOLD, bool OLD>
 __device__ __noinline__ void general_point(const DevCloud &d, ChainItem it, const SweepStage *st, bool forward, int lane,
                                            double *T, Team team, int pos, bool g0_newer) {
     const int p = it.p;
@@ -612,41 +664,32 @@ __device__ __noinline__ void general_point(const DevCloud &d, ChainItem it, cons
             if (e == dd) n = ce;
         }
         const SweepEntry *E = st->ent + lo;
-        const bool shared = (it.info & CI_SHARED) != 0;   // backup driver
+        const bool shared = OLD && (it.info & CI_SHARED) != 0;
         if (!shared) {
             const int cls = wall ? CLS_WALL : (outer ? CLS_OUTER : CLS_INTERIOR);
             unshared_terms<R>(d, it, st, cls, forward, lane, T, g0_newer);
         }
-        double sx = 0.0, sy = 0.0, sz = 0.0;
-#pragma unroll 4
-        for (int j = 0; j < n; ++j) {
-            const int pad = E[j].pad;
-            double t;
-            if (!shared) {
-                t = T[(dd * MAX_SLOTS + ((pad >> 8) & 255)) * 5 + c];
-            } else if (pad & ENT_RING) {
-                const int dist = ((pos - 1 - (pad >> ENT_RING_SHIFT)) & (CHAIN_RING - 1)) + 1;
-                const unsigned w = smem_addr(team.ring + ring_slot(team, pos, dist) * 32 + word);
-                int spins = 0;
-                do {
-                    t = lds_relaxed(w);
-                } while (is_pending(t) && team_spin_continue(spins, d));
-            } else {
-                // a term from before the sweep reads dg_old
-                const double *s = (pad & ENT_OLD) ? d.dg_old : (forward ? d.dgf : d.dgb);
-                t = poll_word(s + DG_STRIDE * (size_t)E[j].k + DG_LIST * dd + c, d);
-            }
-            sx = sx + t * E[j].w[0];
-            if constexpr (!FOLD) {
-                sy = sy + t * E[j].w[1];
-                sz = sz + t * E[j].w[2];
+        Sums<FOLD> s;
+        if (OLD && shared) {
+            const double *src = (forward ? d.dgf : d.dgb) + (DG_LIST * dd + c);
+            old_sums<FOLD>(d, E, n, src, d.dg_old + (DG_LIST * dd + c), smem_addr(team.ring + word), team, pos, s);
+        } else {
+            const double *Tl = T + dd * MAX_SLOTS * 5 + c;
+            const int nmax = (int)__reduce_max_sync(FULL, (unsigned)n);
+            for (int j = 0; j < nmax; j += 2) {
+                // past the list's end: its first terms, unused
+                double t[2];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) t[q] = Tl[((E[j + q < n ? j + q : 0].pad >> 8) & (MAX_SLOTS - 1)) * 5];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) s.term(j + q < n, t[q], E[j + q < n ? j + q : 0]);
             }
         }
         __syncwarp();
-        double G = sx;
+        double G = s.x;
         if constexpr (!FOLD) {
             const double *g = st->geo + ((outer && dd == 4) ? 5 : dd) * 8;   // outer z+ over conn: row 5
-            G = cramer_select(dd >> 1, g, sx, sy, sz) / g[6];
+            G = cramer_select(dd >> 1, g, s.x, s.y, s.z) / g[6];
         }
         double gd[NDIR];
 #pragma unroll
@@ -737,7 +780,7 @@ __device__ __forceinline__ void chain_sweep(const DevCloud &d, int forward, int 
             if ((cur.info & (CI_SHARED | CI_WALL)) && d.shared_frame && !d.dg_old)
                 common_point<R, FOLD, AXES>(d, cur, &stg[s], forward != 0, lane, word, dd, c, T, team, pos, more);
             else
-                general_point<R, FOLD>(d, cur, &stg[s], forward != 0, lane, T, team, pos, more);
+                general_point<R, FOLD, !AXES>(d, cur, &stg[s], forward != 0, lane, T, team, pos, more);
             cur = nxt;
             nxt = after;
             s ^= 1;

@@ -1662,9 +1662,10 @@ static void with_chain_kernel(bool axes, bool mixed, bool dense, F f) {
         if (k++ == (axes ? 0 : 3) + (mixed ? 2 : dense ? 1 : 0)) f(kern, group);
     });
 }
-// Whether a cloud's sweeps may take the kernels of the global axes (no point
-// of a cloud without a shared frame takes the path in question).
-static bool chain_axes(const DevCloud &d) { return !d.shared_frame || d.frame0_axes; }
+// Whether a cloud's sweeps may take the kernels of the global axes and the
+// alias driver (no point of a cloud without a shared frame takes the paths in
+// question).
+static bool chain_axes(const DevCloud &d) { return !d.shared_frame || (d.frame0_axes && !d.dg_old); }
 
 cudaError_t launch_chain_group(const ChainGroup &g, const ChainShape &c, int precision, int forward, cudaStream_t s) {
     const int blocks = g.block_start[g.count], smem = chain_smem(c), threads = CH_WPB * 32;
