@@ -458,7 +458,7 @@ int run_iterations(mfcfd_handle *h, int32_t t0, int32_t iters, double *res_hist)
     int status = MFCFD_OK;
     for (int32_t done = 0; done < iters;) {
         ChunkSlots slots{SlotPool::Lease(), h->stream};
-        if (int rc = take_slots(h, SLOTS_EVEN, true, &slots.lease)) return rc;
+        if (int rc = take_slots(h, SLOTS_ALL, true, &slots.lease)) return rc;
         const int chunk = slots.lease.chunk(std::min<int32_t>(iters - done, h->res_cap));
         int rc = launch_chunk(h, chunk, false);
         if (!rc) rc = chunk_launched(h, &slots.lease);
@@ -1236,7 +1236,8 @@ int mfcfd_debug_digest(mfcfd_handle *h, const char *name, uint64_t *digest, int6
             {"fwd_need", d.fwd_need, 4 * n}, {"bwd_need", d.bwd_need, 4 * n},
             {"fwd_old", d.fwd_old, 4 * n}, {"bwd_old", d.bwd_old, 4 * n},
             {"sweep_slot_mask", d.sweep_slot_mask, n * MAX_SLOTS}, {"res_order", d.res_order, 4 * (size_t)d.n_res},
-            {"pre_order", nullptr, 0}, {"g0_pts", d.g0_pts, 4 * (size_t)d.n_g0},
+            {"pre_order", nullptr, 0},   // an array the handle no longer has; its name stays known
+            {"g0_pts", d.g0_pts, 4 * (size_t)d.n_g0},
             {"ch_ptr0", d.ch_ptr[0], ch ? 4 * w1 : 0}, {"ch_pts0", d.ch_pts[0], ch ? 4 * nsw : 0},
             {"ch_own0", d.ch_own[0], ch ? 4 * n : 0}, {"ch_items0", d.ch_items[0], ch ? sizeof(ChainItem) * nsw : 0},
             {"ch_ptr1", d.ch_ptr[1], ch ? 4 * w1 : 0}, {"ch_pts1", d.ch_pts[1], ch ? 4 * nsw : 0},
@@ -1591,7 +1592,7 @@ int mfcfd_run_group(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
             graphs = graphs && hs[i]->P.graphs >= 1 && !hs[i]->graphs_off;
         }
         int first_err = MFCFD_OK;
-        const SlotAsk ask{chains.data(), count, d0.precision, h0->P.chain_spread, slots, SLOTS_EVEN};
+        const SlotAsk ask{chains.data(), count, d0.precision, h0->P.chain_spread, slots, SLOTS_ALL};
         for (int32_t done = 0; done < iters;) {
             ChunkSlots held{SlotPool::Lease(), gr.s};
             if (int rc = take_slots(h0, ask, true, gr.s, &held.lease)) return rc;

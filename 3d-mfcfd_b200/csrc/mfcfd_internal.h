@@ -427,7 +427,8 @@ int chain_budget_slots(int budget, int wpb, int precision, int spread);
 // times the level.  FP64, ms per iteration with 1, 1.5 (default), 1.83 and 2.17
 // times the level: 62k points 5.10, 4.97, 4.88, 4.90; 260k 10.00, 9.85, 10.73,
 // 10.84; 1.1M points, whose level is 376, 27.8 with 376 or (default) 396 chains,
-// 39.0 and 47.7 with more than teams of four fit.
+// 39.0 and 47.7 with more than teams of four fit.  With fewer than the level,
+// 0.85, 0.75 and 0.6 times: 260k 10.3, 12.7, 30.1; 1.1M 28.7, 38.8, 91.
 int chain_count(int device, int budget, int want, int width, int spread);
 // Whether the chain kernels hold the blocks per SM that the slots count on.
 bool chain_fits(int device, bool group);

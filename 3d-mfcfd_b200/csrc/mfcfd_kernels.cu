@@ -1181,10 +1181,10 @@ namespace mfcfd {
 // mixed precision (three per SM: at most 168 registers and 76 KB of shared
 // memory), 3 in FP64 (two per SM: 254 registers, no spills), or 2 in the dense
 // FP64 build (168 registers, 100 bytes spilled), which a cloud takes whose teams
-// need more than two blocks per SM (1.1M points, 376 teams of four: 37.0 ms
-// per iteration against 41.5 as teams of two on more chains).  The sweeps at
-// once take at most 6 * (SMs - CH_FREE_SMS) slots, or 4 of each of these SMs
-// where their blocks differ in size (SlotPool); the other SMs' room is for the
+// need more than two blocks per SM (1.1M points, 396 teams of four: 27.9 ms
+// per iteration against 31.6 as teams of two without the spills).  The sweeps at
+// once take at most 6 * (SMs - CH_FREE_SMS) slots, a block half an SM at least
+// where they differ in size (SlotPool); the other SMs' room is for the
 // kernels of other handles between their sweeps.
 constexpr int CH_FREE_SMS = 16;
 
@@ -1730,9 +1730,9 @@ cudaError_t launch_iteration(const DevCloud &d, int iter_slot, const IterStreams
         else k_g0<double><<<gb, 128, 0, s>>>(d);
     }
     if (chains) {
-        // before the sweeps, whose teams leave no room beside them (1.1M points:
-        // 37.0 ms per iteration against 39.5 to 112 with the flux residual
-        // beside the forward sweep; 62k: 7.0 against 6.9)
+        // before the sweeps, whose teams leave no room beside them (when the
+        // teams came, 1.1M points took about 5% longer with the flux residual
+        // beside the forward sweep, 62,400 points 1% less)
         const size_t fsm = FLUX_WARPS * FLUX_SMEM_PER_WARP * 8;
         // a smaller grid walks the same order with its warps striding through it
         const int fgrid = d.flux_grid > 0 && d.flux_grid < fblocks ? d.flux_grid : fblocks;

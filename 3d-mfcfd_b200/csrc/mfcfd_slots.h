@@ -41,37 +41,41 @@ inline int chain_slots(int chains, const ChainShape &c, int precision) {
 }
 
 // A run's claim: its handles' chain counts, the slots of their budgets, and the
-// slots it would use if they were free (SLOTS_EVEN: an even share with the runs
-// that hold slots).
+// slots it would use if they were free (SLOTS_ALL: any).
 struct SlotAsk {
     const int *chains;
     int count, precision, spread, budget, want;
 };
-constexpr int SLOTS_EVEN = -1;
-// Iterations that a chunk beyond its run's budget lasts at most, so that whoever
-// asks next does not wait for it long.
+constexpr int SLOTS_ALL = 1 << 20;
+// Iterations that a chunk lasts at most beyond its run's budget, so that whoever
+// asks next does not wait for it long, or beside others, so that their room is
+// taken up soon after they have ended.
 constexpr int LENT_CHUNK = 64;
 
 // Slots of a device's chain sweeps in use (chain_slot_capacity), over every
 // handle and thread of the process.  A run takes slots for one chunk of
-// iterations at a time: its handles' budgets (mfcfd_info.chain_slots) at once,
-// and more while they are free.  Where its budget does not fit beside the
-// chunks that hold slots, its own chunk waits on the device for some of them
-// to end (those that hold more than their budgets first, the oldest first): a
-// host thread waits for another's launch calls at most, never for its
-// iterations.  What a run holds counts from the moment it asks, so the others'
-// next chunks leave it room.
+// iterations at a time: the most that it wants and that are free, at least its
+// handles' budgets (mfcfd_info.chain_slots).  Where these do not fit beside the
+// chunks that hold slots, its own chunk waits on the device for as few of them
+// as it must (those that hold more than their budgets first, the oldest first)
+// and takes what they leave: a host thread waits for another's launch calls at
+// most, never for its iterations.  What a run holds counts from the moment it
+// asks, so the others' next chunks leave it room or queue behind it, and runs
+// that each want the whole device alternate (sharing it would leave each with
+// teams of one: 62,400 points 10.7 ms an iteration against 5.0 with teams of
+// four; two groups of converging clouds 0.421 solves/s alternating, 0.389 with
+// the second beside the first).
 //
 // The sweeps on the device at any time fit it together: of those running, the
 // one that asked last had, when it asked, room beside all others that it did
 // not wait for.
 //
-// Blocks of one size fill SMs without a remainder: they may take all slots.
-// Where sizes differ, an SM that holds four slots may have no room for one
-// more block (two blocks of two slots beside one of three, or beside a spread
-// one, which needs half of the SM's shared memory): together they may take
-// four slots of each SM.  A handle in FP64 has a build of either size, so it
-// usually joins the size that is running.
+// Blocks of one size fill SMs without a remainder.  Where sizes differ, two
+// blocks of any size may leave no room for one more (two blocks of two slots
+// none for one of three, or for a spread one, which needs half of the SM's
+// shared memory), but never fewer: a block then counts as half an SM at least,
+// so some SM always has room for the next.  A handle in FP64 has a build of
+// either size and takes the one that fits.
 class SlotPool {
 public:
     // Slots taken, given back when the object goes: on every path, so with an
@@ -92,7 +96,7 @@ public:
         int slots() const { return slots_; }
         bool lent() const { return lent_; }                  // beyond the budget
         // Iterations of the next chunk, of `iters` to run.
-        int chunk(int iters) const { return lent_ ? std::min(iters, LENT_CHUNK) : iters; }
+        int chunk(int iters) const { return lent_ || beside_ ? std::min(iters, LENT_CHUNK) : iters; }
         const ChainShape &shape() const { return shape_; }
         // The chunk is launched; `end` is recorded behind it, and stays
         // recorded until the slots are given back.
@@ -107,17 +111,18 @@ public:
             std::swap(id_, o.id_);
             std::swap(slots_, o.slots_);
             std::swap(lent_, o.lent_);
+            std::swap(beside_, o.beside_);
             std::swap(shape_, o.shape_);
         }
         SlotPool *pool_ = nullptr;
         long id_ = 0;
         int slots_ = 0;
-        bool lent_ = false;
+        bool lent_ = false, beside_ = false;
         ChainShape shape_{};
     };
 
-    // Slots with the largest teams within max(budget, want) that have room now,
-    // or else with the shape within the budget that waits for the fewest chunks.
+    // Slots with the shape within max(budget, want) that waits for the fewest
+    // chunks, and of these the one with the largest teams.
     // after(end): has the chunk about to be launched wait for another's; false
     // if that fails.  Empty if it failed or, with `wait` false, instead of any
     // such wait (for a caller with chunks of its own to attend to).
@@ -125,24 +130,25 @@ public:
     Lease take(int capacity, const SlotAsk &a, bool wait, After after) {
         Lease l;
         std::unique_lock<std::mutex> lock(mu_);
-        const int want = a.want == SLOTS_EVEN ? capacity / ((int)held_.size() + 1) : a.want;
         // the order in which chunks are waited for
         std::vector<const Held *> order;
         for (int lent = 1; lent >= 0; --lent)
             for (const Held &h : held_)
                 if (h.lent == (lent != 0)) order.push_back(&h);
         size_t waits = order.size() + 1;
-        int block = 0;
+        int block = 0, halves = 0;
         for (ChainShape c{a.spread ? 1 : CH_WPB, 0, a.spread};;) {
-            int slots = 0;
-            for (int i = 0; i < a.count; ++i) slots += chain_slots(a.chains[i], c, a.precision);
-            slots = std::max(slots, a.budget);
+            const int each = chain_block_slots(c, a.precision);
+            int blocks = 0;
+            for (int i = 0; i < a.count; ++i) blocks += chain_blocks(a.chains[i], c);
+            const int slots = std::max(blocks * each, a.budget), half = std::max(slots, blocks * 3);
             const bool last = c.team == 1 && (c.dense || c.spread || a.precision != MFCFD_PRECISION_FP64);
-            const size_t w = waits_for(order, capacity, slots, chain_block_slots(c, a.precision));
+            const size_t w = waits_for(order, capacity, slots, half, each);
             const bool own = slots <= a.budget || (c.team == 1 && !c.dense);   // (teams of one fit their budget)
-            if (w < waits && (own || (w == 0 && slots <= want))) {
+            if (w < waits && (own || slots <= a.want)) {
                 waits = w;
-                block = chain_block_slots(c, a.precision);
+                block = each;
+                halves = half;
                 l.shape_ = c;
                 l.slots_ = slots;
             }
@@ -152,9 +158,10 @@ public:
         }
         if (waits > 0 && !wait) return Lease();
         l.lent_ = l.slots_ > a.budget;
+        l.beside_ = !held_.empty();
         std::vector<long> ids;
         for (size_t k = 0; k < waits; ++k) ids.push_back(order[k]->id);
-        held_.push_back({next_, l.slots_, block, l.lent_, false, nullptr});
+        held_.push_back({next_, l.slots_, halves, block, l.lent_, false, nullptr});
         l.id_ = next_++;
         l.pool_ = this;
         // each was taken before this one, so no two wait for each other
@@ -177,21 +184,22 @@ public:
 private:
     struct Held {
         long id;
-        int slots, block;                                    // of them, slots of a block
+        int slots, halves, block;                            // slots beside blocks of other sizes; of a block
         bool lent, launched;
         void *end;
     };
     // How many of the chunks in `order` have to end before `slots` in blocks of
-    // `block` have room beside the others.
-    static size_t waits_for(const std::vector<const Held *> &order, int capacity, int slots, int block) {
+    // `block` (beside other sizes: `halves`) have room beside the others.
+    static size_t waits_for(const std::vector<const Held *> &order, int capacity, int slots, int halves, int block) {
         for (size_t w = 0; w < order.size(); ++w) {
-            int sum = slots;
+            int sum = slots, apart = halves;
             bool same = true;
             for (size_t k = w; k < order.size(); ++k) {
                 sum += order[k]->slots;
+                apart += order[k]->halves;
                 same = same && order[k]->block == block;
             }
-            if (sum <= (same ? capacity : capacity / 6 * 4)) return w;
+            if ((same ? sum : apart) <= capacity) return w;
         }
         return order.size();
     }

@@ -98,22 +98,27 @@ int launch_beside_a_run() {
     int end = 0;
     std::vector<void *> waited;
     auto after = [&](void *e) { return waited.push_back(e), true; };
-    SlotPool::Lease run = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 198, SLOTS_EVEN), true, no_wait);
+    SlotPool::Lease run = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 198, SLOTS_ALL), true, no_wait);
     REQUIRE(run.lent() && run.slots() == CAP);
     run.launched(&end);
     REQUIRE(!p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 300, 0), false, after) && waited.empty());
     SlotPool::Lease launch = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 300, 0), true, after);
     REQUIRE(run.chunk(1000) == LENT_CHUNK && run.chunk(10) == 10);   // not kept waiting for long
-    REQUIRE(launch.chunk(1000) == 1000);
+    REQUIRE(launch.chunk(1000) == LENT_CHUNK);                       // nor at its budget once there is room
     REQUIRE(launch && !launch.lent() && launch.slots() == 300 && waited == std::vector<void *>{&end});
     run = SlotPool::Lease();
-    run = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 198, SLOTS_EVEN), true, no_wait);
+    run = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 198, SLOTS_ALL), true, no_wait);
     REQUIRE(run && run.slots() <= CAP - 300);
     // a chunk whose wait cannot be queued does not run, and holds nothing
+    REQUIRE(run.chunk(1000) == LENT_CHUNK);
     const int before = p.held();
     run.launched(&end);
     launch.launched(&end);
     REQUIRE(!p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, CAP, 0), true, no_wait) && p.held() == before);
+    run = SlotPool::Lease();
+    launch = SlotPool::Lease();
+    launch = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 300, 0), true, no_wait);
+    REQUIRE(launch.chunk(1000) == 1000);                             // alone, within its budget
     return 0;
 }
 
@@ -134,7 +139,7 @@ int threads_share() {
                 while (!stop) {
                     all[k].emplace_back(new Chunk());
                     Chunk *c = all[k].back().get();
-                    SlotPool::Lease l = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, budget, SLOTS_EVEN), true, [&](void *e) {
+                    SlotPool::Lease l = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, budget, SLOTS_ALL), true, [&](void *e) {
                         c->after.push_back((Chunk *)e);
                         return true;
                     });
@@ -172,30 +177,46 @@ bool fits_sm(const int n[4]) {
     return regs <= 65536 && smem <= 228;
 }
 
-// The fewest slots that blocks of the kinds in `have` can hold on an SM without
-// room for another block of kind b.
-int fewest_without_room(const bool have[4], int b) {
-    int least = 1 << 20;
-    int n[4];
-    for (n[0] = 0; n[0] <= (have[0] ? 3 : 0); ++n[0])
-        for (n[1] = 0; n[1] <= (have[1] ? 3 : 0); ++n[1])
-            for (n[2] = 0; n[2] <= (have[2] ? 2 : 0); ++n[2])
-                for (n[3] = 0; n[3] <= (have[3] ? 2 : 0); ++n[3]) {
-                    if (!fits_sm(n)) continue;
-                    ++n[b];
-                    const bool room = fits_sm(n);
-                    --n[b];
-                    if (room) continue;
-                    int slots = 0;
-                    for (int k = 0; k < 4; ++k) slots += n[k] * BLOCKS[k].slots;
-                    least = std::min(least, slots);
-                }
-    return least;
+// Whether an SM that holds n has no room for another block of kind b.
+bool full_for(const int n[4], int b) {
+    int m[4] = {n[0], n[1], n[2], n[3]};
+    ++m[b];
+    return fits_sm(n) && !fits_sm(m);
+}
+
+// The most SMs that `blocks` (of each kind) can leave without room for one more
+// of kind b, bounded by duality: with weights of which every SM without room
+// holds 1 or more, the weight of all blocks.  In sixtieths.
+int most_without_room(const int blocks[4], int b) {
+    static std::vector<std::vector<int>> weights[16][4];
+    int have = 0;
+    for (int k = 0; k < 4; ++k) have |= blocks[k] > 0 ? 1 << k : 0;
+    auto &ws = weights[have][b];
+    if (ws.empty()) {
+        const int W[] = {0, 10, 15, 20, 30, 40, 60};
+        int n[4];
+        std::vector<std::vector<int>> full;
+        for (n[0] = 0; n[0] <= (have & 1 ? 3 : 0); ++n[0])
+            for (n[1] = 0; n[1] <= (have & 2 ? 3 : 0); ++n[1])
+                for (n[2] = 0; n[2] <= (have & 4 ? 2 : 0); ++n[2])
+                    for (n[3] = 0; n[3] <= (have & 8 ? 2 : 0); ++n[3])
+                        if (full_for(n, b)) full.push_back({n[0], n[1], n[2], n[3]});
+        for (int i = 0; i < 7 * 7 * 7 * 7; ++i) {
+            const int w[4] = {W[i % 7], W[i / 7 % 7], W[i / 49 % 7], W[i / 343]};
+            bool valid = true;
+            for (const auto &f : full) valid = valid && f[0] * w[0] + f[1] * w[1] + f[2] * w[2] + f[3] * w[3] >= 60;
+            if (valid) ws.push_back({w[0], w[1], w[2], w[3]});
+        }
+    }
+    int least = 1 << 30;
+    for (const auto &w : ws) least = std::min(least, blocks[0] * w[0] + blocks[1] * w[1] + blocks[2] * w[2] + blocks[3] * w[3]);
+    return least / 60;
 }
 
 // Blocks of different sizes leave parts of SMs that no other block fits, so
 // counting slots is not enough: the sweeps that the pool lets run at once are
-// all resident together, in whatever order their blocks were placed.
+// all resident together, in whatever order their blocks were placed, since
+// every block finds an SM with room whatever the others hold.
 int block_sizes() {
     unsigned seed = 1;
     auto rnd = [&](int n) { return (int)((seed = seed * 1664525u + 1013904223u) >> 8) % n; };
@@ -203,8 +224,8 @@ int block_sizes() {
     for (int round = 0; round < 20000; ++round) {
         SlotPool p;
         std::vector<SlotPool::Lease> running;
-        std::vector<int> kinds;
-        const int share = rnd(3) ? 1 + rnd(CAP) : SLOTS_EVEN;
+        int blocks[4] = {0, 0, 0, 0};
+        const int share = rnd(3) ? 1 + rnd(CAP) : SLOTS_ALL;
         for (int k = 0; k < 12; ++k) {
             const int precision = rnd(2) ? MFCFD_PRECISION_FP64 : MFCFD_PRECISION_MIXED, spread = rnd(8) == 0;
             const int chains = 1 + rnd(spread ? 100 : 264);
@@ -213,20 +234,23 @@ int block_sizes() {
             SlotPool::Lease l = p.take(CAP, a, false, no_wait);
             if (!l) continue;
             const ChainShape c = l.shape();
-            kinds.push_back(spread ? (precision == MFCFD_PRECISION_FP64 ? 2 : 3)
-                                   : (precision == MFCFD_PRECISION_FP64 && !c.dense ? 1 : 0));
+            blocks[spread ? (precision == MFCFD_PRECISION_FP64 ? 2 : 3)
+                          : (precision == MFCFD_PRECISION_FP64 && !c.dense ? 1 : 0)] += chain_blocks(chains, c);
             REQUIRE(l.slots() >= chain_slots(chains, c, precision) && (l.lent() || l.slots() == budget));
             running.push_back(std::move(l));
         }
-        bool have[4] = {false, false, false, false};
-        for (const int k : kinds) have[k] = true;
-        mixed_sizes += have[0] + have[1] + (have[2] || have[3]) > 1;
-        for (int b = 0; b < 4; ++b)
-            if (have[b] && !(p.held() - BLOCKS[b].slots < 148 * fewest_without_room(have, b))) {
-                std::printf("%d slots in use, a block of kind %d has no room where every SM holds %d\n", p.held(), b,
-                            fewest_without_room(have, b));
+        mixed_sizes += (blocks[0] > 0) + (blocks[1] > 0) + (blocks[2] + blocks[3] > 0) > 1;
+        for (int b = 0; b < 4; ++b) {
+            if (!blocks[b]) continue;
+            --blocks[b];
+            const int without = most_without_room(blocks, b);
+            ++blocks[b];
+            if (without >= 148) {
+                std::printf("%d, %d, %d and %d blocks: one of kind %d may have room on none of 148 SMs\n", blocks[0], blocks[1],
+                            blocks[2], blocks[3], b);
                 return 1;
             }
+        }
     }
     REQUIRE(mixed_sizes > 1000);
     return 0;
@@ -244,6 +268,7 @@ int block_size_choice() {
     SlotPool::Lease mixed = p.take(CAP, ask(many, MFCFD_PRECISION_MIXED, 132, 528), true, no_wait);
     REQUIRE(mixed.slots() == 528 && mixed.shape().team == 4);
     mixed.launched(&end);
+    // (blocks of three slots would count the running ones as half an SM each)
     SlotPool::Lease f64 = p.take(CAP, ask(few, MFCFD_PRECISION_FP64, 66, 264), true, no_wait);
     REQUIRE(f64 && f64.shape().dense == 1 && f64.shape().team == 4 && f64.slots() == 176);
     f64 = SlotPool::Lease();
