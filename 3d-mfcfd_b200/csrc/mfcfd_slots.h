@@ -145,7 +145,7 @@ public:
             const bool last = c.team == 1 && (c.dense || c.spread || a.precision != MFCFD_PRECISION_FP64);
             const size_t w = waits_for(order, capacity, slots, half, each);
             const bool own = slots <= a.budget || (c.team == 1 && !c.dense);   // (teams of one fit their budget)
-            if (w < waits && (own || slots <= a.want)) {
+            if (w < waits && (own || slots <= std::min(a.want, capacity))) {
                 waits = w;
                 block = each;
                 halves = half;

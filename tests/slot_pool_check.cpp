@@ -228,11 +228,13 @@ int block_sizes() {
         const int share = rnd(3) ? 1 + rnd(CAP) : SLOTS_ALL;
         for (int k = 0; k < 12; ++k) {
             const int precision = rnd(2) ? MFCFD_PRECISION_FP64 : MFCFD_PRECISION_MIXED, spread = rnd(8) == 0;
-            const int chains = 1 + rnd(spread ? 100 : 264);
+            const int chains = 1 + rnd(spread ? 130 : rnd(3) ? 264 : 1000);
             const int budget = (chains + 3) / 4 * (spread ? 6 : precision == MFCFD_PRECISION_FP64 ? 3 : 2);
             const SlotAsk a{&chains, 1, precision, spread, budget, share};
+            if (budget > CAP) continue;
             SlotPool::Lease l = p.take(CAP, a, false, no_wait);
             if (!l) continue;
+            REQUIRE(p.held() <= CAP);
             const ChainShape c = l.shape();
             blocks[spread ? (precision == MFCFD_PRECISION_FP64 ? 2 : 3)
                           : (precision == MFCFD_PRECISION_FP64 && !c.dense ? 1 : 0)] += chain_blocks(chains, c);
@@ -261,6 +263,15 @@ int block_sizes() {
 // neither fits beside the other.
 int block_size_choice() {
     SlotPool p;
+    {
+        // alone, too many chains for teams of four in either build but one
+        const int many = 396, more = 528;
+        const SlotPool::Lease l = p.take(CAP, ask(many, MFCFD_PRECISION_FP64, 297, SLOTS_ALL), true, no_wait);
+        REQUIRE(l.shape().team == 4 && l.shape().dense == 1 && l.slots() == CAP);
+        SlotPool q;
+        const SlotPool::Lease m = q.take(CAP, ask(more, MFCFD_PRECISION_FP64, 396, SLOTS_ALL), true, no_wait);
+        REQUIRE(m.shape().team == 2 && m.shape().dense == 0 && m.slots() == CAP);
+    }
     const int few = 88, many = 264;
     int end = 0;
     std::vector<void *> waited;
