@@ -86,7 +86,7 @@ struct mfcfd_handle {
     };
     GraphSlot graphs[4];
     int graph_next = 0;
-    cudaEvent_t batch_ev = nullptr;        // end of the handle's chunk in mfcfd_run_batch / mfcfd_launch
+    cudaEvent_t batch_ev = nullptr;        // end of the handle's last chunk
     int pending_chunk = 0;                 // mfcfd_launch: iterations not yet completed
     ChunkSlots pending_slots;              // ... and their slots
     // chain schedule: the warps it may hold beside other handles' (in blocks
@@ -276,7 +276,6 @@ int take_slots(mfcfd_handle *h, const SlotAsk &a, bool wait, cudaStream_t s, Slo
 // ... of one handle (none for the other schedules), its shape set; the chunk's
 // end is recorded in batch_ev.
 int take_slots(mfcfd_handle *h, int want, bool wait, SlotPool::Lease *l) {
-    if (!h->batch_ev) CK(cudaEventCreateWithFlags(&h->batch_ev, cudaEventDisableTiming));
     if (h->d.sweep_mode != MFCFD_SWEEP_CHAINS) return MFCFD_OK;
     const SlotAsk a{&h->d.ch_chains, 1, h->d.precision, h->P.chain_spread, budget_slots(h), want};
     if (int rc = take_slots(h, a, wait, h->stream, l)) return rc;
@@ -675,7 +674,7 @@ void keep_pool_memory(int device) {
     done.push_back(device);
 }
 
-// The handle's stream, of the highest priority, and its event.
+// The handle's stream, of the highest priority, and its events.
 int create_streams(mfcfd_handle *h) {
     if (cudaSetDevice(h->P.device) != cudaSuccess) return fail(h, MFCFD_ERR_CUDA, "cudaSetDevice failed");
     keep_pool_memory(h->P.device);
@@ -683,6 +682,7 @@ int create_streams(mfcfd_handle *h) {
     CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
     CK(cudaStreamCreateWithPriority(&h->stream, cudaStreamNonBlocking, greatest));
     CK(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&h->batch_ev, cudaEventDisableTiming));
     return MFCFD_OK;
 }
 
@@ -1408,11 +1408,18 @@ int mfcfd_run_batch(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
         std::vector<int32_t> done(count, 0);
         std::vector<int> chunk_of(count, 0);
         std::deque<int32_t> ready;
+        std::vector<ChunkSlots> slots(count);
         // every launched chunk ends (and its slots return) before an error
         // leaves the call
-        std::vector<ChunkSlots> slots(count);
         std::vector<int32_t> running;
         running.reserve(count);
+        struct Drain {
+            mfcfd_handle *const *hs;
+            const std::vector<int32_t> &running;
+            ~Drain() {
+                for (const int32_t i : running) cudaStreamSynchronize(hs[i]->stream);
+            }
+        } drain{hs, running};
         for (int32_t i = 0; i < count; ++i) {
             slots[i].stream = hs[i]->stream;
             if (iters > 0) ready.push_back(i);
@@ -1572,9 +1579,6 @@ int mfcfd_run_group(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
                             std::to_string(chain_slot_capacity(dev)) + ")");
         if (!chain_fits(dev, true))
             return fail(h, MFCFD_ERR_UNSUPPORTED, "the group sweep kernel holds fewer blocks per SM than a handle's");
-        for (int32_t i = 0; i < count; ++i)
-            if (!hs[i]->batch_ev && cudaEventCreateWithFlags(&hs[i]->batch_ev, cudaEventDisableTiming) != cudaSuccess)
-                return cuda_fail(hs[i], cudaGetLastError(), "cudaEventCreateWithFlags");
         prepare_launches(dev);
         auto G = std::make_unique<ChainGroup>();
         G->count = count;

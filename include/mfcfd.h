@@ -105,8 +105,8 @@ typedef struct mfcfd_params {
     int32_t sweep_variant;    /* MFCFD_SWEEPS_ALIAS (default) or MFCFD_SWEEPS_BACKUP */
     int32_t chain_warps;      /* CHAINS: warps the sweep may hold beside other handles'
                                  sweeps; 0 picks about twice the widest level (fewer
-                                 leave SMs to other clouds).  A sweep with the device to
-                                 itself takes more */
+                                 leave SMs to other clouds; more warps are more chains).  A
+                                 sweep with the device to itself takes more */
     int32_t gpu_setup;        /* 1: the set-up runs on params->device with the host's
                                  results.  mfcfd_create computes every topology array on
                                  the device (the host classifies and orders the points
@@ -471,8 +471,9 @@ int mfcfd_forces(mfcfd_handle *h, double wall_area, double ref_area, double *cl,
  */
 int mfcfd_tune_chain(mfcfd_handle *h, const int32_t *candidates, int32_t count, int32_t iters, int32_t *chosen,
                      double *ms);
-/* Rebuild the chain schedule for a budget of about `warps` warps (prepared or
- * attached handle); *actual (may be NULL) receives the budget.  In a batch,
+/* Rebuild the chain schedule for a budget of about `warps` warps, more warps
+ * being more chains (prepared or attached handle); *actual (may be NULL)
+ * receives the budget.  In a batch,
  * fewer warps per cloud (about the widest level) let more clouds share the
  * device; alone, about twice the widest level is fastest. */
 int mfcfd_set_chain_warps(mfcfd_handle *h, int32_t warps, int32_t *actual);
