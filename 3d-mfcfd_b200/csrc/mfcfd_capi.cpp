@@ -458,7 +458,7 @@ int run_iterations(mfcfd_handle *h, int32_t t0, int32_t iters, double *res_hist)
     for (int32_t done = 0; done < iters;) {
         ChunkSlots slots{SlotPool::Lease(), h->stream};
         if (int rc = take_slots(h, SLOTS_ALL, true, &slots.lease)) return rc;
-        const int chunk = slots.lease.chunk(std::min<int32_t>(iters - done, h->res_cap));
+        const int chunk = slots.lease.chunk(std::min<int32_t>(iters - done, h->res_cap), h->d.n);
         int rc = launch_chunk(h, chunk, false);
         if (!rc) rc = chunk_launched(h, &slots.lease);
         if (!rc) rc = finish_chunk(h, t0 + done, chunk, res_hist ? res_hist + 2 * (size_t)done : nullptr, &status);
@@ -1045,7 +1045,7 @@ extern "C++" int mfcfd::launch_within(mfcfd_handle *h, int32_t t0, int32_t iters
         CK(cudaSetDevice(h->P.device));
         ChunkSlots taken{SlotPool::Lease(), h->stream};
         if (int rc = take_slots(h, slots, wait, &taken.lease)) return rc;
-        if (launched) *launched = iters = taken.lease.chunk(iters);
+        if (launched) *launched = iters = taken.lease.chunk(iters, h->d.n);
         if (int rc = launch_chunk(h, iters, true)) return rc;
         if (int rc = chunk_launched(h, &taken.lease)) return rc;
         if (held) *held = taken.lease.slots();
@@ -1437,7 +1437,7 @@ int mfcfd_run_batch(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
                 int rc = take_slots(h, share, running.empty(), &slots[i].lease);
                 if (rc == MFCFD_ERR_BUSY) break;
                 ready.pop_front();
-                const int chunk = slots[i].lease.chunk(std::min<int32_t>(iters - done[i], std::max(h->res_cap, 1)));
+                const int chunk = slots[i].lease.chunk(std::min<int32_t>(iters - done[i], std::max(h->res_cap, 1)), h->d.n);
                 if (!rc) rc = launch_chunk(h, chunk, true);
                 if (!rc) rc = chunk_launched(h, &slots[i].lease);
                 if (rc) return rc;
@@ -1569,7 +1569,9 @@ int mfcfd_run_group(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
         if (cudaSetDevice(dev) != cudaSuccess) return MFCFD_ERR_CUDA;
         std::vector<int> chains(count);
         int slots = 0;
+        long points = 0;
         for (int32_t i = 0; i < count; ++i) {
+            points += hs[i]->d.n;
             chains[i] = hs[i]->d.ch_chains;
             slots += budget_slots(hs[i]);
         }
@@ -1604,7 +1606,7 @@ int mfcfd_run_group(mfcfd_handle *const *hs, int32_t count, const int32_t *t0, i
             G->block_start[0] = 0;
             for (int32_t i = 0; i < count; ++i)
                 G->block_start[i + 1] = G->block_start[i] + chain_blocks(chains[i], gr.shape);
-            const int chunk = held.lease.chunk(std::min<int32_t>(iters - done, res_cap));
+            const int chunk = held.lease.chunk(std::min<int32_t>(iters - done, res_cap), points);
             for (int32_t i = 0; i < count; ++i) hs[i]->res_valid = false;
             std::vector<int> cur(count), last(count);
             for (int32_t i = 0; i < count; ++i) cur[i] = hs[i]->cur, last[i] = hs[i]->last;

@@ -103,14 +103,14 @@ int launch_beside_a_run() {
     run.launched(&end);
     REQUIRE(!p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 300, 0), false, after) && waited.empty());
     SlotPool::Lease launch = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 300, 0), true, after);
-    REQUIRE(run.chunk(1000) == LENT_CHUNK && run.chunk(10) == 10);   // not kept waiting for long
-    REQUIRE(launch.chunk(1000) == LENT_CHUNK);                       // nor at its budget once there is room
+    REQUIRE(run.chunk(1000, 60000) == LENT_CHUNK && run.chunk(10, 60000) == 10);   // not kept waiting for long
+    REQUIRE(launch.chunk(1000, 600) == LENT_CHUNK);                       // nor at its budget once there is room
     REQUIRE(launch && !launch.lent() && launch.slots() == 300 && waited == std::vector<void *>{&end});
     run = SlotPool::Lease();
     run = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 198, SLOTS_ALL), true, no_wait);
     REQUIRE(run && run.slots() <= CAP - 300);
     // a chunk whose wait cannot be queued does not run, and holds nothing
-    REQUIRE(run.chunk(1000) == LENT_CHUNK);
+    REQUIRE(run.chunk(1000, 1104000) == 14 && run.chunk(1000, 100000000) == 2 && run.chunk(1, 100000000) == 1);
     const int before = p.held();
     run.launched(&end);
     launch.launched(&end);
@@ -118,7 +118,7 @@ int launch_beside_a_run() {
     run = SlotPool::Lease();
     launch = SlotPool::Lease();
     launch = p.take(CAP, ask(chains, MFCFD_PRECISION_FP64, 300, 0), true, no_wait);
-    REQUIRE(launch.chunk(1000) == 1000);                             // alone, within its budget
+    REQUIRE(launch.chunk(1000, 1104000) == 1000);                             // alone, within its budget
     return 0;
 }
 

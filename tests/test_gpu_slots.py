@@ -127,3 +127,30 @@ def test_chunks_beyond_the_budget_are_parts_of_longer_ones(mfcfd_lib, small_clou
     assert st["rounds"] == 2 and st["iterations"] == 200
     ref.close()
     s.close()
+
+
+def test_a_small_cloud_steps_beside_a_run_that_fills_the_device(mfcfd_lib):
+    """A run that holds every slot leaves another thread's cloud room from its
+    next chunk on, so that it steps while the run goes on."""
+    import threading
+    import time
+    from mfcfd import cloud
+    from mfcfd.solver import Solver
+    big = Solver(cloud.shell_cloud(96, 11500, seed=7, knn_device=0), 0.5, 1.0, gpu_setup=1)
+    (small,) = _solvers(cloud.small_sphere(6, 100, r1=1.5, seed=3), 1)
+    big.initial_conditions()
+    (ref,) = _solvers(cloud.small_sphere(6, 100, r1=1.5, seed=3), 1)
+    over = []
+    th = threading.Thread(target=lambda: (big.q_lskum(100), over.append(1)))
+    th.start()
+    time.sleep(0.2)                        # of about 2.6 s
+    steps = 0
+    while not over and steps < 200:
+        steps += 1
+        small.fpi_solver(steps)
+    th.join()
+    assert steps >= 100
+    ref.q_lskum(steps)
+    assert np.array_equal(small.get(mfcfd_lib.FIELD_PRIM), ref.get(mfcfd_lib.FIELD_PRIM))
+    for s in (big, small, ref):
+        s.close()
